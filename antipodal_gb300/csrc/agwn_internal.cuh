@@ -10,6 +10,7 @@
 #include <cstring>
 
 #include "../../include/antipodal_gb300.h"
+#include "intfp.cuh"
 
 namespace agwn
 {
@@ -240,7 +241,8 @@ struct agwn_context : agwn::Context
 namespace agwn
 {
 // Unfused IEEE arithmetic.  Each operation rounds once, like the reference's default (FMA-free) CPU build, so a
-// formula written with these reproduces the CPU's values exactly.  The intrinsics are never contracted.
+// formula written with these reproduces the CPU's values exactly.  The intrinsics are never contracted.  Division
+// and square root of doubles run on the integer pipe (intfp.cuh), with the same bits.
 struct rd
 {
     double v;
@@ -249,7 +251,7 @@ struct rd
     __device__ __forceinline__ friend rd operator+(rd a, rd b) { return rd(__dadd_rn(a.v, b.v)); }
     __device__ __forceinline__ friend rd operator-(rd a, rd b) { return rd(__dsub_rn(a.v, b.v)); }
     __device__ __forceinline__ friend rd operator*(rd a, rd b) { return rd(__dmul_rn(a.v, b.v)); }
-    __device__ __forceinline__ friend rd operator/(rd a, rd b) { return rd(__ddiv_rn(a.v, b.v)); }
+    __device__ __forceinline__ friend rd operator/(rd a, rd b) { return rd(div_rn_int(a.v, b.v)); }
     __device__ __forceinline__ friend rd operator-(rd a) { return rd(-a.v); }
 };
 struct rf
@@ -278,7 +280,7 @@ struct exact_of<float>
 
 __device__ __forceinline__ rd ex_sqrt(rd a)
 {
-    return rd(__dsqrt_rn(a.v));
+    return rd(sqrt_rn_int(a.v));
 }
 __device__ __forceinline__ rf ex_sqrt(rf a)
 {
@@ -286,7 +288,7 @@ __device__ __forceinline__ rf ex_sqrt(rf a)
 }
 __device__ __forceinline__ double ex_atan2(rd y, rd x)
 {
-    return atan2(y.v, x.v);
+    return atan2_int(y.v, x.v);
 }
 __device__ __forceinline__ float ex_atan2(rf y, rf x)
 {

@@ -570,7 +570,7 @@ __device__ __forceinline__ double l_plus_x(qv3<typename P::C> v, double l)
     double const vx = P::cdbl(v.x);
     if (v.x >= 0)
         return __dadd_rn(l, vx);
-    return __ddiv_rn(dot_yz<P>(v, v), __dsub_rn(l, vx));
+    return div_rn_int(dot_yz<P>(v, v), __dsub_rn(l, vx));
 }
 
 // Half-area contribution of one boundary segment.  gwn_mesh_robust.hh:272-321.
@@ -599,7 +599,7 @@ __device__ __forceinline__ double robust_contrib(qv3<typename P::C> q, RSeg<type
     double const yz = dot_yz<P>(v0, v1);
     double const den = __dadd_rn(__dmul_rn(l_plus_x<P>(v0, l0), l_plus_x<P>(v1, l1)), yz);
     if (P::sgn(num) != 0)
-        return atan2(P::dbl(num), den);
+        return atan2_int(P::dbl(num), den);
     if (v0.y == 0 && v0.z == 0 && v0.x < 0 && (v1.y != 0 || v1.z != 0))
         return v1.z != 0 ? atan2(P::cdbl(v1.z), -P::cdbl(v1.y)) : (v1.y > 0 ? -pi : 0.0);
     if (v1.y == 0 && v1.z == 0 && v1.x < 0 && (v0.y != 0 || v0.z != 0))
