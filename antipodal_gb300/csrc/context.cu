@@ -286,6 +286,7 @@ int agwn_context_destroy(agwn_context* ctx)
         cudaStreamSynchronize(ctx->stream);
     for (auto& b : ctx->scratch)
         b.release();
+    ctx->bernstein.release();
     ctx->ray_cache.h.release();
     ctx->ray_cache.cells.release();
     for (int i = 0; i < Context::kMaxPending; ++i)

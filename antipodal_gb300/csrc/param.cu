@@ -2,12 +2,14 @@
 // eval_gwnr_parametric_batch_fractional (src/antipodal/gwn_parametric.hh:168-186) with IntegratorGK15
 // (src/antipodal/math/integrate_gk15.hh:63-290) and the integrand of gwn_parametric.hh:73-103.
 //
-// One thread per query walks the curves in order (curves staged in shared memory by cp.async.bulk) and
-// integrates each with an explicit stack instead of recursion.  A panel is (depth, index): its end points are the
-// dyadic numbers index * 2^-depth and its local tolerance tol * 2^-depth, exactly what the reference's halving
-// computes, so a panel fits in 32 bits.  A second stack of values replays the reference's `left + right`
-// summation order (post-order), and the integrand and the G7/K15 sums are written unfused, so the result equals
-// the CPU reference bit for bit.
+// A panel is (depth, index): its end points are the dyadic numbers index * 2^-depth and its local tolerance
+// tol * 2^-depth, exactly what the reference's halving computes, so a panel fits in 32 bits.  The tree is walked
+// without recursion in the reference's order, and a finished left sibling's value per level replays its
+// `left + right` summation (post-order).  Two arithmetic forms:
+//  * exact -- the integrand and the G7/K15 sums in FP64, unfused, in the reference's order (k_param_exact): the
+//    result equals the CPU reference bit for bit.
+//  * mixed -- double-float arithmetic on the FP32 pipe (k_param_gk15), curves staged in shared memory by
+//    cp.async.bulk.
 //
 // Proposal hook: a per-(query, curve) start depth s (from the learned proposal; 0 for the plain method).  Panels
 // above depth s are split without being evaluated; every panel at depth >= s is evaluated and accepted or split by
@@ -27,7 +29,6 @@ namespace
 {
 constexpr int kParamMaxDepth = 24; // deepest panel the integrator can reach (2^24 panels per curve)
 constexpr int kParamBlock = 128;
-constexpr int kParamTileMax = 1024; // curves staged per tile (96 KB of shared memory)
 // The double-float form stages 384 curves (36 KB, room for the per-panel network's weights beside them), so that
 // six blocks reside per SM, the number its 80 registers allow.  Measured on 256 bicubic patches at tol 1e-10:
 // 40K queries, 768 was 10% faster than 1024 and flat down to 128; 250K queries (one work item per query block),
@@ -69,9 +70,13 @@ __device__ __forceinline__ dual smul(rd s, dual b)
     return {s * b.v, s * b.d};
 }
 
-// w(t) - d_eta(t) for the cubic Bezier curve c at parameter t, with the dual-number evaluation of the curve
-// (Bernstein basis, summed c0*b0 + c1*b1 + c2*b2 + c3*b3) and normalize_fd (src/antipodal/math/fwd_diff.hh:497-532).
-__device__ __forceinline__ double integrand(const double* c, ev3<rd> p, ev3<rd> x0, double tt)
+// The cubic Bernstein polynomials and their derivatives at t, by the reference's dual-number evaluation: the values
+// b0..b3, then the derivatives.
+struct Bernstein
+{
+    rd v[4], d[4];
+};
+__device__ __forceinline__ Bernstein bernstein(double tt)
 {
     dual const t{rd(tt), rd(1.0)};
     dual const u{rd(1.0) - rd(tt), rd(-1.0)};
@@ -79,11 +84,20 @@ __device__ __forceinline__ double integrand(const double* c, ev3<rd> p, ev3<rd> 
     dual const b1 = dmul(dmul(smul(rd(3.0), u), u), t);
     dual const b2 = dmul(dmul(smul(rd(3.0), u), t), t);
     dual const b3 = dmul(dmul(t, t), t);
+    return {{b0.v, b1.v, b2.v, b3.v}, {b0.d, b1.d, b2.d, b3.d}};
+}
+
+// w(t) - d_eta(t) for the cubic Bezier curve c at the parameter of basis B (summed c0*b0 + c1*b1 + c2*b2 + c3*b3) and
+// normalize_fd (src/antipodal/math/fwd_diff.hh:497-532).  The reference's x1 = -x0 appears negated: each of its
+// products and sums is the exact negative of the one with x0, so b = -a, b' = -a', and x1 b = x0 a.
+__device__ __forceinline__ double integrand(const double (&c)[12], Bernstein const& B, ev3<rd> p, ev3<rd> x0)
+{
     rd phi[3], dphi[3];
+#pragma unroll
     for (int k = 0; k < 3; ++k)
     {
-        phi[k] = rd(c[k]) * b0.v + rd(c[3 + k]) * b1.v + rd(c[6 + k]) * b2.v + rd(c[9 + k]) * b3.v;
-        dphi[k] = rd(c[k]) * b0.d + rd(c[3 + k]) * b1.d + rd(c[6 + k]) * b2.d + rd(c[9 + k]) * b3.d;
+        phi[k] = rd(c[k]) * B.v[0] + rd(c[3 + k]) * B.v[1] + rd(c[6 + k]) * B.v[2] + rd(c[9 + k]) * B.v[3];
+        dphi[k] = rd(c[k]) * B.d[0] + rd(c[3 + k]) * B.d[1] + rd(c[6 + k]) * B.d[2] + rd(c[9 + k]) * B.d[3];
     }
     ev3<rd> const r{phi[0] - p.x, phi[1] - p.y, phi[2] - p.z};
     ev3<rd> const dr{dphi[0], dphi[1], dphi[2]};
@@ -99,63 +113,59 @@ __device__ __forceinline__ double integrand(const double* c, ev3<rd> p, ev3<rd> 
     Gp.x = (dr.x - G.x * s1) * inv_s;
     Gp.y = (dr.y - G.y * s1) * inv_s;
     Gp.z = (dr.z - G.z * s1) * inv_s;
-    ev3<rd> const x1{-x0.x, -x0.y, -x0.z};
     rd const a = edot(x0, G);
     rd const ap = edot(x0, Gp);
     ev3<rd> const X = x0 - ev3<rd>{G.x * a, G.y * a, G.z * a};
     ev3<rd> const Xp = ev3<rd>{G.x * -ap, G.y * -ap, G.z * -ap} - ev3<rd>{Gp.x * a, Gp.y * a, Gp.z * a};
     rd const d_eta = edot(G, ecross(X, Xp)) / edot(X, X);
-    rd const b = edot(x1, G);
-    rd const bp = edot(x1, Gp);
-    ev3<rd> const v = G - ev3<rd>{x1.x * b, x1.y * b, x1.z * b};
-    ev3<rd> const vp = Gp - ev3<rd>{x1.x * bp, x1.y * bp, x1.z * bp};
-    rd const w = edot(x1, ecross(v, vp)) / edot(v, v);
+    ev3<rd> const v = G - ev3<rd>{x0.x * a, x0.y * a, x0.z * a};
+    ev3<rd> const vp = Gp - ev3<rd>{x0.x * ap, x0.y * ap, x0.z * ap};
+    rd const w = -(edot(x0, ecross(v, vp)) / edot(v, v));
     return (w - d_eta).v;
 }
 
-// One GK15 panel (depth, j) = [j 2^-depth, (j+1) 2^-depth] of curve c: the Kronrod and Gauss estimates in the
-// reference's node and summation order (integrate_gk15.hh:155-217).  Returns Ik; *err = |Ik - Ig|.
-__device__ __forceinline__ double gk15_panel(const double* c, ev3<rd> p, ev3<rd> x0, int depth, uint32_t j,
-                                             double* err)
+// ---- exact form -----------------------------------------------------------------------------------------------
+// A panel's 15 nodes are the lanes of a team of 16 (half a warp): lane 0 the centre, lanes 1-7 the nodes
+// centre - h x_k, lanes 8-14 centre + h x_(lane - 7), lane 15 a copy of the centre.
+constexpr int kTeam = 16;
+// The nodes' Bernstein bases depend on the panel alone, not on the curve or the query.  They are tabulated once per
+// context down to this depth: double2 [panel 2^d - 1 + j][4][16 lanes], the four pairs (v0 v1), (v2 v3), (d0 d1),
+// (d2 d3) -- 2.1 MB, read coalesced from L2, in place of 34 of the integrand's FP64 instructions.
+constexpr int kBernDepth = 10;
+constexpr int kBernPanels = (2 << kBernDepth) - 1;
+
+__device__ __forceinline__ double node_x(int lane)
 {
-    double const scale = ldexp(1.0, -depth);
+    return kGkX[lane == 15 ? 0 : (lane < 8 ? lane : lane - 7)];
+}
+__device__ __forceinline__ double pow2_neg(int e) // 2^-e
+{
+    return of_bits(uint64_t(1023 - e) << 52);
+}
+// The team's node of panel (depth, j) = [j 2^-depth, (j + 1) 2^-depth].
+__device__ __forceinline__ double panel_node(int depth, uint32_t j, int lane, double xk)
+{
+    double const scale = pow2_neg(depth);
     double const aa = double(j) * scale, bb = double(j + 1) * scale; // exact: j < 2^24
     rd const cc = (rd(aa) + rd(bb)) * rd(0.5);
     rd const h = (rd(bb) - rd(aa)) * rd(0.5);
-    double const f0 = integrand(c, p, x0, cc.v);
-    double fm[8], fp[8];
-#pragma unroll 1
-    for (int k = 1; k <= 7; ++k)
+    rd const dx = h * rd(xk);
+    return (lane < 8 ? cc - dx : cc + dx).v;
+}
+
+__global__ void k_bernstein(double2* __restrict__ table)
+{
+    int const i = int(blockIdx.x * blockDim.x + threadIdx.x), lane = i % kTeam, panel = i / kTeam;
+    if (panel >= kBernPanels)
+        return;
+    int const d = 31 - __clz(panel + 1);
+    Bernstein const B = bernstein(panel_node(d, uint32_t(panel + 1 - (1 << d)), lane, node_x(lane)));
+    double2* const o = table + size_t(panel) * 4 * kTeam + lane;
+    for (int k = 0; k < 2; ++k)
     {
-        rd const dx = h * rd(kGkX[k]);
-        fm[k] = integrand(c, p, x0, (cc - dx).v);
-        fp[k] = integrand(c, p, x0, (cc + dx).v);
+        o[k * kTeam] = make_double2(B.v[2 * k].v, B.v[2 * k + 1].v);
+        o[(k + 2) * kTeam] = make_double2(B.d[2 * k].v, B.d[2 * k + 1].v);
     }
-    rd ig = rd(kGkWgCenter) * rd(f0);
-    rd ik = rd(kGkWk[0]) * rd(f0);
-    ik = ik + rd(kGkWk[1]) * (rd(fm[1]) + rd(fp[1]));
-    {
-        rd const s2 = rd(fm[2]) + rd(fp[2]);
-        ik = ik + rd(kGkWk[2]) * s2;
-        ig = ig + rd(kGkWg2) * s2;
-    }
-    ik = ik + rd(kGkWk[3]) * (rd(fm[3]) + rd(fp[3]));
-    {
-        rd const s4 = rd(fm[4]) + rd(fp[4]);
-        ik = ik + rd(kGkWk[4]) * s4;
-        ig = ig + rd(kGkWg4) * s4;
-    }
-    ik = ik + rd(kGkWk[5]) * (rd(fm[5]) + rd(fp[5]));
-    {
-        rd const s6 = rd(fm[6]) + rd(fp[6]);
-        ik = ik + rd(kGkWk[6]) * s6;
-        ig = ig + rd(kGkWg6) * s6;
-    }
-    ik = ik + rd(kGkWk[7]) * (rd(fm[7]) + rd(fp[7]));
-    ig = ig * h;
-    ik = ik * h;
-    *err = fabs((ik - ig).v);
-    return ik.v;
 }
 
 // ---- double-float form ----------------------------------------------------------------------------------------
@@ -293,23 +303,6 @@ __global__ void k_curves_df(const double* __restrict__ curves, int64_t n_curves,
         out[i / 12].c[i % 12] = df_from(curves[i]);
 }
 
-// out[q] = (sum over curves of the curve integral) / (4 pi).
-//
-// The cost of one (query, curve) integral is heavy-tailed: a query whose line along x0 passes close to a curve
-// needs a deep tree there.  So the work is shared out by pair, not by query.  A block owns up to kParamBlock
-// queries and, for each shared-memory tile of curves, the pool of (query, curve) pairs of that tile; a lane that
-// finishes its pair takes the next one from the pool (one shared-memory atomic per warp).  Each lane walks its
-// pair's panel tree without a stack: after a split the next panel is the left child (depth + 1, 2j); after an
-// accepted leaf the walk climbs while the finished node is a right child (j odd), combining left + right from
-// `pending` (the finished left sibling's value per level), then moves to the right sibling (depth, j + 1).
-// Panels above the pair's start depth are not evaluated: the walk descends to the leftmost descendant at the
-// start depth.  A finished pair's integral goes to the block's slab of `pair_vals`; after the tile each thread
-// adds its query's row in curve order.  Every sum is the reference's (post-order left + right within a curve,
-// curves in order), so the result does not depend on how the pairs were shared out.
-//
-// start_depth: per (query, curve), row-major [n][n_curves], nullable = all 0.  stats (nullable): per (query,
-// curve) packed as leaves | shallowest leaf depth << 16 | deepest leaf depth << 24.  nodes_total (nullable):
-// panels evaluated per query.  pair_vals: gridDim.x * kParamBlock * tile doubles.
 // Optional work of the integrator kernel.
 //   panel_log: training data for the per-panel network, 2 words per evaluated panel below max_depth -- the pair's
 //     index (query * n_curves + curve) and (depth << 25) | (j << 1) | accepted; entries past log_cap are counted,
@@ -330,6 +323,199 @@ struct ParamExtras
     unsigned long long* skip_count;
 };
 
+// Pair integrals in the exact form: vals[k * nq + i] for the curves c0 + k and the queries q0 + i.
+//
+// FP64 issue bounds it (one warp instruction per 16 clocks per SM; about 155 for an integrand of 15 nodes x 2 panels,
+// and 12 for a panel's sums).  The cost of one pair is heavy-tailed -- a query whose line along x0 passes close to a
+// curve needs a deep tree there -- so the teams of the whole grid draw their pairs from one counter, and a panel takes
+// one integrand time, not 15: a deep pair is no tail, and a few pairs fill the chip.  Each team walks its pair's panel
+// tree without a stack: after a split the next panel is the left child (depth + 1, 2j); after an accepted leaf the
+// walk climbs while the finished node is a right child (j odd), combining left + right from `pending` (the finished
+// left sibling's value per level), then moves to the right sibling (depth, j + 1).  Panels above the pair's start
+// depth are not evaluated: the walk descends to the leftmost descendant at the start depth.  All lanes of a team hold
+// the same walk state.  Measured against one thread per pair with the pairs of 128 queries on one block: 3,001
+// queries x 96 curves at tol 1e-8 (24 such blocks) 86.5 -> 9.5 ms.
+__global__ void __launch_bounds__(kParamBlock, 4)
+    k_param_exact(const double* __restrict__ pos, int64_t q0, int nq, ev3<rd> x0, const double* __restrict__ curves,
+                  int64_t n_curves, int64_t c0, int nc, int min_depth, int max_depth, double tol,
+                  const uint8_t* __restrict__ start_depth, uint32_t* __restrict__ stats, int32_t* __restrict__ nodes_total,
+                  double* __restrict__ vals, int* __restrict__ next, const double2* __restrict__ table, ParamExtras ex)
+{
+    __shared__ double tol_at[kParamMaxDepth + 1];
+    __shared__ double s_pending[kParamBlock / kTeam][kParamMaxDepth + 1];
+    if (threadIdx.x == 0)
+    {
+        // tol * 2^-d by repeated halving, as the recursion computes it (exact unless it reaches subnormals)
+        tol_at[0] = tol;
+        for (int l = 1; l <= kParamMaxDepth; ++l)
+            tol_at[l] = __dmul_rn(tol_at[l - 1], 0.5);
+    }
+    __syncthreads();
+    int const total = nq * nc;
+    unsigned const lane = threadIdx.x & 31u, tm = 0xffffu << (lane & 16u);
+    int const tl = int(lane & 15u);
+    double const xk = node_x(tl);
+    // lanes 0-7 weigh the node sums for Ik, lanes 8-15 (the same sums again) for Ig: 0 at the odd ones
+    double const wt = tl < 8 ? kGkWk[tl]
+                             : (tl == 8 ? kGkWgCenter : tl == 10 ? kGkWg2 : tl == 12 ? kGkWg4 : tl == 14 ? kGkWg6 : 0.0);
+    bool const weighed = tl < 8 || (tl & 1) == 0;
+    double* const pending = s_pending[threadIdx.x / kTeam];
+    int pi = -1; // this team's pair, -1 = needs one
+    bool drained = false;
+    int k = 0, ql = 0, s = 0, d = 0, leaves = 0, dmin = 0, dmax = 0, pnodes = 0;
+    uint32_t j = 0;
+    ev3<rd> p{};
+    double c[12] = {};
+    for (;;)
+    {
+        unsigned const want = __ballot_sync(0xffffffffu, tl == 0 && pi < 0 && !drained);
+        if (want)
+        {
+            int base = 0;
+            if (lane == 0)
+                base = atomicAdd(next, __popc(want));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (pi < 0 && !drained)
+            {
+                int const mine = base + __popc(want & ((1u << (lane & 16u)) - 1u));
+                if (mine < total)
+                {
+                    pi = mine;
+                    k = mine / nq;
+                    ql = mine - k * nq;
+                    int64_t const q = q0 + ql;
+                    p = ev3<rd>{rd(pos[3 * q]), rd(pos[3 * q + 1]), rd(pos[3 * q + 2])};
+                    const double* const cv = curves + 12 * (c0 + k);
+#pragma unroll
+                    for (int e = 0; e < 12; ++e)
+                        c[e] = cv[e];
+                    s = start_depth ? min(int(start_depth[q * n_curves + c0 + k]), max_depth) : 0;
+                    d = s;
+                    j = 0;
+                    leaves = 0;
+                    dmin = 255;
+                    dmax = 0;
+                    pnodes = 0;
+                }
+                else
+                    drained = true;
+            }
+        }
+        if (!__any_sync(0xffffffffu, pi >= 0))
+            break;
+        if (pi >= 0) // the team's lanes agree
+        {
+            rd const h = rd(pow2_neg(d + 1)); // half the panel's width, exact
+            Bernstein B;
+            if (d <= kBernDepth)
+            {
+                const double2* const r = table + size_t((1u << d) - 1u + j) * 4 * kTeam + tl;
+                double2 const b0 = __ldg(r), b1 = __ldg(r + kTeam), b2 = __ldg(r + 2 * kTeam), b3 = __ldg(r + 3 * kTeam);
+                B = {{rd(b0.x), rd(b0.y), rd(b1.x), rd(b1.y)}, {rd(b2.x), rd(b2.y), rd(b3.x), rd(b3.y)}};
+            }
+            else
+                B = bernstein(panel_node(d, j, tl, xk));
+            double const f = integrand(c, B, p, x0);
+            // the sums of the reference (integrate_gk15.hh:155-217): s_0 = f(centre), s_k = f(-k) + f(+k), then
+            // Ik = (wk_0 s_0 + wk_1 s_1 + ...) h term by term, Ig likewise over the even k (lanes 8-15 add exact
+            // zeros for the others)
+            double const other = __shfl_sync(tm, f, (tl & 7) + 7, kTeam);
+            double const mine = __shfl_sync(tm, f, tl & 7, kTeam);
+            double const sum2 = (tl & 7) ? (rd(mine) + rd(other)).v : mine;
+            double const term = weighed ? (rd(wt) * rd(sum2)).v : 0.0;
+            rd acc = rd(__shfl_sync(tm, term, tl & 8, kTeam));
+#pragma unroll
+            for (int e = 1; e < 8; ++e)
+                acc = acc + rd(__shfl_sync(tm, term, (tl & 8) + e, kTeam));
+            acc = acc * h;
+            double const twin = __shfl_xor_sync(tm, acc.v, 8, kTeam);
+            double const err = fabs((acc - rd(twin)).v);
+            double v = tl < 8 ? acc.v : twin;
+            ++pnodes;
+            bool const accept = d >= max_depth || (d >= min_depth && err <= tol_at[d]);
+            if (ex.panel_log && d < max_depth && tl == 0)
+            {
+                unsigned long long const slot = atomicAdd(ex.log_count, 1ull);
+                if ((long long)slot < ex.log_cap)
+                {
+                    ex.panel_log[2 * slot] = uint32_t((q0 + ql) * n_curves + c0 + k);
+                    ex.panel_log[2 * slot + 1] = (uint32_t(d) << 25) | (j << 1) | (accept ? 1u : 0u);
+                }
+            }
+            if (!accept)
+            {
+                ++d; // split: left child next
+                j <<= 1;
+            }
+            else
+            {
+                ++leaves;
+                dmin = min(dmin, d);
+                dmax = max(dmax, d);
+                while (d > 0 && (j & 1u))
+                {
+                    v = __dadd_rn(pending[d], v); // left + right
+                    --d;
+                    j >>= 1;
+                }
+                if (d > 0)
+                {
+                    pending[d] = v; // a finished left child (every lane stores the same value): its sibling is next
+                    ++j;
+                    while (d < s)
+                    {
+                        ++d;
+                        j <<= 1;
+                    }
+                }
+                else
+                {
+                    // the root is done: v is this pair's integral
+                    if (tl == 0)
+                    {
+                        vals[int64_t(k) * nq + ql] = v;
+                        if (stats)
+                            stats[(q0 + ql) * n_curves + c0 + k] = uint32_t(min(leaves, 0xffff)) |
+                                                                   (uint32_t(dmin) << 16) | (uint32_t(dmax) << 24);
+                        if (nodes_total)
+                            atomicAdd(nodes_total + q0 + ql, pnodes);
+                    }
+                    pi = -1;
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// The pair integrals of each query added in curve order: out[i] (the running sum, from 0 with `first`) over this
+// chunk's curves, divided by 4 pi with `last`.
+__global__ void k_param_sum(const double* __restrict__ vals, int nq, int nc, bool first, bool last,
+                            double* __restrict__ out)
+{
+    int const i = int(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= nq)
+        return;
+    rd sum = first ? rd(0.0) : rd(out[i]);
+#pragma unroll 8
+    for (int k = 0; k < nc; ++k)
+        sum = sum + rd(vals[int64_t(k) * nq + i]);
+    out[i] = last ? (sum / (rd(4.0) * rd(3.141592653589793238462643383279502884))).v : sum.v;
+}
+
+// out[q] = (sum over curves of the curve integral) / (4 pi).
+//
+// The double-float form.  The cost of one (query, curve) integral is heavy-tailed, so the work is shared out by pair,
+// not by query.  A block owns up to kParamBlock
+// queries and, for each shared-memory tile of curves, the pool of (query, curve) pairs of that tile; a lane that
+// finishes its pair takes the next one from the pool (one shared-memory atomic per warp).  Each lane walks its
+// pair's panel tree as a team of the exact form does.  A finished pair's integral goes to the block's slab of `pair_vals`; after the tile each thread
+// adds its query's row in curve order.  Every sum is the reference's (post-order left + right within a curve,
+// curves in order), so the result does not depend on how the pairs were shared out.
+//
+// start_depth: per (query, curve), row-major [n][n_curves], nullable = all 0.  stats (nullable): per (query,
+// curve) packed as leaves | shallowest leaf depth << 16 | deepest leaf depth << 24.  nodes_total (nullable):
+// panels evaluated per query.  pair_vals: gridDim.x * kParamBlock * tile doubles.
 // The per-panel network's shared memory, after the curve tile.
 struct PanelSmem
 {
@@ -338,18 +524,18 @@ struct PanelSmem
     float logit[kParamBlock / 32][32][2];
 };
 
-// DF: double-float panels.  PANEL (DF only): the per-panel network runs (its code and shared memory are compiled
-// only into this instance, so the other instances keep their registers).  n_groups > 1 (DF only): the curve tiles
+// PANEL: the per-panel network runs (its code and shared memory are compiled only into this instance, so the other
+// instance keeps its registers).  n_groups > 1: the curve tiles
 // of a query block are split into n_groups consecutive groups, one work item each, and each item writes its raw
 // partial sum to partial[g * n + i] (a later kernel adds the groups in order) and adds its panel counts to
 // nodes_total[i] (zeroed first).
-template <bool DF, bool PANEL>
+template <bool PANEL>
 constexpr int param_min_blocks()
 {
-    return DF && !PANEL ? 6 : 1; // the double-float panels in 80 registers (no spills), six blocks per SM
+    return !PANEL ? 6 : 1; // the double-float panels in 80 registers (no spills), six blocks per SM
 }
-template <bool DF, bool PANEL>
-__global__ void __launch_bounds__(kParamBlock, param_min_blocks<DF, PANEL>()) k_param_gk15(const double* __restrict__ pos, int64_t n,
+template <bool PANEL>
+__global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>()) k_param_gk15(const double* __restrict__ pos, int64_t n,
                                                             double* __restrict__ out, double x0x, double x0y,
                                                             double x0z, const Bez* __restrict__ curves,
                                                             int64_t n_curves, int tile, int min_depth, int max_depth,
@@ -368,7 +554,6 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<DF, PANEL>()) k_
     bool const use_panel = PANEL && ex.pwb != nullptr;
     unsigned long long skips = 0;
     double* const slab = pair_vals + size_t(blockIdx.x) * kParamBlock * tile;
-    ev3<rd> const x0{rd(x0x), rd(x0y), rd(x0z)};
     df3 const x0df{df_from(x0x), df_from(x0y), df_from(x0z)};
     double const x0n = x0x * x0x + x0y * x0y + x0z * x0z;
     bool const x0_unit = fabs(x0n - 1.0) <= 1e-15;
@@ -426,7 +611,7 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<DF, PANEL>()) k_
             int k = 0, ql = 0, s = 0, d = 0, leaves = 0, dmin = 0, dmax = 0, pnodes = 0;
             uint32_t j = 0;
             ev3<rd> p{};
-            df cp[DF ? 12 : 1]; // DF: this pair's curve minus its query, as power coefficients about t = 1/2
+            df cp[12]; // this pair's curve minus its query, as power coefficients about t = 1/2
             double pending[kParamMaxDepth + 1];
             for (;;)
             {
@@ -448,15 +633,12 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<DF, PANEL>()) k_
                             ql = mine - k * nq;
                             int64_t const q = q0 + ql;
                             p = ev3<rd>{rd(pos[3 * q]), rd(pos[3 * q + 1]), rd(pos[3 * q + 2])};
-                            if constexpr (DF)
-                            {
-                                df const pd[3] = {df_from(p.x.v), df_from(p.y.v), df_from(p.z.v)};
-                                CurveDF const& cv = reinterpret_cast<const CurveDF*>(buf)[k];
+                            df const pd[3] = {df_from(p.x.v), df_from(p.y.v), df_from(p.z.v)};
+                            CurveDF const& cv = reinterpret_cast<const CurveDF*>(buf)[k];
 #pragma unroll
-                                for (int e = 0; e < 12; ++e)
-                                    cp[e] = cv.c[e] - pd[e % 3];
-                                power_about_half(cp);
-                            }
+                            for (int e = 0; e < 12; ++e)
+                                cp[e] = cv.c[e] - pd[e % 3];
+                            power_about_half(cp);
                             s = start_depth ? min(int(start_depth[q * n_curves + c0 + k]), max_depth) : 0;
                             d = s;
                             j = 0;
@@ -471,80 +653,70 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<DF, PANEL>()) k_
                 }
                 if (!__any_sync(0xffffffffu, pi >= 0))
                     break;
-                if constexpr (DF)
+                // the per-panel network: up to four rounds of "split it without evaluating", all lanes together
+                for (int round = 0; PANEL && use_panel && round < 4; ++round)
                 {
-                    // the per-panel network: up to four rounds of "split it without evaluating", all lanes together
-                    for (int round = 0; PANEL && use_panel && round < 4; ++round)
+                    bool const cand = pi >= 0 && d < max_depth;
+                    float f[kF];
+                    if (cand)
                     {
-                        bool const cand = pi >= 0 && d < max_depth;
-                        float f[kF];
-                        if (cand)
-                        {
-                            // the control points minus the query, as the network was trained on them
-                            df const pd[3] = {df_from(p.x.v), df_from(p.y.v), df_from(p.z.v)};
-                            CurveDF const& cv = reinterpret_cast<const CurveDF*>(buf)[k];
-                            float cpf[12];
+                        // the control points minus the query, as the network was trained on them
+                        df const pd[3] = {df_from(p.x.v), df_from(p.y.v), df_from(p.z.v)};
+                        CurveDF const& cv = reinterpret_cast<const CurveDF*>(buf)[k];
+                        float cpf[12];
 #pragma unroll
-                            for (int e = 0; e < 12; ++e)
-                                cpf[e] = (cv.c[e] - pd[e % 3]).hi;
-                            panel_features(cpf, d, j, x0f, ex.log10_tol, f);
-                        }
-                        else
-                        {
+                        for (int e = 0; e < 12; ++e)
+                            cpf[e] = (cv.c[e] - pd[e % 3]).hi;
+                        panel_features(cpf, d, j, x0f, ex.log10_tol, f);
+                    }
+                    else
+                    {
 #pragma unroll
-                            for (int e = 0; e < kF; ++e)
-                                f[e] = 0.f;
-                        }
-                        uint32_t* const row = ps->feat[warp][lane];
+                        for (int e = 0; e < kF; ++e)
+                            f[e] = 0.f;
+                    }
+                    uint32_t* const row = ps->feat[warp][lane];
 #pragma unroll
-                        for (int e = 0; e < kF / 2; ++e)
-                            row[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
-                        row[6] = 0u;
-                        row[7] = 0u;
-                        __syncwarp();
-                        int const g = int(lane >> 2), tig = int(lane & 3u);
+                    for (int e = 0; e < kF / 2; ++e)
+                        row[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
+                    row[6] = 0u;
+                    row[7] = 0u;
+                    __syncwarp();
+                    int const g = int(lane >> 2), tig = int(lane & 3u);
 #pragma unroll
-                        for (int mt = 0; mt < 2; ++mt)
+                    for (int mt = 0; mt < 2; ++mt)
+                    {
+                        uint32_t a0[4] = {ps->feat[warp][mt * 16 + g][tig], ps->feat[warp][mt * 16 + g + 8][tig],
+                                          ps->feat[warp][mt * 16 + g][4 + tig],
+                                          ps->feat[warp][mt * 16 + g + 8][4 + tig]};
+                        float z1[8][4], z2[8][4], z3[2][4];
+                        mlp_forward(ps->w, a0, z1, z2, z3);
+                        if (tig == 0) // columns 0 and 1: the split and accept logits
                         {
-                            uint32_t a0[4] = {ps->feat[warp][mt * 16 + g][tig], ps->feat[warp][mt * 16 + g + 8][tig],
-                                              ps->feat[warp][mt * 16 + g][4 + tig],
-                                              ps->feat[warp][mt * 16 + g + 8][4 + tig]};
-                            float z1[8][4], z2[8][4], z3[2][4];
-                            mlp_forward(ps->w, a0, z1, z2, z3);
-                            if (tig == 0) // columns 0 and 1: the split and accept logits
-                            {
-                                ps->logit[warp][mt * 16 + g][0] = z3[0][0];
-                                ps->logit[warp][mt * 16 + g][1] = z3[0][1];
-                                ps->logit[warp][mt * 16 + g + 8][0] = z3[0][2];
-                                ps->logit[warp][mt * 16 + g + 8][1] = z3[0][3];
-                            }
+                            ps->logit[warp][mt * 16 + g][0] = z3[0][0];
+                            ps->logit[warp][mt * 16 + g][1] = z3[0][1];
+                            ps->logit[warp][mt * 16 + g + 8][0] = z3[0][2];
+                            ps->logit[warp][mt * 16 + g + 8][1] = z3[0][3];
                         }
-                        __syncwarp();
-                        bool const skip =
-                            cand && (ps->logit[warp][lane][1] - ps->logit[warp][lane][0]) < ex.skip_logit;
-                        __syncwarp();
-                        if (!__any_sync(0xffffffffu, skip))
-                            break;
-                        if (skip)
-                        {
-                            ++d; // split without evaluating: left child next
-                            j <<= 1;
-                            ++skips;
-                        }
+                    }
+                    __syncwarp();
+                    bool const skip =
+                        cand && (ps->logit[warp][lane][1] - ps->logit[warp][lane][0]) < ex.skip_logit;
+                    __syncwarp();
+                    if (!__any_sync(0xffffffffu, skip))
+                        break;
+                    if (skip)
+                    {
+                        ++d; // split without evaluating: left child next
+                        j <<= 1;
+                        ++skips;
                     }
                 }
                 if (pi < 0)
                     continue;
-                double err;
-                double v;
-                if constexpr (DF)
-                {
-                    float e32;
-                    v = gk15_panel_df(cp, x0df, x0n_df, x0_unit, d, j, &e32);
-                    err = double(e32);
-                }
-                else
-                    v = gk15_panel(buf[k].c, p, x0, d, j, &err);
+                float e32;
+                double v = gk15_panel_df(cp, x0df, x0n_df, x0_unit, d, j, &e32);
+                double const err = double(e32);
                 ++pnodes;
                 bool const accept = d >= max_depth || (d >= min_depth && err <= tol_at[d]);
                 if (ex.panel_log && d < max_depth)
@@ -628,6 +800,52 @@ __global__ void k_param_groups(const double* __restrict__ partial, int n_groups,
         out[i] = (sum / (rd(4.0) * rd(3.141592653589793238462643383279502884))).v;
     }
 }
+
+// The exact form over chunks of at most 2^25 pairs (268 MB of pair integrals): queries first, and curves where one
+// query has more.
+int param_run_exact(Context& ctx, const double* d_pos, int64_t n, double* d_out, const double* x0, const double* d_curves,
+                    int64_t n_curves, int min_depth, int max_depth, double tol, const uint8_t* d_start,
+                    uint32_t* d_stats, int32_t* d_nodes, ParamExtras const& ex)
+{
+    if (!ctx.bernstein.ptr)
+    {
+        AGWN_TRY(ctx.bernstein.reserve(sizeof(double2) * 4 * kTeam * kBernPanels));
+        AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
+        k_bernstein<<<div_up(kBernPanels * kTeam, 256), 256, 0, ctx.stream>>>(static_cast<double2*>(ctx.bernstein.ptr));
+        AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
+    }
+    constexpr int64_t most = int64_t(1) << 25;
+    int64_t const nc_max = std::min(n_curves, most);
+    int64_t const nq_max = std::min(n, std::max<int64_t>(1, most / nc_max));
+    double* vals = nullptr;
+    int* next = nullptr;
+    AGWN_TRY(ctx.scratch_reserve(S_SEGS_RAW, sizeof(double) * size_t(nc_max) * size_t(nq_max),
+                                 reinterpret_cast<void**>(&vals)));
+    AGWN_TRY(ctx.scratch_reserve(S_PARTIAL, sizeof(int), reinterpret_cast<void**>(&next)));
+    if (d_nodes)
+        AGWN_TRY_CUDA(cudaMemsetAsync(d_nodes, 0, sizeof(int32_t) * n, ctx.stream));
+    int per_sm = 0;
+    AGWN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_param_exact, kParamBlock, 0));
+    ev3<rd> const x0v{rd(x0[0]), rd(x0[1]), rd(x0[2])};
+    for (int64_t q0 = 0; q0 < n; q0 += nq_max)
+        for (int64_t c0 = 0; c0 < n_curves; c0 += nc_max)
+        {
+            int const nq = int(std::min(nq_max, n - q0)), nc = int(std::min(nc_max, n_curves - c0));
+            int const grid = int(std::min<int64_t>(div_up(int64_t(nq) * nc, kParamBlock / kTeam),
+                                                   int64_t(std::max(per_sm, 1)) * ctx.sm_count));
+            AGWN_TRY_CUDA(cudaMemsetAsync(next, 0, sizeof(int), ctx.stream));
+            AGWN_TRY(ctx.launch_begin(AGWN_K_PARAMETRIC));
+            k_param_exact<<<grid, kParamBlock, 0, ctx.stream>>>(d_pos, q0, nq, x0v, d_curves, n_curves, c0, nc,
+                                                                min_depth, max_depth, tol, d_start, d_stats, d_nodes,
+                                                                vals, next,
+                                                                static_cast<const double2*>(ctx.bernstein.ptr), ex);
+            AGWN_TRY(ctx.launch_end(AGWN_K_PARAMETRIC));
+            AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
+            k_param_sum<<<div_up(nq, 64), 64, 0, ctx.stream>>>(vals, nq, nc, c0 == 0, c0 + nc == n_curves, d_out + q0);
+            AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
+        }
+    return AGWN_OK;
+}
 } // namespace
 
 int param_run(Context& ctx, const double* d_pos, int64_t n, double* d_out, const double* x0, const double* d_curves,
@@ -659,9 +877,12 @@ int param_run(Context& ctx, const double* d_pos, int64_t n, double* d_out, const
             AGWN_TRY_CUDA(cudaMemsetAsync(d_nodes, 0, sizeof(int32_t) * n, ctx.stream));
         return AGWN_OK;
     }
+    if (!dfm)
+        return param_run_exact(ctx, d_pos, n, d_out, x0, d_curves, n_curves, min_depth, max_depth, tol, d_start,
+                               d_stats, d_nodes, ex);
     static_assert(sizeof(CurveDF) == sizeof(Bez), "both curve forms stage through the same tile");
-    auto const kern = dfm ? (panel ? k_param_gk15<true, true> : k_param_gk15<true, false>) : k_param_gk15<false, false>;
-    int tile = int(std::min<int64_t>(dfm ? kParamTileDF : kParamTileMax, n_curves));
+    auto const kern = panel ? k_param_gk15<true> : k_param_gk15<false>;
+    int tile = int(std::min<int64_t>(kParamTileDF, n_curves));
     size_t smem = 0;
     int per_sm = 0;
     auto shape = [&](int t) -> int
@@ -678,7 +899,7 @@ int param_run(Context& ctx, const double* d_pos, int64_t n, double* d_out, const
     int n_groups = 1;
     // two waves of work items; tiles of at least 128 curves (measured: more waves or other tiles change <1%)
     int64_t const waves = 2, min_tile = 128;
-    if (dfm && n_blocks_q < waves * int64_t(per_sm) * ctx.sm_count)
+    if (n_blocks_q < waves * int64_t(per_sm) * ctx.sm_count)
     {
         // Few query blocks (a sample of queries, or many curves per query): the curves of each block are split
         // into groups of tiles, one work item each, so that every SM gets work.  Smaller tiles cost the
@@ -706,20 +927,15 @@ int param_run(Context& ctx, const double* d_pos, int64_t n, double* d_out, const
         if (d_nodes)
             AGWN_TRY_CUDA(cudaMemsetAsync(d_nodes, 0, sizeof(int32_t) * n, ctx.stream));
     }
-    const void* tile_src = d_curves;
-    if (dfm)
-    {
-        void* cdf = nullptr;
-        AGWN_TRY(ctx.scratch_reserve(S_FRAME, sizeof(CurveDF) * size_t(n_curves), &cdf));
-        AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-        k_curves_df<<<int(std::min<int64_t>(div_up(12 * n_curves, 256), 4 * ctx.sm_count)), 256, 0, ctx.stream>>>(
-            d_curves, n_curves, static_cast<CurveDF*>(cdf));
-        AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
-        tile_src = cdf;
-    }
+    void* cdf = nullptr;
+    AGWN_TRY(ctx.scratch_reserve(S_FRAME, sizeof(CurveDF) * size_t(n_curves), &cdf));
+    AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
+    k_curves_df<<<int(std::min<int64_t>(div_up(12 * n_curves, 256), 4 * ctx.sm_count)), 256, 0, ctx.stream>>>(
+        d_curves, n_curves, static_cast<CurveDF*>(cdf));
+    AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
     AGWN_TRY(ctx.launch_begin(AGWN_K_PARAMETRIC));
     kern<<<grid, kParamBlock, smem, ctx.stream>>>(d_pos, n, d_out, x0[0], x0[1], x0[2],
-                                                 reinterpret_cast<const Bez*>(tile_src), n_curves, tile, min_depth,
+                                                 static_cast<const Bez*>(cdf), n_curves, tile, min_depth,
                                                  max_depth, tol, d_start, d_stats, d_nodes, pair_vals, ctx.d_flags,
                                                  ex, n_groups, partial);
     AGWN_TRY(ctx.launch_end(AGWN_K_PARAMETRIC));
