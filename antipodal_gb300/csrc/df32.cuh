@@ -1,9 +1,9 @@
 // Double-float arithmetic: a value is hi + lo, two floats with |lo| <= ulp(hi) / 2, about 44 significant bits,
 // computed on the FP32 pipe (64x the FP64 rate of this GPU).  Built from the error-free transformations TwoSum
 // (Knuth), FastTwoSum (Dekker, |a| >= |b|) and TwoProduct by FMA; add is the "sloppy" variant (error relative to
-// |a| + |b|), multiply folds the cross terms into the FMA error term, divide takes two Newton-style corrections of
-// a float estimate and sqrt one.  Every step is written with explicit round-to-nearest intrinsics so the compiler
-// cannot reassociate or contract them.
+// |a| + |b|), multiply folds the cross terms into the FMA error term, divide takes three float digits and sqrt one
+// Newton-style correction of a float estimate.  Every step is written with explicit round-to-nearest intrinsics so
+// the compiler cannot reassociate or contract them.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -72,15 +72,42 @@ __device__ __forceinline__ df df_scale(df a, float p2)
 {
     return {__fmul_rn(a.hi, p2), __fmul_rn(a.lo, p2)};
 }
+// a b + c in one chain: the product's two floats, its cross terms and c.lo go into one low word
+__device__ __forceinline__ df df_fma(df a, df b, df c)
+{
+    df const p = two_prod(a.hi, b.hi);
+    float const e = __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.lo, p.lo));
+    df const s = two_sum(p.hi, c.hi);
+    return fast_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(e, c.lo)));
+}
+// a b + c d, and a b - c d
+__device__ __forceinline__ df df_dot2(df a, df b, df c, df d)
+{
+    df const p = two_prod(a.hi, b.hi), q = two_prod(c.hi, d.hi);
+    float const e = __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.lo, p.lo));
+    float const f = __fmaf_rn(c.lo, d.hi, __fmaf_rn(c.hi, d.lo, q.lo));
+    df const s = two_sum(p.hi, q.hi);
+    return fast_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(e, f)));
+}
+__device__ __forceinline__ df df_det2(df a, df b, df c, df d)
+{
+    return df_dot2(a, b, df{-c.hi, -c.lo}, d);
+}
+// a + b for |a| >= |b|
+__device__ __forceinline__ df df_add_ordered(df a, df b)
+{
+    df const s = fast_two_sum(a.hi, b.hi);
+    return fast_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo)));
+}
+// The quotient as three float digits q1 + q2 + q3 of one reciprocal; a.hi - q1 b.hi is exact in an FMA.
 __device__ __forceinline__ df operator/(df a, df b)
 {
-    float const rb = rcp_approx(b.hi); // one reciprocal for the three float quotients
+    float const rb = rcp_approx(b.hi);
     float const q1 = __fmul_rn(a.hi, rb);
-    df const r = a - b * df_make(q1);
-    float const q2 = __fmul_rn(r.hi, rb);
-    df const q = fast_two_sum(q1, q2);
-    df const r2 = a - b * q; // a second correction brings the quotient to double-float accuracy
-    return q + df_make(__fmul_rn(r2.hi, rb));
+    float const r1 = __fmaf_rn(-q1, b.hi, a.hi), l = __fmaf_rn(-q1, b.lo, a.lo);
+    float const q2 = __fmul_rn(__fadd_rn(r1, l), rb);
+    float const r2 = __fadd_rn(__fmaf_rn(-q2, b.hi, r1), l);
+    return fast_two_sum(q1, __fmaf_rn(r2, rb, q2));
 }
 __device__ __forceinline__ df df_sqrt(df a)
 {
@@ -88,28 +115,8 @@ __device__ __forceinline__ df df_sqrt(df a)
         return {sqrtf(a.hi), 0.f};
     float const ri = rsqrt_approx(a.hi);
     float const y = __fmul_rn(a.hi, ri);
-    df const e = a - two_prod(y, y);
-    return fast_two_sum(y, __fmul_rn(__fmul_rn(e.hi, ri), 0.5f));
-}
-
-struct df3
-{
-    df x, y, z;
-};
-__device__ __forceinline__ df3 operator-(df3 a, df3 b)
-{
-    return {a.x - b.x, a.y - b.y, a.z - b.z};
-}
-__device__ __forceinline__ df3 operator*(df3 a, df s)
-{
-    return {a.x * s, a.y * s, a.z * s};
-}
-__device__ __forceinline__ df dot(df3 a, df3 b)
-{
-    return a.x * b.x + a.y * b.y + a.z * b.z;
-}
-__device__ __forceinline__ df3 cross(df3 a, df3 b)
-{
-    return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+    df const p = two_prod(y, y);
+    float const e = __fadd_rn(__fsub_rn(__fsub_rn(a.hi, p.hi), p.lo), a.lo); // a.hi - p.hi is exact
+    return fast_two_sum(y, __fmul_rn(__fmul_rn(e, ri), 0.5f));
 }
 } // namespace agwn

@@ -18,6 +18,7 @@
 
 #include "agwn_internal.cuh"
 #include "df32.cuh"
+#include "hier.cuh"
 #include "mlp.cuh"
 #include "tma.cuh"
 
@@ -34,11 +35,6 @@ constexpr int kParamBlock = 128;
 // 40K queries, 768 was 10% faster than 1024 and flat down to 128; 250K queries (one work item per query block),
 // 384 is 1.7% faster than 768 (three blocks per SM) and 256 1.4%.
 constexpr int kParamTileDF = 384;
-
-struct alignas(16) Bez
-{
-    double c[12];
-};
 
 // G7-K15 abscissae and weights: the published Gauss-Kronrod constants at the precision the reference carries
 // (integrate_gk15.hh:13-36); identical doubles make the sums identical.
@@ -170,8 +166,8 @@ __global__ void k_bernstein(double2* __restrict__ table)
 
 // ---- double-float form ----------------------------------------------------------------------------------------
 // The same integrand and panel rule in double-float arithmetic (df32.cuh, ~44 significant bits on the FP32 pipe):
-// the curve relative to the query in power form about t = 1/2 (power_about_half) and w - d_eta in the closed form
-// below -- the same quantities in fewer operations.  Not bit-identical to the reference (the value differs in the
+// the curve relative to the query in power form about t = 1/2 (k_curves_df), in the frame of x0, and w - d_eta in
+// the closed form below -- the same quantities in fewer operations.  Not bit-identical to the reference (the value differs in the
 // last ~1e-13 relative, and a panel whose |Ik - Ig| sits at the tolerance can be decided the other way); the tree
 // rule, the tolerances and the summation order are the plain integrator's.
 struct alignas(16) CurveDF
@@ -209,8 +205,18 @@ __device__ __forceinline__ df df_mulf(df a, float f)
     return fast_two_sum(p.hi, __fmaf_rn(a.lo, f, p.lo));
 }
 
-// w(t) - d_eta(t) with cp = the curve's control points minus the query, in closed form.  The plain kernel evaluates
-// the reference's expression (integrand, gwn_parametric.hh:73-103): with G = r / |r|, G' its derivative, a = x0.G,
+// The frame of the double-float form: x0 along +z (rows e1, e2, x0 / |x0|).  Curves and queries are rotated into it in
+// FP64 once per call, before their rounding to double-float.
+struct FrameDF
+{
+    double r[9];
+    df len;   // |x0|
+    df scale; // (|x0|^2 - 2) |x0|^2
+    bool unit;
+};
+
+// w(t) - d_eta(t) in closed form.  The exact kernel evaluates the reference's expression (integrand,
+// gwn_parametric.hh:73-103): with G = r / |r|, G' its derivative, a = x0.G,
 // X = x0 - G a, X' = -(G (x0.G') + G' a), v = G - x0 a, v' = G' - x0 (x0.G'), d_eta = G.(X x X') / |X|^2 and
 // w = -x0.(v x v') / |v|^2.  Expanding (G x G = 0, G.(G x G') = 0, |G| = 1): G.(X x X') = a c and
 // x0.(v x v') = c with c = x0.(G x G'), |X|^2 = n - a^2 = |x0 x G|^2 (Lagrange's identity) and
@@ -219,65 +225,52 @@ __device__ __forceinline__ df df_mulf(df a, float f)
 //   w - d_eta = -T / (q + (n - 2) m^2) - m T / (s |x0 x r|^2),
 // and for a unit x0 (n = 1 to double precision) -T / (s (s - m)), free of the two terms' cancellation near
 // m = -s.  Near m = s (the curve crossing the ray of x0 from the query) s - m, formed by subtraction, would keep
-// only the square of the angle's relative precision; there it is |x0 x r|^2 / (s + m), whose cross product keeps
-// the angle's own.  For a unit x0: one square root and one quotient, against the expression's square root and three
+// only the square of the angle's relative precision; there it is |x0 x r|^2 / (s + m), whose squares keep the
+// angle's own.  For a unit x0: one square root and one quotient, against the expression's square root and three
 // quotients.
-// pc: the pair's curve minus its query as power coefficients about t = 1/2 (power_about_half), dl = t - 1/2.
-__device__ __forceinline__ df integrand_df(const df (&pc)[12], df3 x0, df x0n, bool unit, df dl)
+//
+// In the frame with x0 = |x0| z these are two-term forms: m = |x0| z, T = |x0| (x y' - y x'), |x0 x r|^2 = n (x^2 + y^2),
+// and z' is not needed.  With the fused chains of df32.cuh a node takes about 320 FP32 operations; with x0's three
+// coordinates and separate products and sums it took about 660 (20,000 queries x 1,024 curves at tol 1e-10: 57.9 -> 26.2
+// ms).  Errors against the exact form did not grow: p50 4.2e-15 -> 2.9e-15, p99 2.6e-11 -> 1.9e-11, p99.9 3.8e-10 ->
+// 2.7e-10 over 4 x 30,000 queries, 30% of them within 1e-3 of a curve.
+// pc: the pair's curve minus its query as power coefficients about t = 1/2 (k_curves_df), dl = t - 1/2.
+__device__ __forceinline__ df integrand_df(const df (&pc)[12], FrameDF const& F, df dl)
 {
-    // r = a0 + dl (a1 + dl (a2 + dl a3)) and r' = a1 + dl (2 a2 + 3 dl a3), per coordinate
-    df r3[3], dr3[3];
+    // r = a0 + dl (a1 + dl (a2 + dl a3)) by Horner's rule, and r' = a1 + dl (2 a2 + 3 dl a3) from its partial sums
+    df r[3], d[2];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
     {
-        df const a3d = pc[9 + c] * dl;
-        r3[c] = pc[c] + dl * (pc[3 + c] + dl * (pc[6 + c] + a3d));
-        dr3[c] = pc[3 + c] + dl * (df_scale(pc[6 + c], 2.f) + df_mulf(a3d, 3.f));
+        df const t2 = df_fma(dl, pc[9 + c], pc[6 + c]);
+        df const t1 = df_fma(dl, t2, pc[3 + c]);
+        r[c] = df_fma(dl, t1, pc[c]);
+        if (c < 2)
+            d[c] = df_fma(dl, df_fma(dl, pc[9 + c], t2), t1);
     }
-    df3 const r{r3[0], r3[1], r3[2]}, dr{dr3[0], dr3[1], dr3[2]};
-    df const q = dot(r, r);
+    df const rho = df_dot2(r[0], r[0], r[1], r[1]);
+    df const q = df_fma(r[2], r[2], rho);
     df const s = df_sqrt(q);
-    df3 const xr = cross(x0, r);
-    df const T = dot(dr, xr), m = dot(x0, r);
-    if (unit)
+    df const T = df_det2(r[0], d[1], r[1], d[0]);
+    if (F.unit)
     {
-        bool const behind = m.hi < 0.f;
-        df const num = behind ? T : T * (s + m);
-        df const den = s * (behind ? s - m : dot(xr, xr));
-        return df_neg(num / den);
+        bool const behind = r[2].hi < 0.f;
+        // s + |z|: s - m behind, s + m in front
+        df const sm = df_add_ordered(s, behind ? df_neg(r[2]) : r[2]);
+        df const num = T * sm;
+        df const den = s * df{behind ? sm.hi : rho.hi, behind ? sm.lo : rho.lo};
+        return df_neg(df{behind ? T.hi : num.hi, behind ? T.lo : num.lo} / den);
     }
-    return df_neg(T / (q + (x0n - df_make(2.f)) * (m * m))) - (m * T) / (s * dot(xr, xr));
+    return df_neg(F.len * T / df_fma(F.scale, r[2] * r[2], q)) - (r[2] * T) / (s * rho);
 }
 
-// Control points c0..c3 (minus the query) to power coefficients about t = 1/2, in place: with s03 = c0 + c3,
-// s12 = c1 + c2, d30 = c3 - c0 and d21 = c2 - c1, r(1/2) = (s03 + 3 s12) / 8, r'(1/2) = 3/4 (d30 + d21),
-// r''(1/2) / 2 = 3/2 (s03 - s12) and r''' / 6 = d30 - 3 d21.  Evaluated at |t - 1/2| <= 1/2 the power form rounds
-// a little worse than the Bernstein form (in FP32 on bicubic patch boundaries, relative error of r: median 1.2x at
-// random pairs with a lower maximum, median 1.7x and p99 2.1x for queries 1e-4 to 1e-2 from a curve near their
-// closest point), and takes 12 double-float products, 3 products by a float and 15 sums per node against the
-// Bernstein form's 31, 5 and 21.
-__device__ __forceinline__ void power_about_half(df (&cp)[12])
-{
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-    {
-        df const s03 = cp[c] + cp[9 + c], s12 = cp[3 + c] + cp[6 + c];
-        df const d30 = cp[9 + c] - cp[c], d21 = cp[6 + c] - cp[3 + c];
-        cp[c] = df_scale(s03 + df_mulf(s12, 3.f), 0.125f);
-        cp[3 + c] = df_mulf(d30 + d21, 0.75f);
-        cp[6 + c] = df_mulf(s03 - s12, 1.5f);
-        cp[9 + c] = d30 - df_mulf(d21, 3.f);
-    }
-}
-
-__device__ __forceinline__ double gk15_panel_df(const df (&pc)[12], df3 x0, df x0n, bool unit, int depth, uint32_t j,
-                                                float* err)
+__device__ __forceinline__ double gk15_panel_df(const df (&pc)[12], FrameDF const& F, int depth, uint32_t j, float* err)
 {
     float const scale = ldexpf(1.f, -depth);
     float const h = 0.5f * scale;
-    // the centre (j + 1/2) 2^-depth less 1/2, exact: j 2^-depth - 1/2 is a multiple of 2^-depth below 1 in magnitude
-    df const cc = two_sum(__fmaf_rn(float(j), scale, -0.5f), h);
-    df const f0 = integrand_df(pc, x0, x0n, unit, cc);
+    // the centre (j + 1/2) 2^-depth less 1/2: a multiple of 2^-(depth + 1) below 1/2 in magnitude, so a float exactly
+    float const cc = __fadd_rn(__fmaf_rn(float(j), scale, -0.5f), h);
+    df const f0 = integrand_df(pc, F, df_make(cc));
     // the Kronrod and Gauss sums accumulated node pair by node pair, in the order of the sums above (the same
     // values), so no node value stays live
     df ig = kGkWgdf[0] * f0;
@@ -286,21 +279,53 @@ __device__ __forceinline__ double gk15_panel_df(const df (&pc)[12], df3 x0, df x
     for (int k = 1; k <= 7; ++k)
     {
         df const dx = df_scale(kGkXdf[k], h);
-        df const s = integrand_df(pc, x0, x0n, unit, cc - dx) + integrand_df(pc, x0, x0n, unit, cc + dx);
-        ik = ik + kGkWkdf[k] * s;
+        df const up = two_sum(cc, dx.hi), dn = two_sum(cc, -dx.hi);
+        df const s = integrand_df(pc, F, fast_two_sum(dn.hi, __fsub_rn(dn.lo, dx.lo))) +
+                     integrand_df(pc, F, fast_two_sum(up.hi, __fadd_rn(up.lo, dx.lo)));
+        ik = df_fma(kGkWkdf[k], s, ik);
         if ((k & 1) == 0)
-            ig = ig + kGkWgdf[k >> 1] * s;
+            ig = df_fma(kGkWgdf[k >> 1], s, ig);
     }
     df const diff = df_scale(ik - ig, h);
     *err = fabsf(diff.hi + diff.lo);
     return df_to(df_scale(ik, h));
 }
 
-__global__ void k_curves_df(const double* __restrict__ curves, int64_t n_curves, CurveDF* __restrict__ out)
+// Queries in the frame, as double-float coordinates.
+__global__ void k_queries_df(const double* __restrict__ pts, int64_t n, FrameDF F, df* __restrict__ out)
 {
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < 12 * n_curves;
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+    {
+        double const x = pts[3 * i], y = pts[3 * i + 1], z = pts[3 * i + 2];
+        for (int c = 0; c < 3; ++c)
+            out[3 * i + c] = df_from(F.r[3 * c] * x + F.r[3 * c + 1] * y + F.r[3 * c + 2] * z);
+    }
+}
+
+// Curves in the frame, as power coefficients about t = 1/2: with s03 = c0 + c3, s12 = c1 + c2, d30 = c3 - c0 and
+// d21 = c2 - c1, r(1/2) = (s03 + 3 s12) / 8, r'(1/2) = 3/4 (d30 + d21), r^(2)(1/2) / 2 = 3/2 (s03 - s12) and
+// r^(3) / 6 = d30 - 3 d21, formed in FP64 and rounded to double-float once.  A query enters r(1/2) only, so a pair
+// subtracts three coordinates.  (Evaluated at |t - 1/2| <= 1/2 the power form rounds a little worse than the Bernstein
+// form: in FP32 on bicubic patch boundaries, relative error of r, median 1.2x at random pairs with a lower maximum,
+// median 1.7x and p99 2.1x for queries 1e-4 to 1e-2 from a curve near their closest point.)
+__global__ void k_curves_df(const double* __restrict__ curves, int64_t n_curves, FrameDF F, CurveDF* __restrict__ out)
+{
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < 3 * n_curves;
          i += int64_t(gridDim.x) * blockDim.x)
-        out[i / 12].c[i % 12] = df_from(curves[i]);
+    {
+        int64_t const k = i / 3;
+        int const c = int(i - 3 * k);
+        const double* const v = curves + 12 * k;
+        double p[4];
+        for (int e = 0; e < 4; ++e)
+            p[e] = F.r[3 * c] * v[3 * e] + F.r[3 * c + 1] * v[3 * e + 1] + F.r[3 * c + 2] * v[3 * e + 2];
+        double const s03 = p[0] + p[3], s12 = p[1] + p[2], d30 = p[3] - p[0], d21 = p[2] - p[1];
+        df* const o = out[k].c + c;
+        o[0] = df_from(0.125 * (s03 + 3.0 * s12));
+        o[3] = df_from(0.75 * (d30 + d21));
+        o[6] = df_from(1.5 * (s03 - s12));
+        o[9] = df_from(d30 - 3.0 * d21);
+    }
 }
 
 // Optional work of the integrator kernel.
@@ -535,9 +560,9 @@ constexpr int param_min_blocks()
     return !PANEL ? 6 : 1; // the double-float panels in 80 registers (no spills), six blocks per SM
 }
 template <bool PANEL>
-__global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>()) k_param_gk15(const double* __restrict__ pos, int64_t n,
-                                                            double* __restrict__ out, double x0x, double x0y,
-                                                            double x0z, const Bez* __restrict__ curves,
+__global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>()) k_param_gk15(const df* __restrict__ pos, int64_t n,
+                                                            double* __restrict__ out, FrameDF F,
+                                                            const CurveDF* __restrict__ curves,
                                                             int64_t n_curves, int tile, int min_depth, int max_depth,
                                                             double tol, const uint8_t* __restrict__ start_depth,
                                                             uint32_t* __restrict__ stats,
@@ -549,15 +574,11 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>()) k_para
     __shared__ __align__(8) uint64_t bar;
     __shared__ int s_next;
     __shared__ int s_nodes[kParamBlock];
-    Bez* const buf = reinterpret_cast<Bez*>(smem);
-    PanelSmem* const ps = reinterpret_cast<PanelSmem*>(smem + size_t(tile) * sizeof(Bez));
+    CurveDF* const buf = reinterpret_cast<CurveDF*>(smem);
+    PanelSmem* const ps = reinterpret_cast<PanelSmem*>(smem + size_t(tile) * sizeof(CurveDF));
     bool const use_panel = PANEL && ex.pwb != nullptr;
     unsigned long long skips = 0;
     double* const slab = pair_vals + size_t(blockIdx.x) * kParamBlock * tile;
-    df3 const x0df{df_from(x0x), df_from(x0y), df_from(x0z)};
-    double const x0n = x0x * x0x + x0y * x0y + x0z * x0z;
-    bool const x0_unit = fabs(x0n - 1.0) <= 1e-15;
-    df const x0n_df = df_from(x0n);
     int64_t const n_blocks_q = (n + kParamBlock - 1) / kParamBlock;
     int const n_tiles = int((n_curves + tile - 1) / tile);
     int const tiles_per_group = (n_tiles + n_groups - 1) / n_groups;
@@ -570,7 +591,7 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>()) k_para
         tol_at[l] = __dmul_rn(tol_at[l - 1], 0.5);
     if (use_panel)
         load_weights(ps->w, ex.pwb, ex.pparams);
-    float3 const x0f = make_float3(float(x0x), float(x0y), float(x0z));
+    float3 const x0f = make_float3(0.f, 0.f, F.len.hi);
     int const warp = int(threadIdx.x >> 5);
     if (threadIdx.x == 0)
     {
@@ -597,7 +618,7 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>()) k_para
             if (threadIdx.x == 0)
             {
                 s_next = 0;
-                unsigned const bytes = unsigned(cnt) * unsigned(sizeof(Bez));
+                unsigned const bytes = unsigned(cnt) * unsigned(sizeof(CurveDF));
                 mbar_arrive_expect_tx(&bar, bytes);
                 bulk_copy_g2s(buf, curves + c0, bytes, &bar);
             }
@@ -610,7 +631,6 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>()) k_para
             bool drained = false;
             int k = 0, ql = 0, s = 0, d = 0, leaves = 0, dmin = 0, dmax = 0, pnodes = 0;
             uint32_t j = 0;
-            ev3<rd> p{};
             df cp[12]; // this pair's curve minus its query, as power coefficients about t = 1/2
             double pending[kParamMaxDepth + 1];
             for (;;)
@@ -632,13 +652,11 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>()) k_para
                             k = mine / nq;
                             ql = mine - k * nq;
                             int64_t const q = q0 + ql;
-                            p = ev3<rd>{rd(pos[3 * q]), rd(pos[3 * q + 1]), rd(pos[3 * q + 2])};
-                            df const pd[3] = {df_from(p.x.v), df_from(p.y.v), df_from(p.z.v)};
-                            CurveDF const& cv = reinterpret_cast<const CurveDF*>(buf)[k];
+                            df const pd[3] = {pos[3 * q], pos[3 * q + 1], pos[3 * q + 2]};
+                            CurveDF const& cv = buf[k];
 #pragma unroll
                             for (int e = 0; e < 12; ++e)
-                                cp[e] = cv.c[e] - pd[e % 3];
-                            power_about_half(cp);
+                                cp[e] = e < 3 ? cv.c[e] - pd[e] : cv.c[e];
                             s = start_depth ? min(int(start_depth[q * n_curves + c0 + k]), max_depth) : 0;
                             d = s;
                             j = 0;
@@ -660,13 +678,20 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>()) k_para
                     float f[kF];
                     if (cand)
                     {
-                        // the control points minus the query, as the network was trained on them
-                        df const pd[3] = {df_from(p.x.v), df_from(p.y.v), df_from(p.z.v)};
-                        CurveDF const& cv = reinterpret_cast<const CurveDF*>(buf)[k];
+                        // the control points minus the query, as the network was trained on them: a0 -+ a1/2 + a2/4
+                        // -+ a3/8 at the ends, a0 -+ a1/6 - a2/12 +- a3/8 between
                         float cpf[12];
 #pragma unroll
-                        for (int e = 0; e < 12; ++e)
-                            cpf[e] = (cv.c[e] - pd[e % 3]).hi;
+                        for (int e = 0; e < 3; ++e)
+                        {
+                            df const o1 = df_mulf(cp[3 + e], 1.f / 6.f), e2 = df_mulf(cp[6 + e], 1.f / 12.f);
+                            df const end = cp[e] + df_scale(cp[6 + e], 0.25f), mid = cp[e] - e2;
+                            df const a3 = df_scale(cp[9 + e], 0.125f), odd = df_scale(cp[3 + e], 0.5f) + a3;
+                            cpf[e] = (end - odd).hi;
+                            cpf[3 + e] = (mid - o1 + a3).hi;
+                            cpf[6 + e] = (mid + o1 - a3).hi;
+                            cpf[9 + e] = (end + odd).hi;
+                        }
                         panel_features(cpf, d, j, x0f, ex.log10_tol, f);
                     }
                     else
@@ -715,7 +740,7 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>()) k_para
                 if (pi < 0)
                     continue;
                 float e32;
-                double v = gk15_panel_df(cp, x0df, x0n_df, x0_unit, d, j, &e32);
+                double v = gk15_panel_df(cp, F, d, j, &e32);
                 double const err = double(e32);
                 ++pnodes;
                 bool const accept = d >= max_depth || (d >= min_depth && err <= tol_at[d]);
@@ -880,14 +905,13 @@ int param_run(Context& ctx, const double* d_pos, int64_t n, double* d_out, const
     if (!dfm)
         return param_run_exact(ctx, d_pos, n, d_out, x0, d_curves, n_curves, min_depth, max_depth, tol, d_start,
                                d_stats, d_nodes, ex);
-    static_assert(sizeof(CurveDF) == sizeof(Bez), "both curve forms stage through the same tile");
     auto const kern = panel ? k_param_gk15<true> : k_param_gk15<false>;
     int tile = int(std::min<int64_t>(kParamTileDF, n_curves));
     size_t smem = 0;
     int per_sm = 0;
     auto shape = [&](int t) -> int
     {
-        smem = size_t(t) * sizeof(Bez) + (panel ? sizeof(PanelSmem) : 0);
+        smem = size_t(t) * sizeof(CurveDF) + (panel ? sizeof(PanelSmem) : 0);
         AGWN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
         AGWN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kParamBlock, smem));
         if (per_sm < 1)
@@ -927,17 +951,33 @@ int param_run(Context& ctx, const double* d_pos, int64_t n, double* d_out, const
         if (d_nodes)
             AGWN_TRY_CUDA(cudaMemsetAsync(d_nodes, 0, sizeof(int32_t) * n, ctx.stream));
     }
-    void* cdf = nullptr;
-    AGWN_TRY(ctx.scratch_reserve(S_FRAME, sizeof(CurveDF) * size_t(n_curves), &cdf));
+    // curves and queries in the frame of x0, as double-floats
+    FrameDF F;
+    {
+        Frame64 const f = ray_frame(x0);
+        double const n2 = x0[0] * x0[0] + x0[1] * x0[1] + x0[2] * x0[2], len = std::sqrt(n2);
+        auto const split = [](double v) { return df{float(v), float(v - double(float(v)))}; };
+        for (int k = 0; k < 9; ++k)
+            F.r[k] = f.r[k];
+        F.len = split(len);
+        F.scale = split((n2 - 2.0) * n2);
+        F.unit = std::fabs(n2 - 1.0) <= 1e-15;
+    }
+    CurveDF* cdf = nullptr;
+    AGWN_TRY(ctx.scratch_reserve(S_FRAME, sizeof(CurveDF) * size_t(n_curves) + sizeof(df) * 3 * size_t(n),
+                                 reinterpret_cast<void**>(&cdf)));
+    df* const qdf = reinterpret_cast<df*>(cdf + n_curves);
     AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-    k_curves_df<<<int(std::min<int64_t>(div_up(12 * n_curves, 256), 4 * ctx.sm_count)), 256, 0, ctx.stream>>>(
-        d_curves, n_curves, static_cast<CurveDF*>(cdf));
+    k_curves_df<<<int(std::min<int64_t>(div_up(3 * n_curves, 256), 4 * ctx.sm_count)), 256, 0, ctx.stream>>>(
+        d_curves, n_curves, F, cdf);
+    AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
+    AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
+    k_queries_df<<<int(std::min<int64_t>(div_up(n, 256), 4 * ctx.sm_count)), 256, 0, ctx.stream>>>(d_pos, n, F, qdf);
     AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
     AGWN_TRY(ctx.launch_begin(AGWN_K_PARAMETRIC));
-    kern<<<grid, kParamBlock, smem, ctx.stream>>>(d_pos, n, d_out, x0[0], x0[1], x0[2],
-                                                 static_cast<const Bez*>(cdf), n_curves, tile, min_depth,
-                                                 max_depth, tol, d_start, d_stats, d_nodes, pair_vals, ctx.d_flags,
-                                                 ex, n_groups, partial);
+    kern<<<grid, kParamBlock, smem, ctx.stream>>>(qdf, n, d_out, F, cdf, n_curves, tile,
+                                                 min_depth, max_depth, tol, d_start, d_stats, d_nodes, pair_vals,
+                                                 ctx.d_flags, ex, n_groups, partial);
     AGWN_TRY(ctx.launch_end(AGWN_K_PARAMETRIC));
     if (n_groups == 1)
         return AGWN_OK;
