@@ -75,7 +75,7 @@ enum scratch_slot
     S_MISC1 = 7,
     S_MISC2 = 8,
     S_MISC3 = 9,
-    S_PARTIAL = 10, // the parametric integrator's per-group partial sums
+    S_PARTIAL = 10, // the parametric integrator's per-group partial sums; the split exact kernel's terms
     S_ORDER0 = 11,  // the spatial order of the queries: sort keys, indices, digit counters (order.cu)
     S_ORDER1 = 12,  // the queries in that order and their outputs
     S_COUNT = 13
@@ -141,6 +141,8 @@ struct Context
     long long* d_counters = nullptr; // kCounters: [0] fp64 pairs, [1] pairs, [2] parametric skips, [3] certified pairs, [4..7] integer, [8..11] patches
                                      // term: queries, cell-list entries, candidate leaves, exact tests
     DevBuf scratch[S_COUNT];
+    static constexpr int kArrivals = 2048;
+    int* d_arrivals = nullptr; // kArrivals zeroed counters, left zeroed by each kernel that uses them
     int sm_count = 0;
     RayCache ray_cache;
     DevBuf bernstein; // the exact parametric integrator's node bases (param.cu), filled on first use

@@ -261,6 +261,10 @@ int agwn_context_create(int device, void* stream, agwn_context** out)
             break;
         if ((e = cudaMemset(ctx->d_counters, 0, sizeof(long long) * kCounters)) != cudaSuccess)
             break;
+        if ((e = cudaMalloc(&ctx->d_arrivals, sizeof(int) * Context::kArrivals)) != cudaSuccess)
+            break;
+        if ((e = cudaMemset(ctx->d_arrivals, 0, sizeof(int) * Context::kArrivals)) != cudaSuccess)
+            break;
         if ((e = cudaMallocHost(&ctx->h_flags, sizeof(int) * FLAG_COUNT)) != cudaSuccess)
             break;
         if ((e = cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess)
@@ -300,6 +304,8 @@ int agwn_context_destroy(agwn_context* ctx)
         cudaFree(ctx->d_flags);
     if (ctx->d_counters)
         cudaFree(ctx->d_counters);
+    if (ctx->d_arrivals)
+        cudaFree(ctx->d_arrivals);
     if (ctx->h_flags)
         cudaFreeHost(ctx->h_flags);
     for (cudaEvent_t e : ctx->pipe_ev)

@@ -73,6 +73,8 @@ struct FracPlan
 {
     int64_t n_seg = 0;
     bool mixed = false;
+    const T* raw = nullptr; // the boundary as given, for split launches (fractional_split)
+    bool split_only = false; // every launch of the plan is split: no exact segments were prepared
     int tile = 0;     // segments (exact) or entries (mixed) per shared-memory tile
     int nbuf = 1;     // shared-memory buffers
     T x0[3] = {};
@@ -83,6 +85,13 @@ struct FracPlan
     SegX<double>* seg64 = nullptr;
     Frame* frame = nullptr;
 };
+
+// Whether n queries of the exact form are shared out by segment (k_frac_exact_split): fewer than 8 warps of queries per
+// SM, below which a query per thread leaves the FP64 pipes idle.
+bool split_queries(Context const& ctx, int64_t n)
+{
+    return n < int64_t(32) * std::min(8 * ctx.sm_count, Context::kArrivals);
+}
 
 // n_queries: the queries the plan will serve.  On a boundary shorter than 32 segments, or below ctx.mixed_min_pairs
 // (query, segment) pairs, the mixed mode runs the exact kernels (Context::use_mixed: there they are the faster ones,
@@ -109,6 +118,10 @@ int fractional_prepare(Context& ctx, const T* x0_host, const T* d_seg_raw, int64
               sizeof(T) == 8;
     if (!p.mixed)
     {
+        p.raw = d_seg_raw;
+        p.split_only = split_queries(ctx, n_queries);
+        if (p.split_only)
+            return AGWN_OK;
         p.tile = int(std::min<int64_t>(ctx.seg_tile, n_seg));
         p.nbuf = n_seg > p.tile ? 2 : 1;
         AGWN_TRY(ctx.scratch_reserve(S_SEGS, sizeof(SegX<T>) * n_seg, reinterpret_cast<void**>(&p.seg)));
@@ -158,6 +171,30 @@ template <class T, class FB>
 int fractional_launch_mixed(Context& ctx, const FracPlan<T>& p, const double* d_pos, int64_t n, double* d_out,
                             const int32_t* d_counts, FB fb);
 
+// The exact form shared out by segment: units of g segments so that there are 16 warps per SM or more, in passes over
+// the boundary of at most 64 MB of terms.
+template <class T>
+int fractional_split(Context& ctx, const FracPlan<T>& p, const T* d_pos, int64_t n, T* d_out, const int32_t* d_counts)
+{
+    int64_t const groups = div_up(n, 32);
+    int64_t const pass = std::min<int64_t>(p.n_seg, std::max<int64_t>(1, (int64_t(1) << 26) / (n * int64_t(sizeof(T)))));
+    T* terms = nullptr;
+    AGWN_TRY(ctx.scratch_reserve(S_PARTIAL, sizeof(T) * size_t(pass) * size_t(n), reinterpret_cast<void**>(&terms)));
+    for (int64_t s0 = 0; s0 < p.n_seg; s0 += pass)
+    {
+        int const ns = int(std::min(pass, p.n_seg - s0));
+        int64_t const per_unit = groups * ns / (16 * int64_t(ctx.sm_count));
+        int const g = int(std::max<int64_t>({1, per_unit, div_up(ns, 65535 * kSplitWarps)}));
+        dim3 const grid{unsigned(groups), unsigned(div_up(ns, int64_t(g) * kSplitWarps))};
+        AGWN_TRY(ctx.launch_begin(AGWN_K_FRACTIONAL));
+        k_frac_exact_split<T><<<grid, 32 * kSplitWarps, 0, ctx.stream>>>(
+            d_pos, int(n), d_out, d_counts, p.x0[0], p.x0[1], p.x0[2], p.raw + 7 * s0, ns, g, terms, ctx.d_arrivals,
+            s0 == 0, s0 + ns == p.n_seg);
+        AGWN_TRY(ctx.launch_end(AGWN_K_FRACTIONAL));
+    }
+    return AGWN_OK;
+}
+
 template <class T>
 int fractional_launch(Context& ctx, const FracPlan<T>& p, const T* d_pos, int64_t n, T* d_out,
                       const int32_t* d_counts)
@@ -171,12 +208,18 @@ int fractional_launch(Context& ctx, const FracPlan<T>& p, const T* d_pos, int64_
                                                                                                       n);
         return ctx.launch_end(AGWN_K_FRACTIONAL);
     }
-    int const K = ctx.queries_per_thread;
-    int const block = ctx.frac_block ? ctx.frac_block : 128;
-    int64_t const per_tile = int64_t(block) * K;
-    int64_t const n_qtiles = (n + per_tile - 1) / per_tile;
+    if (!p.mixed && (p.split_only || split_queries(ctx, n)))
+        return fractional_split<T>(ctx, p, d_pos, n, d_out, d_counts);
     if (!p.mixed)
     {
+        // Doubles below 2^20 queries: one query per thread in blocks of 64.  The FP64 pipe is full from 8 warps, and
+        // the SMs' shares then differ by a small block (100,000 queries x 4 segments: 78 -> 73 us).  In float, two
+        // queries per thread hide the chain of one (884,736 queries x 102 segments: 412 us with one, 393 with two).
+        bool const small = sizeof(T) == 8 && n < int64_t(1) << 20;
+        int const K = small ? 1 : ctx.queries_per_thread;
+        int const block = ctx.frac_block ? ctx.frac_block : (small ? 64 : 128);
+        int64_t const per_tile = int64_t(block) * K;
+        int64_t const n_qtiles = (n + per_tile - 1) / per_tile;
         size_t const smem = size_t(p.nbuf) * p.tile * sizeof(SegX<T>);
         auto launch = [&](auto kern) -> int
         {

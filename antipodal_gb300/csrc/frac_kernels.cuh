@@ -203,6 +203,62 @@ __global__ void __launch_bounds__(256) k_frac_exact(const T* __restrict__ pos, i
     }
 }
 
+// The exact form for few queries: the (query, segment) terms of 32 queries are shared out over warps and blocks, and the
+// block that finishes a query group last adds its terms in segment order, so the values are k_frac_exact's.  Block
+// (x, y): the queries 32 x .. 32 x + 31, its warp w the segments [g (4 y + w), + g) of [0, n_seg).  terms: n_seg x n;
+// arrivals: one zeroed counter per query group, left zeroed.  first / last: whether the sums start here (else they
+// continue from out) and whether they are normalised and given their counts.
+//
+// FP64 issue bounds a full SM (about 60 instructions of 16 clocks per 32 terms), which takes 8 warps or so; with a
+// query per thread, 257 queries x 24 segments kept 2 SMs busy (the whole call 185 -> 55 us).
+constexpr int kSplitWarps = 4;
+template <class T>
+__global__ void __launch_bounds__(32 * kSplitWarps)
+    k_frac_exact_split(const T* __restrict__ pos, int n, T* out, const int32_t* __restrict__ counts, T x0x, T x0y,
+                       T x0z, const T* __restrict__ raw, int n_seg, int g, T* terms, int* arrivals, bool first,
+                       bool last)
+{
+    using S = typename exact_of<T>::type;
+    __shared__ bool s_sum;
+    int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int const i = int(blockIdx.x) * 32 + lane, ii = min(i, n - 1);
+    ev3<S> const x1{S(-x0x), S(-x0y), S(-x0z)};
+    ev3<S> const p{S(pos[3 * ii]), S(pos[3 * ii + 1]), S(pos[3 * ii + 2])};
+    int const s0 = min((int(blockIdx.y) * kSplitWarps + warp) * g, n_seg), s1 = min(s0 + g, n_seg);
+    for (int s = s0; s < s1; ++s)
+    {
+        const T* const r = raw + 7 * size_t(s);
+        ev3<S> const v0 = ev3<S>{S(__ldg(r)), S(__ldg(r + 1)), S(__ldg(r + 2))} - p;
+        ev3<S> const v1 = ev3<S>{S(__ldg(r + 3)), S(__ldg(r + 4)), S(__ldg(r + 5))} - p;
+        S const term = S(__ldg(r + 6)) * S(vos_exact(x1, v0, v1));
+        if (i < n)
+            terms[size_t(s) * n + i] = term.v;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        s_sum = atomicAdd(arrivals + blockIdx.x, 1) == int(gridDim.y) - 1;
+        if (s_sum)
+            arrivals[blockIdx.x] = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_sum || warp != 0 || i >= n)
+        return;
+    S area = first ? S(T(0)) : S(out[i]);
+#pragma unroll 8
+    for (int s = 0; s < n_seg; ++s)
+        area = area + S(__ldcg(terms + size_t(s) * n + i));
+    if (last)
+    {
+        area = area / S(T(2) * kPi<T>);
+        if (counts)
+            area = area + S(T(counts[i]));
+    }
+    out[i] = area.v;
+}
+
 // --------------------------------------------------------------------------------------------------------------
 // mixed form
 // --------------------------------------------------------------------------------------------------------------
