@@ -117,6 +117,31 @@ AGWN_FN float lead_float(uint32_t h, uint32_t l)
     return float_of_bits((((h << 3) | (l >> 29)) & 0x007fffffu) | 0x3f800000u);
 }
 
+// Integers as doubles by their bits, exact: |v| < 2^32, and |v| < 2^53.  (The conversion instructions run at the FP64
+// rate.)
+AGWN_FN uint32_t leading_zeros(uint32_t v)
+{
+#ifdef __CUDACC__
+    return uint32_t(__clz(int(v)));
+#else
+    return v ? uint32_t(__builtin_clz(v)) : 32u;
+#endif
+}
+AGWN_FN double double_of(int32_t v)
+{
+    uint32_t const m = v < 0 ? 0u - uint32_t(v) : uint32_t(v), z = leading_zeros(m);
+    uint32_t const t = z < 32 ? m << z : 0u; // the leading one at bit 31
+    uint32_t const h = (t >> 11) + ((1053u - z) << 20) + (uint32_t(v) & 0x80000000u);
+    return of_bits(m ? (uint64_t(h) << 32) | (t << 21) : 0ull);
+}
+AGWN_FN double double_of_53(int64_t v)
+{
+    uint64_t const m = v < 0 ? 0ull - uint64_t(v) : uint64_t(v);
+    uint32_t const h = uint32_t(m >> 32), z = h ? leading_zeros(h) : 32 + leading_zeros(uint32_t(m));
+    uint64_t const t = m << (z & 63u); // the leading one at bit 63
+    return of_bits(m ? (t >> 11) + (uint64_t(1085u - z) << 52) + (uint64_t(v) & 0x8000000000000000ull) : 0ull);
+}
+
 // a / b, rounded to nearest even.
 //
 // With A, B the 53-bit significands, the quotient A / B in (1/2, 2) is built in units of 2^-55 as

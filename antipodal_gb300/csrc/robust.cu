@@ -306,6 +306,29 @@ int robust_run(Context& ctx, const Robust& r, const T* d_pos, int64_t n, T* d_ou
     }
     // the mixed form (int64_grid only) walks the vertex chains built with the evaluator
     bool const mixed = std::is_same_v<P, P64> && ctx.robust_mode == AGWN_ROBUST_MIXED && r.chain != nullptr;
+    if (!mixed && r.n_seg > 0 && n < int64_t(32) * std::min(8 * ctx.sm_count, Context::kArrivals))
+    {
+        // fewer than 8 warps of queries per SM: shared out by segment, in units that give 16 warps per SM or more and
+        // passes of at most 64 MB of terms (as the mesh functions' exact form, frac.cu)
+        int64_t const groups = div_up(n, 32);
+        int64_t const pass = std::min<int64_t>(r.n_seg, std::max<int64_t>(1, (int64_t(1) << 26) / (n * 8)));
+        double* terms = nullptr;
+        AGWN_TRY(ctx.scratch_reserve(S_PARTIAL, sizeof(double) * size_t(pass + 1) * size_t(n),
+                                     reinterpret_cast<void**>(&terms)));
+        for (int64_t s0 = 0; s0 < r.n_seg; s0 += pass)
+        {
+            int const ns = int(std::min(pass, r.n_seg - s0));
+            int64_t const per_unit = groups * ns / (16 * int64_t(ctx.sm_count));
+            int const g = int(std::max<int64_t>({1, per_unit, div_up(ns, 65535 * kSplitWarps)}));
+            dim3 const grid{unsigned(groups), unsigned(div_up(ns, int64_t(g) * kSplitWarps))};
+            AGWN_TRY(ctx.launch_begin(AGWN_K_ROBUST));
+            k_robust_frac_split<T, P><<<grid, 32 * kSplitWarps, 0, st>>>(
+                d_pos, int(n), qz, static_cast<const Seg*>(r.seg) + s0, ns, g, d_counts, d_out, d_frac, terms,
+                terms + size_t(pass) * size_t(n), ctx.d_arrivals, s0 == 0, s0 + ns == r.n_seg);
+            AGWN_TRY(ctx.launch_end(AGWN_K_ROBUST));
+        }
+        return AGWN_OK;
+    }
     int64_t const n_elem = mixed ? r.n_entries : r.n_seg;
     int const tile = int(std::max<int64_t>(1, std::min<int64_t>(ctx.seg_tile, n_elem)));
     int const n_tiles = int((n_elem + tile - 1) / tile);
@@ -315,14 +338,16 @@ int robust_run(Context& ctx, const Robust& r, const T* d_pos, int64_t n, T* d_ou
         if (mixed)
             kern = k_robust_frac<T, P, true>;
     AGWN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    // the exact form's FP64 pipe is full from 8 warps, and small blocks even out the SMs' shares
+    int const block = mixed ? kRobBlock : 64;
     int per_sm = 0;
-    AGWN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kRobBlock, smem));
+    AGWN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, block, smem));
     if (per_sm < 1)
         return fail(AGWN_ERR_UNSUPPORTED, "robust kernel does not fit on an SM");
-    int64_t const n_qtiles = (n + kRobBlock - 1) / kRobBlock;
+    int64_t const n_qtiles = (n + block - 1) / block;
     int const grid = int(std::max<int64_t>(1, std::min<int64_t>(n_qtiles, int64_t(per_sm) * ctx.sm_count)));
     AGWN_TRY(ctx.launch_begin(AGWN_K_ROBUST));
-    kern<<<grid, kRobBlock, smem, st>>>(d_pos, n, qz, static_cast<const Seg*>(r.seg), r.n_seg,
+    kern<<<grid, block, smem, st>>>(d_pos, n, qz, static_cast<const Seg*>(r.seg), r.n_seg,
                                         static_cast<const RChain*>(r.chain), r.n_entries, tile, d_counts, d_out,
                                         d_frac, ctx.d_flags, float(ctx.robust_term_err),
                                         ctx.timing ? ctx.d_counters : nullptr);

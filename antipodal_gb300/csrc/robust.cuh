@@ -573,6 +573,14 @@ __device__ __forceinline__ double l_plus_x(qv3<typename P::C> v, double l)
     return div_rn_int(dot_yz<P>(v, v), __dsub_rn(l, vx));
 }
 
+// l + x for differences below 2^24 (robust_contrib's short form): |v|^2 = x^2 + yz and yz = y^2 + z^2 are exact integers
+// below 2^50, as the reference's double products and sums of them are.
+__device__ __forceinline__ double l_plus_x_small(int32_t x, int64_t yz)
+{
+    double const l = sqrt_rn_int(double_of_53(int64_t(x) * x + yz)), vx = double_of(x);
+    return x >= 0 ? __dadd_rn(l, vx) : div_rn_int(double_of_53(yz), __dsub_rn(l, vx));
+}
+
 // Half-area contribution of one boundary segment.  gwn_mesh_robust.hh:272-321.
 template <class P>
 __device__ __forceinline__ double robust_contrib(qv3<typename P::C> q, RSeg<typename P::C> const& s)
@@ -591,15 +599,38 @@ __device__ __forceinline__ double robust_contrib(qv3<typename P::C> q, RSeg<type
         v0 = {__dsub_rn(p0.x, q.x), __dsub_rn(p0.y, q.y), __dsub_rn(p0.z, q.z)};
         v1 = {__dsub_rn(p1.x, q.x), __dsub_rn(p1.y, q.y), __dsub_rn(p1.z, q.z)};
     }
-    ev3<rd> const d0{rd(P::cdbl(v0.x)), rd(P::cdbl(v0.y)), rd(P::cdbl(v0.z))};
-    ev3<rd> const d1{rd(P::cdbl(v1.x)), rd(P::cdbl(v1.y)), rd(P::cdbl(v1.z))};
-    double const l0 = ex_sqrt(edot(d0, d0)).v;
-    double const l1 = ex_sqrt(edot(d1, d1)).v;
-    auto const num = atan2_num<P>(q, p0, p1);
-    double const yz = dot_yz<P>(v0, v1);
-    double const den = __dadd_rn(__dmul_rn(l_plus_x<P>(v0, l0), l_plus_x<P>(v1, l1)), yz);
-    if (P::sgn(num) != 0)
-        return atan2_int(P::dbl(num), den);
+    double den;
+    bool small = false;
+    if constexpr (std::is_same_v<P, P64>)
+    {
+        // Differences below 2^24 (every query within 16 grid extents of the mesh): all products and sums up to l are
+        // exact integers, so they run on the integer pipe, conversions included, and 13 FP64 instructions are left
+        // of about 40 (150,000 queries x 41 segments: call 972 -> 536 us).
+        unsigned const off = 1u << 24, lim = 1u << 25;
+        small = unsigned(v0.x) + off < lim && unsigned(v0.y) + off < lim && unsigned(v0.z) + off < lim &&
+                unsigned(v1.x) + off < lim && unsigned(v1.y) + off < lim && unsigned(v1.z) + off < lim;
+        if (small)
+        {
+            int64_t const n = int64_t(v0.z) * v1.y - int64_t(v0.y) * v1.z;
+            double const b0 = l_plus_x_small(v0.x, int64_t(v0.y) * v0.y + int64_t(v0.z) * v0.z);
+            double const b1 = l_plus_x_small(v1.x, int64_t(v1.y) * v1.y + int64_t(v1.z) * v1.z);
+            den = __dadd_rn(__dmul_rn(b0, b1), double_of_53(int64_t(v0.y) * v1.y + int64_t(v0.z) * v1.z));
+            if (n != 0)
+                return atan2_int(double_of_53(n), den);
+        }
+    }
+    if (!small)
+    {
+        ev3<rd> const d0{rd(P::cdbl(v0.x)), rd(P::cdbl(v0.y)), rd(P::cdbl(v0.z))};
+        ev3<rd> const d1{rd(P::cdbl(v1.x)), rd(P::cdbl(v1.y)), rd(P::cdbl(v1.z))};
+        double const l0 = ex_sqrt(edot(d0, d0)).v;
+        double const l1 = ex_sqrt(edot(d1, d1)).v;
+        auto const num = atan2_num<P>(q, p0, p1);
+        double const yz = dot_yz<P>(v0, v1);
+        den = __dadd_rn(__dmul_rn(l_plus_x<P>(v0, l0), l_plus_x<P>(v1, l1)), yz);
+        if (P::sgn(num) != 0)
+            return atan2_int(P::dbl(num), den);
+    }
     if (v0.y == 0 && v0.z == 0 && v0.x < 0 && (v1.y != 0 || v1.z != 0))
         return v1.z != 0 ? atan2(P::cdbl(v1.z), -P::cdbl(v1.y)) : (v1.y > 0 ? -pi : 0.0);
     if (v1.y == 0 && v1.z == 0 && v1.x < 0 && (v0.y != 0 || v0.z != 0))
@@ -842,6 +873,55 @@ __device__ __forceinline__ void robust_chain_step(RChain const* sb, int s, int n
         while (fq.tail - fq.head >= 32)
             rq_flush<P, K>(fq, 32, lane, gseg, q, half);
     }
+}
+
+// The exact form for few queries, shared out by segment as k_frac_exact_split (frac_kernels.cuh): block (x, y) takes the
+// queries 32 x .. 32 x + 31, its warp w the segments [g (4 y + w), + g); the block that finishes a query group last adds
+// its terms in segment order.  first / last: whether the sums start here (else they continue from acc) and end here.
+template <class T, class P>
+__global__ void __launch_bounds__(32 * kSplitWarps)
+    k_robust_frac_split(const T* __restrict__ pos, int n, Quant qz, const RSeg<typename P::C>* __restrict__ seg,
+                        int n_seg, int g, const int32_t* __restrict__ counts, T* __restrict__ out,
+                        T* __restrict__ out_frac, double* terms, double* acc, int* arrivals, bool first, bool last)
+{
+    __shared__ bool s_sum;
+    int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int const i = int(blockIdx.x) * 32 + lane, ii = min(i, n - 1);
+    auto const q = quantize<P>(double(pos[3 * ii]), double(pos[3 * ii + 1]), double(pos[3 * ii + 2]), qz);
+    int const s0 = min((int(blockIdx.y) * kSplitWarps + warp) * g, n_seg), s1 = min(s0 + g, n_seg);
+    for (int s = s0; s < s1; ++s)
+    {
+        RSeg<typename P::C> const sg = seg[s];
+        double const term = __dmul_rn(sg.w, robust_contrib<P>(q, sg));
+        if (i < n)
+            terms[size_t(s) * n + i] = term;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        s_sum = atomicAdd(arrivals + blockIdx.x, 1) == int(gridDim.y) - 1;
+        if (s_sum)
+            arrivals[blockIdx.x] = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_sum || warp != 0 || i >= n)
+        return;
+    double half = first ? 0.0 : acc[i];
+#pragma unroll 8
+    for (int s = 0; s < n_seg; ++s)
+        half = __dadd_rn(half, __ldcg(terms + size_t(s) * n + i));
+    if (!last)
+    {
+        acc[i] = half;
+        return;
+    }
+    constexpr double f_norm = 2.0 / (4.0 * 3.141592653589793238462643383279502884);
+    T const fr = T(__dmul_rn(half, f_norm));
+    out[i] = fr + T(counts ? counts[i] : 0);
+    if (out_frac)
+        out_frac[i] = fr;
 }
 
 // Mixed = true (int64_grid only): FP32 pairs on the boundary's vertex chains (robust_chain_step) with TwoSum
