@@ -256,8 +256,7 @@ int fractional_launch_mixed(Context& ctx, const FracPlan<T>& p, const double* d_
     // (34.9 ms against 40.5 on 1,066 segments), since more queries share each staged tile and its barriers
     int const block = ctx.frac_block ? ctx.frac_block : (p.nbuf > 1 || p.tile > 512 ? 256 : 128);
     int64_t const n_qtiles = (n + int64_t(block) * K - 1) / (int64_t(block) * K);
-    size_t const smem = size_t(p.nbuf) * p.tile * sizeof(SegM);
-    auto launch = [&](auto kern) -> int
+    auto launch = [&](auto kern, size_t smem) -> int
     {
         int grid = 0;
         AGWN_TRY(launch_persistent(ctx, kern, block, smem, n_qtiles, &grid));
@@ -271,11 +270,11 @@ int fractional_launch_mixed(Context& ctx, const FracPlan<T>& p, const double* d_
     switch (K)
     {
     case 2:
-        return launch(k_frac_mixed<2, FB>);
+        return launch(k_frac_mixed<2, FB>, mixed_smem<2>(p.nbuf, p.tile, block));
     case 4:
-        return launch(k_frac_mixed<4, FB>);
+        return launch(k_frac_mixed<4, FB>, mixed_smem<4>(p.nbuf, p.tile, block));
     default:
-        return launch(k_frac_mixed<8, FB>);
+        return launch(k_frac_mixed<8, FB>, mixed_smem<8>(p.nbuf, p.tile, block));
     }
 }
 

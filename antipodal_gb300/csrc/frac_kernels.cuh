@@ -757,10 +757,13 @@ constexpr int mixed_min_blocks()
 // max(kappa L_max, near distance), with a relative and an absolute slack for the float arithmetic of the test.
 // Groups holding a chain start, the first group of a tile (its vertex before lies in the previous tile) and a
 // tile's last, partial group take the full path.  A certified group's terms are bit-identical to the full path's:
-// the same operations minus the selects that the certificate fixes.  Groups of 8 entries with kappa 10 certify 82%
-// of the pairs of a 212-segment loop with 256^3 grid queries (16 entries, kappa 11.9: 72%; 3% slower).
-constexpr int kCertG = 8;
-constexpr int kCertMaxGroups = 256; // tiles of up to 2,048 entries
+// the same operations minus the selects that the certificate fixes.  Groups of 4 entries (their circles are half as
+// wide as those of 8) and two circles per query slot (a run of grid points is a line) certify 89% of the pairs of a
+// 212-segment loop with 256^3 grid queries against 82% for 8 and one.  The groups and the FP64 queues live in dynamic
+// shared memory, sized for the tile and the block, so that registers alone limit the blocks per SM (6 of 128 threads).
+// The whole call, 256^3 queries x 212 segments: 7.15 -> 6.55 ms; robust exact_float, 1.5e6 x 498: 2.73 -> 2.38 ms.
+constexpr int kCertG = 4;
+constexpr int kCertSub = 2;         // circles per query slot
 
 __device__ __forceinline__ float4 cert_group(SegM const* __restrict__ sb, int g, float kappa)
 {
@@ -797,6 +800,18 @@ __device__ __forceinline__ float4 cert_group(SegM const* __restrict__ sb, int g,
     return make_float4(cx, cy, 1.01f * reach + slack, 0.f);
 }
 
+__host__ __device__ constexpr int cert_groups(int tile)
+{
+    return (tile + kCertG - 1) / kCertG;
+}
+// Dynamic shared memory of k_frac_mixed.
+template <int K>
+constexpr size_t mixed_smem(int nbuf, int tile, int block)
+{
+    size_t const per_warp = sizeof(double) * 32 + sizeof(uint32_t) * Fp64Queue<K>::kCap;
+    return sizeof(float4) * cert_groups(tile) + per_warp * (block / 32) + sizeof(SegM) * size_t(nbuf) * tile;
+}
+
 // fb: the FP64 rule for the pairs the FP32 path turns down (MeshFallback, or the robust evaluator's).  K (even)
 // queries per thread, evaluated as K / 2 packed pairs.
 template <int K, class FB>
@@ -812,16 +827,18 @@ __global__ void __launch_bounds__(256, mixed_min_blocks<K>())
     __shared__ __align__(8) uint64_t bars[2];
     __shared__ int abort_cta;
     __shared__ double centre[3];
-    __shared__ uint32_t q_entries[8][Fp64Queue<K>::kCap];
-    __shared__ double q_results[8][32];
-    __shared__ float4 s_grp[kCertMaxGroups];
+    // dynamic shared memory (mixed_smem): the tile's groups, each warp's queue and results, the tile buffers
+    int const warps = int(blockDim.x) >> 5;
+    float4* const s_grp = reinterpret_cast<float4*>(smem);
+    double* const q_results = reinterpret_cast<double*>(s_grp + cert_groups(tile));
+    uint32_t* const q_entries = reinterpret_cast<uint32_t*>(q_results + 32 * warps);
 
     // the entry stream (chain starts and segments, k_prep_mixed) is what the tiles walk
     int64_t const n_entries = frame->n_entries;
     TilePipe<SegM> pipe;
     pipe.n_tiles = int((n_entries + tile - 1) / tile);
     pipe.single = pipe.n_tiles == 1;
-    pipe.buf[0] = reinterpret_cast<SegM*>(smem);
+    pipe.buf[0] = reinterpret_cast<SegM*>(q_entries + Fp64Queue<K>::kCap * warps);
     pipe.buf[1] = pipe.buf[0] + (pipe.single ? 0 : tile);
     pipe.bar = bars;
     pipe.gseg = seg;
@@ -858,7 +875,7 @@ __global__ void __launch_bounds__(256, mixed_min_blocks<K>())
     // the certified groups of the tile in shared memory (every thread calls it; ends with a block barrier)
     auto groups_of = [&](SegM const* sb, int cnt)
     {
-        int const ng = min(cnt / kCertG, kCertMaxGroups);
+        int const ng = cnt / kCertG;
         for (int g = threadIdx.x; g < ng; g += blockDim.x)
             s_grp[g] = cert_group(sb, g, kappa);
         __syncthreads();
@@ -866,8 +883,8 @@ __global__ void __launch_bounds__(256, mixed_min_blocks<K>())
     double const two_pi = 2.0 * kPi<double>;
     ev3<rd> const x1{rd(-x0x), rd(-x0y), rd(-x0z)};
     Fp64Queue<K> fq;
-    fq.e = q_entries[warp];
-    fq.res = q_results[warp];
+    fq.e = q_entries + Fp64Queue<K>::kCap * warp;
+    fq.res = q_results + 32 * warp;
 
     int it = 0;
     long long n_cert = 0; // entries of certified groups this warp evaluated (warp-uniform)
@@ -922,7 +939,7 @@ __global__ void __launch_bounds__(256, mixed_min_blocks<K>())
             float x0 = x, x1 = x, y0 = y, y1 = y;
             bool sane = fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) <= 16777216.f;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
+            for (int o = 16 / kCertSub; o > 0; o >>= 1)
             {
                 x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
                 x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
@@ -1092,13 +1109,13 @@ __global__ void __launch_bounds__(256, mixed_min_blocks<K>())
             }
             SegM const* sb = pipe.buf[b];
             int const cnt = pipe.tile_count(st);
-            int const ng = min(cnt / kCertG, kCertMaxGroups);
+            int const ng = cnt / kCertG;
             if (!pipe.single || j == 0)
                 groups_of(sb, cnt);
             // tiles start at even positions of the stream (the tile and the group are even), so the alternation runs
             // across groups and tiles; only the last tile can end on an odd count
             uint32_t cmask = 0;
-            for (int s0 = 0; s0 < cnt; s0 += kCertG)
+            for (int s0 = 0; s0 < cnt;)
             {
                 int const g = s0 / kCertG;
                 if ((g & 31) == 0)
@@ -1106,30 +1123,38 @@ __global__ void __launch_bounds__(256, mixed_min_blocks<K>())
                     // lane l tests group g + l against every query slot of the warp
                     int const gl = g + lane;
                     bool ok = gl < ng;
-                    if (ok)
-                    {
-                        float4 const c = s_grp[gl];
+                    float4 const c = s_grp[ok ? gl : 0];
 #pragma unroll
-                        for (int k = 0; k < K; ++k)
+                    for (int k = 0; k < K; ++k)
+#pragma unroll
+                        for (int h = 0; h < kCertSub; ++h)
                         {
-                            float const dx = c.x - scx[k], dy = c.y - scy[k], need = c.z + srad[k];
+                            // the slot's h-th circle, held by its 32 / kCertSub lanes
+                            int const from = 32 / kCertSub * h;
+                            float const dx = c.x - __shfl_sync(0xffffffffu, scx[k], from),
+                                        dy = c.y - __shfl_sync(0xffffffffu, scy[k], from),
+                                        need = c.z + __shfl_sync(0xffffffffu, srad[k], from);
                             ok = ok && dx * dx + dy * dy >= need * need;
                         }
-                    }
                     cmask = __ballot_sync(0xffffffffu, ok);
                 }
-                if ((cmask >> (g & 31)) & 1u)
+                // the run of groups alike from here, within this mask
+                uint32_t const rest = cmask >> (g & 31);
+                int const run = (rest & 1u ? (~rest ? __ffs(~rest) - 1 : 32) : (rest ? __ffs(rest) - 1 : 32));
+                int const e1 = min((g + min(run, 32 - (g & 31))) * kCertG, cnt);
+                if (rest & 1u)
                 {
-                    n_cert += kCertG;
-                    for (int s = s0; s < s0 + kCertG; s += 2)
+                    n_cert += e1 - s0;
+                    for (int s = s0; s < e1; s += 2)
                     {
                         fast(sb[s], st1, st0);
                         fast(sb[s + 1], st0, st1);
                     }
+                    s0 = e1;
                     continue;
                 }
-                int const e1 = min(s0 + kCertG, cnt);
                 int s = s0;
+                s0 = e1;
                 for (; s + 1 < e1; s += 2)
                 {
                     if ((__float_as_int(sb[s].c.w) | __float_as_int(sb[s + 1].c.w)) >= 0)

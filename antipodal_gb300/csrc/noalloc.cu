@@ -133,7 +133,7 @@ extern "C" int agwn_mesh_batch_fractional_mixed_noalloc_f64(void* stream, const 
     int64_t const max_entries = 2 * n_segments;
     int const tile = int(std::min<int64_t>(kNoAllocTile, max_entries));
     int const n_tiles = int((max_entries + tile - 1) / tile);
-    size_t const smem = size_t(n_tiles == 1 ? 1 : 2) * tile * sizeof(SegM);
+    size_t const smem = mixed_smem<kNoAllocK>(n_tiles == 1 ? 1 : 2, tile, kNoAllocBlock);
     auto kern = k_frac_mixed<kNoAllocK, MeshFallback>;
     AGWN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     int per_sm = 0;
