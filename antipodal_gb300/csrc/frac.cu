@@ -15,7 +15,7 @@
 //  * mixed  -- double input only.  Queries and segments are moved to a frame where x1 is +z and centred on the
 //              boundary; queries and boundary vertices are held as float pairs hi + lo and the segment vector
 //              d = P1 - P0 is rounded from FP64.  The boundary is walked as chains of segments that share
-//              vertices (k_prep_mixed), so v = (P_hi - Q_hi) + (P_lo - Q_lo), |v| and the half-angle form of each
+//              vertices (k_prep_chains), so v = (P_hi - Q_hi) + (P_lo - Q_lo), |v| and the half-angle form of each
 //              vertex are computed once for the two segments that meet there.  A pair (query, segment) is
 //              evaluated in FP32 from v0, v1 and d:
 //                num = v0.x*d.y - v0.y*d.x  (no cancellation for a far segment: d is accurate on its own),
@@ -135,7 +135,7 @@ int fractional_prepare(Context& ctx, const T* x0_host, const T* d_seg_raw, int64
     AGWN_CHECK_ARG(x0n > 0 && std::isfinite(x0n), "mixed mode needs a finite nonzero x0");
     p.rot = make_rotation(p.x0d);
     // the entry stream holds between n_seg + 1 and 2 n_seg entries; the tile (even) and the buffers are sized for
-    // the most, the kernel reads the count k_prep_mixed wrote
+    // the most, the kernel reads the count k_prep_chains wrote
     int64_t const max_entries = 2 * n_seg;
     p.tile = int(std::min<int64_t>(ctx.seg_tile, max_entries));
     p.nbuf = max_entries > p.tile ? 2 : 1;
@@ -146,8 +146,12 @@ int fractional_prepare(Context& ctx, const T* x0_host, const T* d_seg_raw, int64
     AGWN_TRY(ctx.scratch_reserve(S_SEGS_RAW, sizeof(SegX<double>) * n_seg, reinterpret_cast<void**>(&p.seg64)));
     AGWN_TRY(ctx.scratch_reserve(S_FRAME, sizeof(Frame), reinterpret_cast<void**>(&p.frame)));
     AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-    k_prep_mixed<<<1, 1024, 0, ctx.stream>>>(reinterpret_cast<const double*>(d_seg_raw), n_seg, p.rot,
-                                             float(ctx.mixed_tau), p.frame, p.segm, p.seg64, order);
+    const double* const raw = reinterpret_cast<const double*>(d_seg_raw);
+    k_prep_chains<<<1, kChainBlock, 0, ctx.stream>>>(raw, n_seg, p.frame, order);
+    AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
+    AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
+    k_prep_entries<<<prep_blocks(n_seg, ctx.sm_count), 128, 0, ctx.stream>>>(raw, n_seg, p.rot, float(ctx.mixed_tau),
+                                                                            p.frame, p.segm, p.seg64, order);
     AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
     // The stream holds n_seg + (number of chains) entries, at most 2 n_seg.  When that bound would take several
     // tiles but the boundary could fit one, the actual count is read back (a wait on the stream): one tile runs

@@ -9,6 +9,7 @@
 
 #include <type_traits>
 
+#include <algorithm>
 #include <climits>
 #include <cmath>
 
@@ -21,7 +22,7 @@ struct alignas(16) SegX
 {
     T p0x, p0y, p0z, p1x, p1y, p1z, w, pad;
 };
-// Mixed-mode boundary entry: a vertex and the segment that ends at it, in chain order (k_prep_mixed).
+// Mixed-mode boundary entry: a vertex and the segment that ends at it, in chain order (k_prep_entries).
 //   segment entry: a = (P1_hi, w), b = (P1 - P0, near2), c = (P1_lo, segment index as bits);
 //   chain start:   a = (P0_hi, 0), b = (0, 0, 0, near2), c = (P0_lo, -1 as bits).
 // P0 of a segment entry is the vertex of the entry before it.  near2 = (tau * L)^2 with L the longer of the (one or
@@ -37,7 +38,7 @@ struct Rot
 struct Frame
 {
     double c[3];
-    long long n_entries; // boundary entries written by k_prep_mixed
+    long long n_entries; // boundary entries written by k_prep_chains
 };
 
 template <class T>
@@ -291,7 +292,7 @@ __device__ __forceinline__ uint32_t point_hash(double x, double y, double z)
 __device__ __forceinline__ float seg_length(const double* w)
 {
     double const ex = w[3] - w[0], ey = w[4] - w[1], ez = w[5] - w[2];
-    return float(sqrt(ex * ex + ey * ey + ez * ez));
+    return float(sqrt_rn_int(ex * ex + ey * ey + ez * ez));
 }
 
 // Chains of ns <= kChainMax segments by exact endpoint equality, in one block (every thread calls it): segment t
@@ -300,7 +301,9 @@ __device__ __forceinline__ float seg_length(const double* w)
 // s: segment s, ending at end(s) -- open chains from their first segment, then closed loops from their
 // lowest-numbered segment, and wrap[e]: for the first and last entry of a closed loop the segment that closes it
 // at that vertex, else -1.  Returns m in every thread.  start(t), end(s): the endpoints as double3 (exact for the
-// callers' coordinates).  table: chain_table_size(ns) ints of global scratch; the s_ arrays: kChainMax each.
+// callers' coordinates).  table: chain_table_size(ns) ints of global scratch; the s_ arrays: kChainMax each.  A block of
+// kChainBlock threads.
+constexpr int kChainBlock = 1024;
 template <class Start, class End>
 __device__ int block_chains(int ns, Start start, End end, int* __restrict__ order, int* __restrict__ wrap,
                             int* __restrict__ table, int* s_succ, int* s_pred, unsigned char* s_seen, int* s_m)
@@ -351,74 +354,170 @@ __device__ int block_chains(int ns, Start start, End end, int* __restrict__ orde
             s_succ[si] = -1; // t follows a lower-numbered segment
     }
     __syncthreads();
-    if (threadIdx.x == 0)
+    // Every segment's chain head and its rank in the chain by pointer doubling (a serial walk took 0.2 us per segment).
+    // A loop has no head: first the lowest segment number over the 2^r segments that follow each one, which covers a
+    // loop after log2(length) rounds; the lowest becomes the loop's head.  Then the distance to the head over the
+    // predecessors.  The arrays of 16-bit indices share s_succ's storage; a thread owns the same segments throughout.
+    constexpr int kOwn = kChainMax / kChainBlock;
+    short* const ptr = reinterpret_cast<short*>(s_succ);
+    short* const val = ptr + kChainMax;
+    int rounds = 0;
+    while ((1 << rounds) < ns)
+        ++rounds;
+    short rp[kOwn], rv[kOwn];
+    int tail[kOwn]; // of a loop's head: the loop's last segment
+    auto const each = [&](auto f)
     {
-        int m = 0;
-        // pass 0: open chains from their heads (no predecessor); pass 1: what is left lies on closed loops
-        for (int pass = 0; pass < 2; ++pass)
-            for (int si = 0; si < ns; ++si)
+#pragma unroll
+        for (int k = 0; k < kOwn; ++k)
+        {
+            int const t = int(threadIdx.x) + k * kChainBlock;
+            if (t < ns)
+                f(t, k, rp[k], rv[k]);
+        }
+    };
+    each([&](int t, int, short& p, short& v) { p = short(s_succ[t]); v = short(t); });
+    __syncthreads();
+    each([&](int t, int, short& p, short& v) { ptr[t] = p; val[t] = v; });
+    __syncthreads();
+    for (int r = 0; r < rounds; ++r)
+    {
+        each([&](int, int, short& p, short& v)
+             {
+                 if (p >= 0)
+                 {
+                     v = min(v, val[p]);
+                     p = ptr[p];
+                 }
+             });
+        __syncthreads();
+        each([&](int t, int, short& p, short& v) { ptr[t] = p; val[t] = v; });
+        __syncthreads();
+    }
+    // s_seen: 1 for the head of an open chain, 2 for a loop's
+    each([&](int t, int k, short& p, short& v)
+         {
+             tail[k] = s_pred[t];
+             bool const open = s_pred[t] == INT_MAX, loop = p >= 0 && v == t;
+             s_seen[t] = open ? 1 : (loop ? 2 : 0);
+             p = short(open || loop ? t : s_pred[t]);
+             v = open || loop ? 0 : 1;
+         });
+    __syncthreads();
+    each([&](int t, int, short& p, short& v) { ptr[t] = p; val[t] = v; });
+    __syncthreads();
+    for (int r = 0; r < rounds; ++r)
+    {
+        each([&](int, int, short& p, short& v)
+             {
+                 v = short(v + val[p]);
+                 p = ptr[p];
+             });
+        __syncthreads();
+        each([&](int t, int, short& p, short& v) { ptr[t] = p; val[t] = v; });
+        __syncthreads();
+    }
+    // s_pred: the chains' lengths at their heads, then their first entries: open chains first, by their heads
+    each([&](int t, int, short&, short&) { s_pred[t] = 0; });
+    __syncthreads();
+    each([&](int, int, short& p, short& v) { atomicMax(&s_pred[p], v + 1); });
+    __syncthreads();
+    int const warp = int(threadIdx.x) >> 5, lane = int(threadIdx.x) & 31;
+    __shared__ int s_part[kChainBlock / 32];
+    int m = 0;
+    for (int kind = 1; kind <= 2; ++kind)
+#pragma unroll
+        for (int k = 0; k < kOwn; ++k)
+        {
+            if (k * kChainBlock >= ns)
+                break;
+            int const t = int(threadIdx.x) + k * kChainBlock;
+            bool const head = t < ns && s_seen[t] == kind;
+            int const len = head ? s_pred[t] + 1 : 0; // with its start entry
+            int sum = len;
+            for (int o = 1; o < 32; o <<= 1)
             {
-                if (s_seen[si] || (pass == 0 && s_pred[si] != INT_MAX))
-                    continue;
-                int const first = m;
-                order[m++] = ~si;
-                int last = si;
-                for (int cur = si; cur >= 0 && !s_seen[cur]; cur = s_succ[cur])
-                {
-                    s_seen[cur] = 1;
-                    order[m++] = cur;
-                    last = cur;
-                }
-                if (pass == 1)
+                int const u = __shfl_up_sync(0xffffffffu, sum, o);
+                sum += lane >= o ? u : 0;
+            }
+            if (lane == 31)
+                s_part[warp] = sum;
+            __syncthreads();
+            int before = 0, total = 0;
+            for (int w = 0; w < kChainBlock / 32; ++w)
+            {
+                before += w < warp ? s_part[w] : 0;
+                total += s_part[w];
+            }
+            if (head)
+            {
+                int const first = m + before + sum - len;
+                order[first] = ~t;
+                if (kind == 2)
                 {
                     // a closed loop: its last segment ends at the start vertex
-                    wrap[first] = last;
-                    wrap[m - 1] = si;
+                    wrap[first] = tail[k];
+                    wrap[first + len - 1] = t;
                 }
+                s_pred[t] = first;
             }
+            m += total;
+            __syncthreads();
+        }
+    each([&](int t, int, short& p, short& v) { order[s_pred[p] + 1 + v] = t; });
+    if (threadIdx.x == 0)
         *s_m = m;
-    }
     __syncthreads();
     return *s_m;
 }
 
-// One block.  (1) The bounding-box centre of all endpoints.  (2) Chains: segment t follows segment s when
-// P0(t) == P1(s) exactly (all three doubles), each t following at most one s (the lowest-numbered), so the links form
-// disjoint open chains and closed loops.  (3) The entry stream: per chain a start entry (its first segment's P0)
-// and then one entry per segment (its P1), open chains from their first segment and closed loops from their
-// lowest-numbered segment, each vertex moved into the x1 = +z frame around the centre.  Chained vertices are the
-// same doubles, so every segment sees the same P0 and P1 as in a stream of one chain per segment; chaining only
-// lets the fractional kernel share the per-vertex work of consecutive segments.  A vertex's near threshold takes
-// the longer of the segments that meet it in its chain, the last and first segments of a closed loop included, so
-// on a boundary where no more than two segments meet at a vertex it does not depend on the input order.
+// The entry stream of the mixed kernel, in two kernels.  k_prep_chains, one block: (1) the bounding-box centre of all
+// endpoints; (2) chains: segment t follows segment s when P0(t) == P1(s) exactly (all three doubles), each t following
+// at most one s (the lowest-numbered), so the links form disjoint open chains and closed loops.  k_prep_entries, a
+// thread per entry: (3) per chain a start entry (its first segment's P0) and then one entry per segment (its P1), open
+// chains from their first segment and closed loops from their lowest-numbered segment, each vertex moved into the
+// x1 = +z frame around the centre.  Chained vertices are the same doubles, so every segment sees the same P0 and P1 as
+// in a stream of one chain per segment; chaining only lets the fractional kernel share the per-vertex work of
+// consecutive segments.  A vertex's near threshold takes the longer of the segments that meet it in its chain, the last
+// and first segments of a closed loop included, so on a boundary where no more than two segments meet at a vertex it
+// does not depend on the input order.
 // order: chain_scratch_ints(n_seg) ints of scratch (the stream order, each entry's loop-closing neighbour, and an
 // open-addressing hash table of segment starts that finds the links in O(n_seg)).
-__global__ void __launch_bounds__(1024) k_prep_mixed(const double* __restrict__ raw, int64_t n_seg, Rot rot,
-                                                     float tau, Frame* __restrict__ frame, SegM* __restrict__ out,
-                                                     SegX<double>* __restrict__ out64, int* __restrict__ order)
+//
+// FP64 issue bounds the entries (about 100 instructions each), so they take many SMs; in one block, after a serial walk
+// of the chains, 102 / 212 / 498 segments took 38 / 57 / 113 us, now %PREP%.
+__global__ void __launch_bounds__(kChainBlock) k_prep_chains(const double* __restrict__ raw, int64_t n_seg,
+                                                             Frame* __restrict__ frame, int* __restrict__ order)
 {
-    __shared__ double red[2][3][32];
-    __shared__ double centre[3];
+    // the coordinates as integers that order like them (a double comparison takes the FP64 pipe); a NaN is left out
+    __shared__ unsigned long long red[2][3][32];
     __shared__ int s_succ[kChainMax], s_pred[kChainMax];
     __shared__ unsigned char s_seen[kChainMax];
     __shared__ int s_entries;
-    double mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+    unsigned long long mn[3] = {~0ull, ~0ull, ~0ull}, mx[3] = {0, 0, 0};
     for (int64_t s = threadIdx.x; s < n_seg; s += blockDim.x)
     {
         const double* w = raw + 7 * s;
-        for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
         {
-            mn[k] = fmin(mn[k], fmin(w[k], w[3 + k]));
-            mx[k] = fmax(mx[k], fmax(w[k], w[3 + k]));
+            unsigned long long const u = bits_of(w[k]), o = (u >> 63) ? ~u : u | 0x8000000000000000ull;
+            if ((u << 1) > 0xffe0000000000000ull)
+                continue;
+            mn[k % 3] = o < mn[k % 3] ? o : mn[k % 3];
+            mx[k % 3] = o > mx[k % 3] ? o : mx[k % 3];
         }
     }
     int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
     for (int k = 0; k < 3; ++k)
     {
         for (int o = 16; o > 0; o >>= 1)
         {
-            mn[k] = fmin(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
-            mx[k] = fmax(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+            unsigned long long const a = __shfl_xor_sync(0xffffffffu, mn[k], o);
+            unsigned long long const b = __shfl_xor_sync(0xffffffffu, mx[k], o);
+            mn[k] = a < mn[k] ? a : mn[k];
+            mx[k] = b > mx[k] ? b : mx[k];
         }
         if (lane == 0)
         {
@@ -434,14 +533,16 @@ __global__ void __launch_bounds__(1024) k_prep_mixed(const double* __restrict__ 
     if (threadIdx.x < 3)
     {
         int const k = threadIdx.x;
-        double a = INFINITY, b = -INFINITY;
-        for (int w = 0; w < int(blockDim.x + 31) / 32; ++w)
+        unsigned long long lo = ~0ull, hi = 0;
+        for (int w = 0; w < kChainBlock / 32; ++w)
         {
-            a = fmin(a, red[0][k][w]);
-            b = fmax(b, red[1][k][w]);
+            lo = red[0][k][w] < lo ? red[0][k][w] : lo;
+            hi = red[1][k][w] > hi ? red[1][k][w] : hi;
         }
-        centre[k] = (n_seg > 0) ? 0.5 * (a + b) : 0.0;
-        frame->c[k] = centre[k];
+        // no number at all (hi below lo): +-infinity, as from an empty box
+        double const a = lo <= hi ? of_bits((lo >> 63) ? lo & 0x7fffffffffffffffull : ~lo) : INFINITY;
+        double const b = lo <= hi ? of_bits((hi >> 63) ? hi & 0x7fffffffffffffffull : ~hi) : -INFINITY;
+        frame->c[k] = (n_seg > 0) ? 0.5 * (a + b) : 0.0;
     }
     // (2) the chains
     int const mc = block_chains(
@@ -451,20 +552,25 @@ __global__ void __launch_bounds__(1024) k_prep_mixed(const double* __restrict__ 
     int const m = chain ? mc : int(2 * n_seg);
     if (threadIdx.x == 0)
         frame->n_entries = m;
-    // the links are done: s_pred now holds each segment's length
-    float* const s_len = reinterpret_cast<float*>(s_pred);
-    for (int s = threadIdx.x; s < ns; s += blockDim.x)
-        s_len[s] = seg_length(raw + 7 * size_t(s));
-    __syncthreads();
-    auto len_of = [&](int s) { return chain ? s_len[s] : seg_length(raw + 7 * size_t(s)); };
-    double const cx = centre[0], cy = centre[1], cz = centre[2];
+}
+
+__global__ void __launch_bounds__(128) k_prep_entries(const double* __restrict__ raw, int64_t n_seg, Rot rot, float tau,
+                                                      const Frame* __restrict__ frame, SegM* __restrict__ out,
+                                                      SegX<double>* __restrict__ out64, const int* __restrict__ order)
+{
+    bool const chain = n_seg <= kChainMax;
+    const int* const wrap = order + 2 * (chain ? n_seg : 0); // per entry: the segment that closes its loop there, or -1
+    int64_t const m = frame->n_entries;
+    int64_t const stride = int64_t(gridDim.x) * blockDim.x, first = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    auto len_of = [&](int s) { return seg_length(raw + 7 * size_t(s)); };
+    double const cx = frame->c[0], cy = frame->c[1], cz = frame->c[2];
     auto rotated = [&](const double* pt, double (&P)[3])
     {
         double const dx = pt[0] - cx, dy = pt[1] - cy, dz = pt[2] - cz;
         for (int r = 0; r < 3; ++r)
             P[r] = rot.m[3 * r] * dx + rot.m[3 * r + 1] * dy + rot.m[3 * r + 2] * dz;
     };
-    for (int e = threadIdx.x; e < m; e += blockDim.x)
+    for (int64_t e = first; e < m; e += stride)
     {
         int s;
         bool start;
@@ -476,7 +582,7 @@ __global__ void __launch_bounds__(1024) k_prep_mixed(const double* __restrict__ 
         }
         else
         {
-            s = e >> 1;
+            s = int(e >> 1);
             start = (e & 1) == 0;
         }
         const double* w = raw + 7 * size_t(s);
@@ -519,11 +625,17 @@ __global__ void __launch_bounds__(1024) k_prep_mixed(const double* __restrict__ 
         }
         out[e] = mm;
     }
-    for (int64_t s = threadIdx.x; s < n_seg; s += blockDim.x)
+    for (int64_t s = first; s < n_seg; s += stride)
     {
         const double* w = raw + 7 * s;
         out64[s] = SegX<double>{w[0], w[1], w[2], w[3], w[4], w[5], w[6], 0.0};
     }
+}
+
+// Blocks of k_prep_entries: an entry per thread, at most two entries per segment.
+inline int prep_blocks(int64_t n_seg, int sm_count)
+{
+    return int(std::min<int64_t>(div_up(2 * n_seg, 128), 16 * int64_t(sm_count)));
 }
 
 // atan2 for the FP32 terms, our own: reduce to t = min(|y|, |x|) / max(|y|, |x|) in [0, 1], evaluate
@@ -833,7 +945,7 @@ __global__ void __launch_bounds__(256, mixed_min_blocks<K>())
     double* const q_results = reinterpret_cast<double*>(s_grp + cert_groups(tile));
     uint32_t* const q_entries = reinterpret_cast<uint32_t*>(q_results + 32 * warps);
 
-    // the entry stream (chain starts and segments, k_prep_mixed) is what the tiles walk
+    // the entry stream (chain starts and segments, k_prep_entries) is what the tiles walk
     int64_t const n_entries = frame->n_entries;
     TilePipe<SegM> pipe;
     pipe.n_tiles = int((n_entries + tile - 1) / tile);

@@ -126,8 +126,11 @@ extern "C" int agwn_mesh_batch_fractional_mixed_noalloc_f64(void* stream, const 
     }
     Context defaults; // option defaults only (no resources)
     Rot const rot = make_rotation(x0);
-    k_prep_mixed<<<1, 1024, 0, st>>>(boundary, n_segments, rot, float(defaults.mixed_tau), &scr->frame, scr->seg,
-                                     scr->seg64, scr->order);
+    k_prep_chains<<<1, kChainBlock, 0, st>>>(boundary, n_segments, &scr->frame, scr->order);
+    AGWN_TRY_CUDA(cudaGetLastError());
+    k_prep_entries<<<prep_blocks(n_segments, sm_count), 128, 0, st>>>(boundary, n_segments, rot,
+                                                                      float(defaults.mixed_tau), &scr->frame, scr->seg,
+                                                                      scr->seg64, scr->order);
     AGWN_TRY_CUDA(cudaGetLastError());
 
     int64_t const max_entries = 2 * n_segments;

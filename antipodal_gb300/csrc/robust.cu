@@ -159,7 +159,7 @@ int robust_build(Context& ctx, const T* vertices, int64_t nv, const int32_t* ind
             AGWN_TRY(order.alloc(sizeof(int) * std::max<int64_t>(1, chain_scratch_ints(n_seg))));
             AGWN_TRY(cnt.alloc(sizeof(long long)));
             AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-            k_robust_chain<<<1, 1024, 0, st>>>(static_cast<const RSeg<int32_t>*>(out->seg), n_seg,
+            k_robust_chain<<<1, kChainBlock, 0, st>>>(static_cast<const RSeg<int32_t>*>(out->seg), n_seg,
                                                static_cast<RChain*>(out->chain), static_cast<long long*>(cnt.p),
                                                static_cast<int*>(order.p));
             AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));

@@ -396,7 +396,7 @@ __global__ void k_robust_segs(const T* __restrict__ raw, int64_t n_seg, Quant qz
 // One block: the vertex chains of an int64_grid boundary (block_chains on the RSeg endpoints), then the entries;
 // boundaries above kChainMax segments take one chain per segment.  *n_entries receives the count.  order:
 // chain_scratch_ints(n_seg) ints of scratch.
-__global__ void __launch_bounds__(1024) k_robust_chain(const RSeg<int32_t>* __restrict__ seg, int64_t n_seg,
+__global__ void __launch_bounds__(kChainBlock) k_robust_chain(const RSeg<int32_t>* __restrict__ seg, int64_t n_seg,
                                                        RChain* __restrict__ out, long long* __restrict__ n_entries,
                                                        int* __restrict__ order)
 {
