@@ -465,11 +465,15 @@ def build_boundary_segments(dispatcher: CudaDispatcher, vertices, indices):
     i = _View(indices, np.int32, None, "indices")
     fn = getattr(library(), f"agwn_build_boundary_segments_{kind}")
     cnt = C.c_int64()
-    _check(fn(dispatcher.handle, v.ptr, v.n, i.ptr, i.n, None, 0, C.byref(cnt)), "build_boundary_segments")
-    out = _empty_like_input(vertices, (cnt.value, 7), dt)
-    o = _View(out, dt, None, "out", writable=True)
-    _check(fn(dispatcher.handle, v.ptr, v.n, i.ptr, i.n, o.ptr, cnt.value, C.byref(cnt)), "build_boundary_segments")
-    return out
+    rows = 8192  # most boundaries fit; a longer one takes a second call with its count
+    while True:
+        out = _empty_like_input(vertices, (rows, 7), dt)
+        o = _View(out, dt, None, "out", writable=True)
+        _check(fn(dispatcher.handle, v.ptr, v.n, i.ptr, i.n, o.ptr, rows, C.byref(cnt)), "build_boundary_segments")
+        if cnt.value <= rows:
+            break
+        rows = cnt.value
+    return out[:cnt.value]
 
 
 class CudaRobustBatch:

@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <vector>
 
 #include "../../include/antipodal_gb300.h"
 #include "intfp.cuh"
@@ -60,6 +61,23 @@ struct DevBuf
     void* ptr = nullptr;
     size_t cap = 0;
     int reserve(size_t bytes);
+    void release();
+};
+
+// Build temporaries of one context, taken and given back in stack order on the context's stream: cudaMalloc and
+// cudaFree cost more than most of the kernels between them (and a free waits for the device).  The memory stays for
+// the context's next build, up to kKeep bytes.
+struct Arena
+{
+    static constexpr size_t kKeep = size_t(1) << 30;
+    struct Chunk
+    {
+        char* ptr;
+        size_t cap, used;
+    };
+    std::vector<Chunk> chunks;
+    int depth = 0;
+    int take(size_t bytes, void** out);
     void release();
 };
 
@@ -141,6 +159,7 @@ struct Context
     long long* d_counters = nullptr; // kCounters: [0] fp64 pairs, [1] pairs, [2] parametric skips, [3] certified pairs, [4..7] integer, [8..11] patches
                                      // term: queries, cell-list entries, candidate leaves, exact tests
     DevBuf scratch[S_COUNT];
+    Arena arena;
     static constexpr int kArrivals = 2048;
     int* d_arrivals = nullptr; // kArrivals zeroed counters, left zeroed by each kernel that uses them
     int sm_count = 0;
@@ -206,6 +225,33 @@ struct Context
     int launch_end(int kclass);
     int drain_timing(); // folds finished events into kernel_ms (synchronises the stream)
     int check_flags();  // synchronises and reports device flags
+};
+
+// The temporaries taken between its construction and its destruction.
+class ArenaScope
+{
+public:
+    explicit ArenaScope(Context& ctx);
+    ~ArenaScope();
+    ArenaScope(ArenaScope const&) = delete;
+    ArenaScope& operator=(ArenaScope const&) = delete;
+
+private:
+    Context& ctx_;
+    size_t chunk_, used_;
+};
+// One temporary of the enclosing ArenaScope.
+struct Tmp
+{
+    Context& ctx;
+    void* p = nullptr;
+    explicit Tmp(Context& c) : ctx(c) {}
+    int alloc(size_t bytes) { return ctx.arena.take(bytes, &p); }
+    template <class U>
+    U* as() const
+    {
+        return static_cast<U*>(p);
+    }
 };
 
 // ---- host/device pointers ----------------------------------------------------------------------------------

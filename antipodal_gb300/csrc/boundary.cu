@@ -133,33 +133,6 @@ __global__ void k_edge_emit(const unsigned long long* __restrict__ keys, const i
     }
 }
 
-struct Buf
-{
-    void* p = nullptr;
-    ~Buf()
-    {
-        if (p)
-            cudaFree(p);
-    }
-    int alloc(size_t bytes)
-    {
-        cudaError_t const e = cudaMalloc(&p, bytes ? bytes : 1);
-        if (e != cudaSuccess)
-        {
-            cudaGetLastError();
-            p = nullptr;
-            return fail(e == cudaErrorMemoryAllocation ? AGWN_ERR_NOMEM : AGWN_ERR_CUDA, "cudaMalloc(%zu): %s", bytes,
-                        cudaGetErrorString(e));
-        }
-        return AGWN_OK;
-    }
-    template <class X>
-    X* as() const
-    {
-        return static_cast<X*>(p);
-    }
-};
-
 template <class T>
 int boundary_build(agwn_context* ctx, const T* vertices, int64_t nv, const int32_t* indices, int64_t n_idx, T* out,
                    int64_t capacity, int64_t* n_segments)
@@ -180,13 +153,14 @@ int boundary_build(agwn_context* ctx, const T* vertices, int64_t nv, const int32
     AGWN_TRY(stage_in(*ctx, indices, sizeof(int32_t) * n_idx, S_MISC1, &di));
     int const n_rs_blocks = int((m + kRsTile - 1) / kRsTile);
     int64_t const n_sb = (m + kScanBlock - 1) / kScanBlock;
-    Buf ka, kb, va, vb, hist, net, emit, pos, sums;
+    ArenaScope scope(*ctx);
+    Tmp ka(*ctx), kb(*ctx), va(*ctx), vb(*ctx), hist(*ctx), net(*ctx), emit(*ctx), pos(*ctx), sums(*ctx);
     AGWN_TRY(ka.alloc(sizeof(unsigned long long) * m));
     AGWN_TRY(kb.alloc(sizeof(unsigned long long) * m));
     AGWN_TRY(va.alloc(sizeof(int) * m));
     AGWN_TRY(vb.alloc(sizeof(int) * m));
     AGWN_TRY(hist.alloc(sizeof(unsigned) * 256 * size_t(n_rs_blocks)));
-    Buf hsum;
+    Tmp hsum(*ctx);
     AGWN_TRY(hsum.alloc(sizeof(unsigned) * size_t(scan_sums_count(int64_t(256) * n_rs_blocks))));
     AGWN_TRY(net.alloc(sizeof(int) * m));
     AGWN_TRY(emit.alloc(sizeof(unsigned) * m));

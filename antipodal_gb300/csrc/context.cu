@@ -2,6 +2,7 @@
 
 #include "agwn_internal.cuh"
 
+#include <algorithm>
 #include <cmath>
 
 namespace agwn
@@ -58,6 +59,72 @@ void DevBuf::release()
         cudaFree(ptr);
     ptr = nullptr;
     cap = 0;
+}
+
+int Arena::take(size_t bytes, void** out)
+{
+    bytes = (bytes + 255) / 256 * 256 + (bytes == 0 ? 256 : 0);
+    if (chunks.empty() || chunks.back().cap - chunks.back().used < bytes)
+    {
+        size_t total = 0;
+        for (Chunk const& c : chunks)
+            total += c.cap;
+        Chunk c{nullptr, std::max<size_t>({bytes, total, size_t(1) << 18}), 0};
+        cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&c.ptr), c.cap);
+        if (e == cudaErrorMemoryAllocation && c.cap > bytes)
+        {
+            cudaGetLastError();
+            c.cap = bytes;
+            e = cudaMalloc(reinterpret_cast<void**>(&c.ptr), c.cap);
+        }
+        if (e != cudaSuccess)
+        {
+            cudaGetLastError();
+            return fail(e == cudaErrorMemoryAllocation ? AGWN_ERR_NOMEM : AGWN_ERR_CUDA, "cudaMalloc(%zu): %s", bytes,
+                        cudaGetErrorString(e));
+        }
+        chunks.push_back(c);
+    }
+    *out = chunks.back().ptr + chunks.back().used;
+    chunks.back().used += bytes;
+    return AGWN_OK;
+}
+
+void Arena::release()
+{
+    for (Chunk const& c : chunks)
+        cudaFree(c.ptr);
+    chunks.clear();
+}
+
+ArenaScope::ArenaScope(Context& ctx) : ctx_(ctx)
+{
+    chunk_ = ctx.arena.chunks.size();
+    used_ = chunk_ ? ctx.arena.chunks.back().used : 0;
+    ++ctx.arena.depth;
+}
+
+ArenaScope::~ArenaScope()
+{
+    Arena& a = ctx_.arena;
+    size_t total = 0;
+    for (Arena::Chunk& c : a.chunks)
+        total += c.cap;
+    --a.depth;
+    if (a.depth == 0 && (a.chunks.size() > 1 || total > Arena::kKeep))
+    {
+        // several chunks become one for the next build; more than kKeep is given back
+        cudaStreamSynchronize(ctx_.stream);
+        a.release();
+        void* whole = nullptr;
+        if (total <= Arena::kKeep && a.take(total, &whole) == AGWN_OK)
+            a.chunks.back().used = 0;
+        return;
+    }
+    for (size_t k = chunk_; k < a.chunks.size(); ++k)
+        a.chunks[k].used = 0;
+    if (chunk_)
+        a.chunks[chunk_ - 1].used = used_;
 }
 
 int Context::scratch_reserve(int slot, size_t bytes, void** out)
@@ -253,17 +320,14 @@ int agwn_context_create(int device, void* stream, agwn_context** out)
                 break;
             ctx->own_stream = true;
         }
-        if ((e = cudaMalloc(&ctx->d_flags, sizeof(int) * FLAG_COUNT)) != cudaSuccess)
+        // flags, counters and arrival counters in one zeroed allocation (owned by d_counters)
+        size_t const counters = sizeof(long long) * kCounters, flags = sizeof(int) * FLAG_COUNT;
+        size_t const bytes = counters + flags + sizeof(int) * Context::kArrivals;
+        if ((e = cudaMalloc(&ctx->d_counters, bytes)) != cudaSuccess)
             break;
-        if ((e = cudaMemset(ctx->d_flags, 0, sizeof(int) * FLAG_COUNT)) != cudaSuccess)
-            break;
-        if ((e = cudaMalloc(&ctx->d_counters, sizeof(long long) * kCounters)) != cudaSuccess)
-            break;
-        if ((e = cudaMemset(ctx->d_counters, 0, sizeof(long long) * kCounters)) != cudaSuccess)
-            break;
-        if ((e = cudaMalloc(&ctx->d_arrivals, sizeof(int) * Context::kArrivals)) != cudaSuccess)
-            break;
-        if ((e = cudaMemset(ctx->d_arrivals, 0, sizeof(int) * Context::kArrivals)) != cudaSuccess)
+        ctx->d_flags = reinterpret_cast<int*>(ctx->d_counters + kCounters);
+        ctx->d_arrivals = ctx->d_flags + FLAG_COUNT;
+        if ((e = cudaMemset(ctx->d_counters, 0, bytes)) != cudaSuccess)
             break;
         if ((e = cudaMallocHost(&ctx->h_flags, sizeof(int) * FLAG_COUNT)) != cudaSuccess)
             break;
@@ -290,6 +354,7 @@ int agwn_context_destroy(agwn_context* ctx)
         cudaStreamSynchronize(ctx->stream);
     for (auto& b : ctx->scratch)
         b.release();
+    ctx->arena.release();
     ctx->bernstein.release();
     ctx->ray_cache.h.release();
     ctx->ray_cache.cells.release();
@@ -300,12 +365,8 @@ int agwn_context_destroy(agwn_context* ctx)
         if (ctx->ev_end[i])
             cudaEventDestroy(ctx->ev_end[i]);
     }
-    if (ctx->d_flags)
-        cudaFree(ctx->d_flags);
     if (ctx->d_counters)
         cudaFree(ctx->d_counters);
-    if (ctx->d_arrivals)
-        cudaFree(ctx->d_arrivals);
     if (ctx->h_flags)
         cudaFreeHost(ctx->h_flags);
     for (cudaEvent_t e : ctx->pipe_ev)

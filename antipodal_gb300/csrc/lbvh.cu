@@ -707,34 +707,6 @@ __global__ void __launch_bounds__(kScanBlock) k_scan(const double* __restrict__ 
     }
 }
 
-// RAII device buffer for build temporaries.
-struct Tmp
-{
-    void* p = nullptr;
-    ~Tmp()
-    {
-        if (p)
-            cudaFree(p);
-    }
-    int alloc(size_t bytes)
-    {
-        cudaError_t const e = cudaMalloc(&p, bytes ? bytes : 1);
-        if (e != cudaSuccess)
-        {
-            cudaGetLastError();
-            p = nullptr;
-            return fail(e == cudaErrorMemoryAllocation ? AGWN_ERR_NOMEM : AGWN_ERR_CUDA, "cudaMalloc(%zu): %s", bytes,
-                        cudaGetErrorString(e));
-        }
-        return AGWN_OK;
-    }
-    template <class U>
-    U* as() const
-    {
-        return static_cast<U*>(p);
-    }
-};
-
 void bvh_free(Bvh* b)
 {
     if (b && b->tri)
@@ -763,7 +735,8 @@ int bvh_make(Context& ctx, const T* vertices, int64_t nv, const int32_t* indices
     AGWN_TRY(stage_in(ctx, vertices, sizeof(T) * 3 * nv, S_MISC0, &dv));
     AGWN_TRY(stage_in(ctx, indices, sizeof(int32_t) * n_idx, S_MISC1, &di));
     AGWN_TRY_CUDA(cudaMalloc(&out->tri, sizeof(T) * 9 * n_tri));
-    Tmp misc;
+    ArenaScope scope(ctx);
+    Tmp misc(ctx);
     AGWN_TRY(misc.alloc(sizeof(unsigned)));
     AGWN_TRY_CUDA(cudaMemsetAsync(misc.p, 0, sizeof(unsigned), st));
     AGWN_TRY_CUDA(cudaMemsetAsync(ctx.d_flags + FLAG_COUNT - 1, 0, sizeof(int), st));
@@ -822,10 +795,15 @@ int build_hier(Context& ctx, const T* tri_in, int64_t n_tri, const double* dir, 
     AGWN_CHECK_ARG(nn > 0 && std::isfinite(nn), "ray direction must be finite and nonzero");
     cudaStream_t const st = ctx.stream;
     Frame64 const f = ray_frame(dir);
-    AGWN_TRY_CUDA(cudaStreamSynchronize(st)); // the buffers may still be read by queued traversals
-    AGWN_TRY(out.tri.reserve(sizeof(T) * 9 * std::max<int64_t>(1, n_tri)));
-    AGWN_TRY(out.nodes.reserve(sizeof(BvhNode) * std::max<int64_t>(1, n_tri - 1)));
-    AGWN_TRY(out.leaf_uv.reserve(sizeof(float4) * kLeafF4 * std::max<int64_t>(1, n_tri)));
+    size_t const tri_bytes = sizeof(T) * 9 * std::max<int64_t>(1, n_tri);
+    size_t const node_bytes = sizeof(BvhNode) * std::max<int64_t>(1, n_tri - 1);
+    size_t const uv_bytes = sizeof(float4) * kLeafF4 * std::max<int64_t>(1, n_tri);
+    // growing buffers may still be read by queued traversals (rewriting them is ordered by the stream)
+    if (tri_bytes > out.tri.cap || node_bytes > out.nodes.cap || uv_bytes > out.leaf_uv.cap)
+        AGWN_TRY_CUDA(cudaStreamSynchronize(st));
+    AGWN_TRY(out.tri.reserve(tri_bytes));
+    AGWN_TRY(out.nodes.reserve(node_bytes));
+    AGWN_TRY(out.leaf_uv.reserve(uv_bytes));
     T* tri = static_cast<T*>(out.tri.ptr);
     int32_t depth = n_tri > 0 ? 1 : 0;
     unsigned scale_bits = 0;
@@ -837,7 +815,9 @@ int build_hier(Context& ctx, const T* tri_in, int64_t n_tri, const double* dir, 
     }
     if (n_tri > 1)
     {
-        Tmp box, cen, misc, keys0, vals0, keys1, vals1, hist, left, right, pnode, pleaf, nbox, visit, leafbox;
+        ArenaScope scope(ctx);
+        Tmp box(ctx), cen(ctx), misc(ctx), keys0(ctx), vals0(ctx), keys1(ctx), vals1(ctx), hist(ctx), left(ctx), right(ctx),
+            pnode(ctx), pleaf(ctx), nbox(ctx), visit(ctx), leafbox(ctx);
         AGWN_TRY(box.alloc(sizeof(float) * 6 * n_tri));
         AGWN_TRY(cen.alloc(sizeof(float) * 2 * n_tri));
         AGWN_TRY(misc.alloc(sizeof(unsigned) * 8));
@@ -847,7 +827,7 @@ int build_hier(Context& ctx, const T* tri_in, int64_t n_tri, const double* dir, 
         AGWN_TRY(vals1.alloc(sizeof(unsigned) * n_tri));
         int const n_rs_blocks = div_up(n_tri, kRsTile);
         AGWN_TRY(hist.alloc(sizeof(unsigned) * 256 * n_rs_blocks));
-        Tmp hsum;
+        Tmp hsum(ctx);
         AGWN_TRY(hsum.alloc(sizeof(unsigned) * scan_sums_count(int64_t(256) * n_rs_blocks)));
         AGWN_TRY(left.alloc(sizeof(int) * n_tri));
         AGWN_TRY(right.alloc(sizeof(int) * n_tri));
@@ -951,7 +931,8 @@ int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g)
     cudaStream_t const st = ctx.stream;
     float const margin = 4.f * scene_scale * 3.8146973e-6f;
     const float4* leaf_uv = static_cast<const float4*>(h.leaf_uv.ptr);
-    Tmp ext; // 4 order-encoded extents, then the 64-bit entry count
+    ArenaScope scope(ctx);
+    Tmp ext(ctx); // 4 order-encoded extents, then the 64-bit entry count
     AGWN_TRY(ext.alloc(sizeof(unsigned) * 6));
     unsigned const init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u};
     AGWN_TRY_CUDA(cudaMemcpyAsync(ext.p, init, sizeof(init), cudaMemcpyHostToDevice, st));
@@ -983,7 +964,7 @@ int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g)
     AGWN_TRY(g.offsets.reserve(sizeof(unsigned) * (n_cells + 1)));
     unsigned* const off = static_cast<unsigned*>(g.offsets.ptr);
     AGWN_TRY_CUDA(cudaMemsetAsync(off, 0, sizeof(unsigned) * (n_cells + 1), st));
-    Tmp osum;
+    Tmp osum(ctx);
     AGWN_TRY(osum.alloc(sizeof(unsigned) * scan_sums_count(n_cells + 1)));
     AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
     k_cell_bin<<<gl, 256, 0, st>>>(leaf_uv, n, margin, v, off, total64, nullptr, nullptr);
@@ -995,14 +976,13 @@ int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g)
     if (total >= (1ull << 31))
         return AGWN_OK; // the lists would not fit 32-bit offsets: keep the walk
     AGWN_TRY(g.list.reserve(sizeof(int) * std::max<unsigned long long>(1, total)));
-    Tmp cursor;
+    Tmp cursor(ctx);
     AGWN_TRY(cursor.alloc(sizeof(unsigned) * n_cells));
     AGWN_TRY_CUDA(cudaMemcpyAsync(cursor.p, off, sizeof(unsigned) * n_cells, cudaMemcpyDeviceToDevice, st));
     AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
     k_cell_bin<<<gl, 256, 0, st>>>(leaf_uv, n, margin, v, nullptr, nullptr, cursor.as<unsigned>(),
                                    static_cast<int*>(g.list.ptr));
     AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
-    AGWN_TRY_CUDA(cudaStreamSynchronize(st)); // the cursor is freed on return
     g.gu = v.gu;
     g.gv = v.gv;
     g.umin = v.umin;

@@ -26,28 +26,6 @@ namespace agwn
 {
 namespace
 {
-struct RTmp
-{
-    void* p = nullptr;
-    ~RTmp()
-    {
-        if (p)
-            cudaFree(p);
-    }
-    int alloc(size_t bytes)
-    {
-        cudaError_t const e = cudaMalloc(&p, bytes ? bytes : 1);
-        if (e != cudaSuccess)
-        {
-            cudaGetLastError();
-            p = nullptr;
-            return fail(e == cudaErrorMemoryAllocation ? AGWN_ERR_NOMEM : AGWN_ERR_CUDA, "cudaMalloc(%zu): %s", bytes,
-                        cudaGetErrorString(e));
-        }
-        return AGWN_OK;
-    }
-};
-
 void robust_free(Robust* r)
 {
     if (!r)
@@ -77,6 +55,7 @@ int robust_build(Context& ctx, const T* vertices, int64_t nv, const int32_t* ind
     out->device = ctx.device;
     out->scalar_bytes = int(sizeof(T));
     cudaStream_t const st = ctx.stream;
+    ArenaScope scope(ctx);
     const void *dv = nullptr, *di = nullptr, *db = nullptr;
     AGWN_TRY(stage_in(ctx, vertices, sizeof(T) * 3 * nv, S_MISC0, &dv));
     AGWN_TRY(stage_in(ctx, indices, sizeof(int32_t) * n_idx, S_MISC1, &di));
@@ -85,7 +64,7 @@ int robust_build(Context& ctx, const T* vertices, int64_t nv, const int32_t* ind
     Quant qz{{0, 0, 0}, 1.0};
     if (P::grid && nv > 0)
     {
-        RTmp bb;
+        Tmp bb(ctx);
         AGWN_TRY(bb.alloc(sizeof(unsigned long long) * 6));
         unsigned long long init[6] = {~0ull, ~0ull, ~0ull, 0, 0, 0};
         AGWN_TRY_CUDA(cudaMemcpyAsync(bb.p, init, sizeof(init), cudaMemcpyHostToDevice, st));
@@ -114,7 +93,7 @@ int robust_build(Context& ctx, const T* vertices, int64_t nv, const int32_t* ind
     int const g = std::min(div_up(std::max<int64_t>(n_tri, n_seg), 256), 8 * ctx.sm_count);
     if (n_tri > 0)
     {
-        RTmp tq, td, order;
+        Tmp tq(ctx), td(ctx), order(ctx);
         AGWN_TRY(tq.alloc(sizeof(C) * 9 * n_tri));
         AGWN_TRY(td.alloc(sizeof(double) * 9 * n_tri));
         AGWN_TRY(order.alloc(sizeof(unsigned) * n_tri));
@@ -155,7 +134,7 @@ int robust_build(Context& ctx, const T* vertices, int64_t nv, const int32_t* ind
         {
             // the chains of the mixed form's FP32 pairs
             AGWN_TRY_CUDA(cudaMalloc(&out->chain, sizeof(RChain) * 2 * size_t(n_seg)));
-            RTmp order, cnt;
+            Tmp order(ctx), cnt(ctx);
             AGWN_TRY(order.alloc(sizeof(int) * std::max<int64_t>(1, chain_scratch_ints(n_seg))));
             AGWN_TRY(cnt.alloc(sizeof(long long)));
             AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
@@ -216,6 +195,14 @@ int robust_count_chunk(void* user, Context& ctx, const double* d_pos, int64_t m,
     return ctx.launch_end(AGWN_K_ROBUST);
 }
 
+// The evaluator's cell grid, complete on return: other contexts may use the evaluator next.
+int robust_cells(Context& ctx, const Robust& r)
+{
+    AGWN_TRY(build_cells(ctx, r.hier, float(r.hier.scale), r.cells));
+    AGWN_TRY_CUDA(cudaStreamSynchronize(ctx.stream));
+    return AGWN_OK;
+}
+
 template <class T, class P>
 int robust_run(Context& ctx, const Robust& r, const T* d_pos, int64_t n, T* d_out, int32_t* d_counts, T* d_frac,
                bool counts_ready = false)
@@ -232,7 +219,7 @@ int robust_run(Context& ctx, const Robust& r, const T* d_pos, int64_t n, T* d_ou
             ctx.use_mixed(double(n) * double(r.n_seg), r.n_seg))
         {
             if (!r.cells.valid)
-                AGWN_TRY(build_cells(ctx, r.hier, float(r.hier.scale), r.cells));
+                AGWN_TRY(robust_cells(ctx, r));
             if (r.cells.valid)
             {
                 double* raw = nullptr;
@@ -261,7 +248,7 @@ int robust_run(Context& ctx, const Robust& r, const T* d_pos, int64_t n, T* d_ou
             f.r[k] = r.hier.frame[k];
         int const grid = int(std::min<int64_t>(div_up(n, kRobBlock), int64_t(ctx.sm_count) * 16));
         if (ctx.integer_cells && r.n_tri > 1 && !r.cells.valid)
-            AGWN_TRY(build_cells(ctx, r.hier, float(r.hier.scale), r.cells));
+            AGWN_TRY(robust_cells(ctx, r));
         if (ctx.integer_cells && r.n_tri > 1 && r.cells.valid)
         {
             AGWN_TRY(ctx.launch_begin(AGWN_K_ROBUST));

@@ -559,10 +559,13 @@ template <class T>
                                                          reinterpret_cast<float*>(out), cap, n),
                         "build_boundary_segments");
     };
+    // most boundaries fit the first call's rows; a longer one takes a second call with its count
     std::int64_t n = 0;
-    run(nullptr, 0, &n);
-    std::vector<weighted_segment3<T>> out(static_cast<std::size_t>(n));
-    if (n > 0)
+    std::vector<weighted_segment3<T>> out(4096);
+    run(out.data(), std::int64_t(out.size()), &n);
+    bool const more = n > std::int64_t(out.size());
+    out.resize(static_cast<std::size_t>(n));
+    if (more)
         run(out.data(), n, &n);
     return out;
 }
