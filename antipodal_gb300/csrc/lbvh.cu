@@ -475,30 +475,43 @@ __global__ void k_cell_extent(const float4* __restrict__ leaf_uv, int64_t n, flo
         }
 }
 
-// counts[c] += 1 for every cell c of every leaf (cursor == nullptr), or the leaf written at its slot of each of
-// its cells (cursor: a copy of the offsets)
-__global__ void k_cell_bin(const float4* __restrict__ leaf_uv, int64_t n, float margin, CellView g,
-                           unsigned* __restrict__ counts, unsigned long long* __restrict__ total,
-                           unsigned* __restrict__ cursor, int* __restrict__ list)
+// counts[c] += 1 for every cell c of every leaf (cursor == nullptr), or the leaf written at its slot of each of its
+// cells (cursor: a copy of the offsets).  A leaf covers some 30 cells, each an atomic operation: kBinLanes lanes take
+// them side by side (one lane per leaf, with one counter for all entries, took 110 us a pass over 76,496 leaves, now 40).
+constexpr int kBinLanes = 8;
+__global__ void __launch_bounds__(256) k_cell_bin(const float4* __restrict__ leaf_uv, int64_t n, float margin, CellView g,
+                                                  unsigned* __restrict__ counts, unsigned long long* __restrict__ total,
+                                                  unsigned* __restrict__ cursor, int* __restrict__ list)
 {
-    for (int64_t l = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; l < n; l += int64_t(gridDim.x) * blockDim.x)
+    int const lane = threadIdx.x % kBinLanes;
+    int64_t const stride = int64_t(gridDim.x) * (blockDim.x / kBinLanes);
+    unsigned long long entries = 0;
+    for (int64_t l = blockIdx.x * int64_t(blockDim.x / kBinLanes) + threadIdx.x / kBinLanes; l < n; l += stride)
     {
         float u0, v0, u1, v1;
         if (!leaf_box_uv(leaf_uv, l, margin, u0, v0, u1, v1))
             continue;
-        int const iu0 = cell_of(u0, g.umin, g.inv_u, g.gu), iu1 = cell_of(u1, g.umin, g.inv_u, g.gu);
-        int const iv0 = cell_of(v0, g.vmin, g.inv_v, g.gv), iv1 = cell_of(v1, g.vmin, g.inv_v, g.gv);
-        if (total)
-            atomicAdd(total, (unsigned long long)(iu1 - iu0 + 1) * (unsigned long long)(iv1 - iv0 + 1));
-        for (int iv = iv0; iv <= iv1; ++iv)
-            for (int iu = iu0; iu <= iu1; ++iu)
-            {
-                int64_t const c = int64_t(iv) * g.gu + iu;
-                if (cursor)
-                    list[atomicAdd(cursor + c, 1u)] = int(l);
-                else
-                    atomicAdd(counts + c, 1u);
-            }
+        int const iu0 = cell_of(u0, g.umin, g.inv_u, g.gu), w = cell_of(u1, g.umin, g.inv_u, g.gu) - iu0 + 1;
+        int const iv0 = cell_of(v0, g.vmin, g.inv_v, g.gv), h = cell_of(v1, g.vmin, g.inv_v, g.gv) - iv0 + 1;
+        int64_t const cells = int64_t(w) * h;
+        if (lane == 0)
+            entries += (unsigned long long)cells;
+        for (int64_t k = lane; k < cells; k += kBinLanes)
+        {
+            int64_t const row = cells < (1 << 24) ? int(k) / w : k / w;
+            int64_t const c = (iv0 + row) * g.gu + iu0 + (k - row * w);
+            if (cursor)
+                list[atomicAdd(cursor + c, 1u)] = int(l);
+            else
+                atomicAdd(counts + c, 1u);
+        }
+    }
+    if (total)
+    {
+        for (int o = 16; o > 0; o >>= 1)
+            entries += __shfl_xor_sync(0xffffffffu, entries, o);
+        if ((threadIdx.x & 31) == 0 && entries)
+            atomicAdd(total, entries);
     }
 }
 
@@ -967,7 +980,8 @@ int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g)
     Tmp osum(ctx);
     AGWN_TRY(osum.alloc(sizeof(unsigned) * scan_sums_count(n_cells + 1)));
     AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-    k_cell_bin<<<gl, 256, 0, st>>>(leaf_uv, n, margin, v, off, total64, nullptr, nullptr);
+    int const gb = int(std::min<int64_t>(div_up(n * kBinLanes, 256), 32 * int64_t(ctx.sm_count)));
+    k_cell_bin<<<gb, 256, 0, st>>>(leaf_uv, n, margin, v, off, total64, nullptr, nullptr);
     scan_counters(st, off, n_cells + 1, osum.as<unsigned>());
     AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
     unsigned long long total = 0;
@@ -980,7 +994,7 @@ int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g)
     AGWN_TRY(cursor.alloc(sizeof(unsigned) * n_cells));
     AGWN_TRY_CUDA(cudaMemcpyAsync(cursor.p, off, sizeof(unsigned) * n_cells, cudaMemcpyDeviceToDevice, st));
     AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-    k_cell_bin<<<gl, 256, 0, st>>>(leaf_uv, n, margin, v, nullptr, nullptr, cursor.as<unsigned>(),
+    k_cell_bin<<<gb, 256, 0, st>>>(leaf_uv, n, margin, v, nullptr, nullptr, cursor.as<unsigned>(),
                                    static_cast<int*>(g.list.ptr));
     AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
     g.gu = v.gu;
