@@ -110,6 +110,7 @@ struct Hier
     int64_t n_tri = 0;
     float frame[9] = {};
     double scale = 1.0; // largest |coordinate| of the triangles
+    float ext[4] = {};  // min u, min v, max u, max v of the leaves' float corners (min above max: none finite)
     void release()
     {
         nodes.release();
@@ -129,6 +130,8 @@ struct CellGrid
     float margin = 0;  // the widening of every leaf's box
     float tol_max = 0; // queries whose own tolerance exceeds this take the hierarchy walk
     int64_t entries = 0;
+    int per_leaf = 0;   // cells per leaf it was built with
+    int64_t served = 0; // queries prepared for on this hierarchy so far
     bool valid = false;
     void release()
     {

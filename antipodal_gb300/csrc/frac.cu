@@ -403,7 +403,7 @@ int mesh_batch_pipelined(Context& ctx, const agwn_bvh* bvh, const T* positions, 
     FracPlan<T> plan;
     AGWN_TRY(fractional_prepare<T>(ctx, x0, dseg, want_frac ? n_seg : 0, n, &plan));
     if (with_int && n >= 1)
-        AGWN_TRY(integer_prepare<T>(ctx, *bvh, x0)); // the hierarchy and its cell grid, built on the main stream
+        AGWN_TRY(integer_prepare<T>(ctx, *bvh, x0, n)); // the hierarchy and its cell grid, built on the main stream
     AGWN_TRY_CUDA(cudaEventRecord(ready, main));
     AGWN_TRY_CUDA(cudaStreamWaitEvent(cs[1], ready, 0));
     int64_t const n_chunks = (n + chunk - 1) / chunk;
@@ -424,7 +424,7 @@ int mesh_batch_pipelined(Context& ctx, const agwn_bvh* bvh, const T* positions, 
             AGWN_TRY_CUDA(cudaStreamWaitEvent(cs[b], down[b], 0));
         ctx.stream = cs[b]; // the launches below go to this chunk's compute stream
         if (with_int)
-            rc = integer_run<T>(ctx, *bvh, qb, m, cb, x0);
+            rc = integer_run<T>(ctx, *bvh, qb, m, cb, x0, true);
         if (rc == AGWN_OK)
             rc = fractional_launch<T>(ctx, plan, qb, m, ob, cb);
         ctx.stream = main;
@@ -472,7 +472,7 @@ int mesh_batch_chunked(Context& ctx, const agwn_bvh* bvh, const T* dpos, int64_t
     FracPlan<T> plan;
     AGWN_TRY(fractional_prepare<T>(ctx, x0, dseg, n_seg, n, &plan));
     if (with_int)
-        AGWN_TRY(integer_prepare<T>(ctx, *bvh, x0));
+        AGWN_TRY(integer_prepare<T>(ctx, *bvh, x0, n));
     AGWN_TRY_CUDA(cudaEventRecord(ready, main));
     AGWN_TRY_CUDA(cudaStreamWaitEvent(cs[1], ready, 0));
     int64_t const n_chunks = (n + chunk - 1) / chunk;
@@ -483,7 +483,7 @@ int mesh_batch_chunked(Context& ctx, const agwn_bvh* bvh, const T* dpos, int64_t
         int32_t* const cb = with_int ? dcounts + q0 : nullptr;
         ctx.stream = cs[i & 1]; // the launches below go to this chunk's compute stream
         if (with_int)
-            rc = integer_run<T>(ctx, *bvh, dpos + 3 * q0, m, cb, x0);
+            rc = integer_run<T>(ctx, *bvh, dpos + 3 * q0, m, cb, x0, true);
         if (rc == AGWN_OK)
             rc = fractional_launch<T>(ctx, plan, dpos + 3 * q0, m, dout + q0, cb);
         ctx.stream = main;

@@ -38,12 +38,14 @@ int frac_mixed_robust_pf_chunked(Context& ctx, const double* d_pos, int64_t n, d
                                  const double* d_raw, int64_t n_seg, const void* rseg, ChunkCounts count,
                                  void* user);
 
-// Integer term over a BVH for `n` device-resident queries.
+// Integer term over a BVH for `n` device-resident queries.  prepared: integer_prepare has run for them (the chunks of a
+// call, which must not rebuild what the other stream's chunks read).
 template <class T>
-int integer_run(Context& ctx, const Bvh& bvh, const T* d_pos, int64_t n, int32_t* d_counts, const T* dir_host);
-// The hierarchy along dir_host and its cell grid (when enabled), built on ctx.stream unless cached.
+int integer_run(Context& ctx, const Bvh& bvh, const T* d_pos, int64_t n, int32_t* d_counts, const T* dir_host,
+                bool prepared = false);
+// The hierarchy along dir_host and its cell grid (when enabled) for n more queries, built on ctx.stream unless cached.
 template <class T>
-int integer_prepare(Context& ctx, const Bvh& bvh, const T* dir_host);
+int integer_prepare(Context& ctx, const Bvh& bvh, const T* dir_host, int64_t n);
 
 // Spatial order of the queries for the mixed kernels (order.cu).  For n >= kOrderMinQueries device-resident
 // queries whose order is incoherent across the direction dir (3 doubles, host), *perm receives a permutation (device

@@ -314,8 +314,10 @@ __device__ __forceinline__ void integer_stats(long long* counters, long long que
     }
 }
 
-// Builds the cell grid of hierarchy h (lbvh.cu); leaves g invalid when a grid does not apply.
-int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g);
+// Builds the cell grid of hierarchy h with about per_leaf cells per leaf (lbvh.cu); leaves g invalid when a grid does
+// not apply.
+constexpr int kCellsFine = 16, kCellsCoarse = 2;
+int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g, int per_leaf = kCellsFine);
 
 // Orthonormal frame whose third row is dir / |dir|.
 Frame64 ray_frame(const double* dir);

@@ -222,12 +222,14 @@ __global__ void k_karras(const unsigned* __restrict__ keys, int n, int* __restri
 }
 
 // Leaf setup: each sorted triangle's world-space vertices, its ray-frame box and its vertices projected on the
-// (u, v) plane (rounded to float; 8 floats per leaf: u0 v0 u1 v1 u2 v2 0 0) into leaf order.
+// (u, v) plane (rounded to float; 8 floats per leaf: u0 v0 u1 v1 u2 v2 0 0) into leaf order.  ext: min u, min v, max u,
+// max v of the corners of the leaves without a NaN, order-encoded.
 template <class T>
 __global__ void k_leaves(const T* __restrict__ tri_in, const unsigned* __restrict__ order,
                          const float* __restrict__ box, int64_t n_tri, Frame64 f, T* __restrict__ tri,
-                         float* __restrict__ leaf_box, float* __restrict__ leaf_uv)
+                         float* __restrict__ leaf_box, float* __restrict__ leaf_uv, unsigned* ext)
 {
+    unsigned mn[2] = {0xFFFFFFFFu, 0xFFFFFFFFu}, mx[2] = {0u, 0u};
     for (int64_t l = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; l < n_tri; l += int64_t(gridDim.x) * blockDim.x)
     {
         unsigned const t = order[l];
@@ -245,7 +247,27 @@ __global__ void k_leaves(const T* __restrict__ tri_in, const unsigned* __restric
             o[6 + v] = float(f.r[6] * x + f.r[7] * y + f.r[8] * z);
         }
         o[9] = o[10] = o[11] = 0.f;
+        if (!(isnan(o[0]) || isnan(o[1]) || isnan(o[2]) || isnan(o[3]) || isnan(o[4]) || isnan(o[5])))
+            for (int v = 0; v < 3; ++v)
+                for (int k = 0; k < 2; ++k)
+                {
+                    unsigned const u = float_flip(o[2 * v + k]);
+                    mn[k] = min(mn[k], u);
+                    mx[k] = max(mx[k], u);
+                }
     }
+    for (int k = 0; k < 2; ++k)
+        for (int o = 16; o > 0; o >>= 1)
+        {
+            mn[k] = min(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
+            mx[k] = max(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+        }
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < 2; ++k)
+        {
+            atomicMin(ext + k, mn[k]);
+            atomicMax(ext + 2 + k, mx[k]);
+        }
 }
 
 __global__ void k_refit(int n, const int* __restrict__ left, const int* __restrict__ right,
@@ -419,12 +441,7 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(const BvhNode* __restri
 // and they go through the same conditions -- top of the leaf above the query's depth, may_hit -- and the same
 // decision, so the counts are the walk's.  Neighbouring rays share cells, so the lists and leaves are read
 // coherently, and there is no stack.
-// Order-preserving encodings of floats as unsigned (for atomic min / max).
-__device__ __forceinline__ unsigned f2o(float x)
-{
-    unsigned const b = __float_as_uint(x);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
+// The float of an order-preserving encoding (float_flip).
 float o2f(unsigned o)
 {
     unsigned const b = (o & 0x80000000u) ? (o & 0x7FFFFFFFu) : ~o;
@@ -445,34 +462,6 @@ __device__ __forceinline__ bool leaf_box_uv(const float4* __restrict__ leaf_uv, 
     v1 = fmaxf(fmaxf(a.y, a.w), b.y) + margin;
     bool const nan = isnan(a.x) || isnan(a.y) || isnan(a.z) || isnan(a.w) || isnan(b.x) || isnan(b.y);
     return !nan && u0 <= u1 && v0 <= v1;
-}
-
-// ext: min u, min v, max u, max v of the widened boxes, order-encoded
-__global__ void k_cell_extent(const float4* __restrict__ leaf_uv, int64_t n, float margin, unsigned* ext)
-{
-    unsigned mn[2] = {0xFFFFFFFFu, 0xFFFFFFFFu}, mx[2] = {0u, 0u};
-    for (int64_t l = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; l < n; l += int64_t(gridDim.x) * blockDim.x)
-    {
-        float u0, v0, u1, v1;
-        if (!leaf_box_uv(leaf_uv, l, margin, u0, v0, u1, v1))
-            continue;
-        mn[0] = min(mn[0], f2o(u0));
-        mn[1] = min(mn[1], f2o(v0));
-        mx[0] = max(mx[0], f2o(u1));
-        mx[1] = max(mx[1], f2o(v1));
-    }
-    for (int k = 0; k < 2; ++k)
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            mn[k] = min(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
-            mx[k] = max(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
-        }
-    if ((threadIdx.x & 31) == 0)
-        for (int k = 0; k < 2; ++k)
-        {
-            atomicMin(ext + k, mn[k]);
-            atomicMax(ext + 2 + k, mx[k]);
-        }
 }
 
 // counts[c] += 1 for every cell c of every leaf (cursor == nullptr), or the leaf written at its slot of each of its
@@ -833,7 +822,7 @@ int build_hier(Context& ctx, const T* tri_in, int64_t n_tri, const double* dir, 
             pnode(ctx), pleaf(ctx), nbox(ctx), visit(ctx), leafbox(ctx);
         AGWN_TRY(box.alloc(sizeof(float) * 6 * n_tri));
         AGWN_TRY(cen.alloc(sizeof(float) * 2 * n_tri));
-        AGWN_TRY(misc.alloc(sizeof(unsigned) * 8));
+        AGWN_TRY(misc.alloc(sizeof(unsigned) * 12));
         AGWN_TRY(keys0.alloc(sizeof(unsigned) * n_tri));
         AGWN_TRY(vals0.alloc(sizeof(unsigned) * n_tri));
         AGWN_TRY(keys1.alloc(sizeof(unsigned) * n_tri));
@@ -849,8 +838,8 @@ int build_hier(Context& ctx, const T* tri_in, int64_t n_tri, const double* dir, 
         AGWN_TRY(nbox.alloc(sizeof(float) * 6 * n_tri));
         AGWN_TRY(visit.alloc(sizeof(int) * n_tri));
         AGWN_TRY(leafbox.alloc(sizeof(float) * 6 * n_tri));
-        // (u, v) min, (u, v) max, largest |coordinate| bits, -, -, depth
-        unsigned init[8] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u, 0u};
+        // (u, v) min, (u, v) max of the centroids, largest |coordinate| bits, -, -, depth, (u, v) min and max of the corners
+        unsigned init[12] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u, 0u, 0u, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u};
         AGWN_TRY_CUDA(cudaMemcpyAsync(misc.p, init, sizeof(init), cudaMemcpyHostToDevice, st));
         AGWN_TRY_CUDA(cudaMemsetAsync(visit.p, 0, sizeof(int) * n_tri, st));
         int const g = std::min(div_up(n_tri, 256), 8 * ctx.sm_count);
@@ -873,7 +862,7 @@ int build_hier(Context& ctx, const T* tri_in, int64_t n_tri, const double* dir, 
             std::swap(va, vb);
         }
         k_leaves<T><<<g, 256, 0, st>>>(tri_in, va, box.as<float>(), n_tri, f, tri, leafbox.as<float>(),
-                                       static_cast<float*>(out.leaf_uv.ptr));
+                                       static_cast<float*>(out.leaf_uv.ptr), misc.as<unsigned>() + 8);
         k_karras<<<gb, 256, 0, st>>>(ka, int(n_tri), left.as<int>(), right.as<int>(), pnode.as<int>(),
                                      pleaf.as<int>());
         k_refit<<<gb, 256, 0, st>>>(int(n_tri), left.as<int>(), right.as<int>(), pnode.as<int>(), pleaf.as<int>(),
@@ -884,11 +873,13 @@ int build_hier(Context& ctx, const T* tri_in, int64_t n_tri, const double* dir, 
         AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
         if (order_out)
             AGWN_TRY_CUDA(cudaMemcpyAsync(order_out, va, sizeof(unsigned) * n_tri, cudaMemcpyDeviceToDevice, st));
-        unsigned back[8];
+        unsigned back[12];
         AGWN_TRY_CUDA(cudaMemcpyAsync(back, misc.p, sizeof(back), cudaMemcpyDeviceToHost, st));
         AGWN_TRY_CUDA(cudaStreamSynchronize(st));
         depth = int32_t(back[7]);
         scale_bits = back[4];
+        for (int k = 0; k < 4; ++k)
+            out.ext[k] = back[8] == 0xFFFFFFFFu ? (k < 2 ? INFINITY : -INFINITY) : o2f(back[8 + k]);
         if (depth > n_tri)
             return fail(AGWN_ERR_CUDA, "hierarchy build produced a broken parent chain (depth %d for %lld triangles)",
                         depth, (long long)n_tri);
@@ -919,6 +910,7 @@ int ray_hierarchy(Context& ctx, const Bvh& bvh, const T* dir_host)
         return AGWN_OK;
     rc.generation = 0; // invalid until the build completes
     rc.cells.valid = false;
+    rc.cells.served = 0;
     AGWN_TRY(build_hier<T>(ctx, static_cast<const T*>(bvh.tri), bvh.n_tri, dir, rc.h, nullptr));
     std::memcpy(rc.dir, dir, sizeof(dir));
     rc.scalar_bytes = bvh.scalar_bytes;
@@ -928,14 +920,15 @@ int ray_hierarchy(Context& ctx, const Bvh& bvh, const T* dir_host)
 }
 } // namespace
 
-// The cell grid of the cached hierarchy (its leaves' float (u, v) corners), about 16 cells per leaf over the
+// The cell grid of the cached hierarchy (its leaves' float (u, v) corners), about per_leaf cells per leaf over the
 // widened boxes' extent (at most 2^22 cells).  Finer cells hold fewer leaves, so a query reads fewer list entries:
 // on a 76,496-triangle icosphere with 256^3 grid queries 2 cells per leaf read 5.06 entries per query (1.09 ms),
-// 16 read 3.49 (0.83 ms); 32 and 64 gained no more.  Leaf boxes are widened by 4 * 2^-18 of the scene scale; a
+// 16 read 3.49 (0.83 ms); 32 and 64 gained no more.  But a fine grid takes longer to build (two passes of 40 us against 16
+// there), so a mesh starts with 2 and takes 16 when its queries so far could repay it (integer_prepare).  Leaf boxes are widened by 4 * 2^-18 of the scene scale; a
 // query takes the grid while its own tolerance (qmax + scene) * 2^-18 stays below 3.5 * 2^-18 of the scene scale
 // (qmax <= 2.5 * scene), which leaves room for the one-ulp difference between the corners and the walk's
 // outward-rounded boxes.
-int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g)
+int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g, int per_leaf)
 {
     g.valid = false;
     int64_t const n = h.n_tri;
@@ -945,29 +938,22 @@ int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g)
     float const margin = 4.f * scene_scale * 3.8146973e-6f;
     const float4* leaf_uv = static_cast<const float4*>(h.leaf_uv.ptr);
     ArenaScope scope(ctx);
-    Tmp ext(ctx); // 4 order-encoded extents, then the 64-bit entry count
-    AGWN_TRY(ext.alloc(sizeof(unsigned) * 6));
-    unsigned const init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u, 0u};
-    AGWN_TRY_CUDA(cudaMemcpyAsync(ext.p, init, sizeof(init), cudaMemcpyHostToDevice, st));
-    auto* const total64 = reinterpret_cast<unsigned long long*>(ext.as<unsigned>() + 4);
-    int const gl = std::min(div_up(n, 256), 8 * ctx.sm_count);
-    AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-    k_cell_extent<<<gl, 256, 0, st>>>(leaf_uv, n, margin, ext.as<unsigned>());
-    AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
-    unsigned back[4];
-    AGWN_TRY_CUDA(cudaMemcpyAsync(back, ext.p, sizeof(back), cudaMemcpyDeviceToHost, st));
-    AGWN_TRY_CUDA(cudaStreamSynchronize(st));
-    if (back[0] == 0xFFFFFFFFu)
+    Tmp total_buf(ctx);
+    AGWN_TRY(total_buf.alloc(sizeof(unsigned long long)));
+    auto* const total64 = total_buf.as<unsigned long long>();
+    AGWN_TRY_CUDA(cudaMemsetAsync(total64, 0, sizeof(unsigned long long), st));
+    if (!(h.ext[0] <= h.ext[2]))
         return AGWN_OK; // no leaf with a finite box: keep the walk
+    // the extent of the widened boxes (rounding is monotone, so widening the extent widens every box)
     CellView v{};
-    v.umin = o2f(back[0]);
-    v.vmin = o2f(back[1]);
-    v.umax = o2f(back[2]);
-    v.vmax = o2f(back[3]);
+    v.umin = h.ext[0] - margin;
+    v.vmin = h.ext[1] - margin;
+    v.umax = h.ext[2] + margin;
+    v.vmax = h.ext[3] + margin;
     double const W = double(v.umax) - double(v.umin), H = double(v.vmax) - double(v.vmin);
     if (!(W > 0) || !(H > 0) || !std::isfinite(W) || !std::isfinite(H))
         return AGWN_OK;
-    double const target = double(std::min<int64_t>(std::max<int64_t>(16 * n, 1024), int64_t(1) << 22));
+    double const target = double(std::min<int64_t>(std::max<int64_t>(per_leaf * n, 1024), int64_t(1) << 22));
     double const side = std::sqrt(W * H / target);
     v.gu = int(std::min(4096.0, std::max(1.0, std::ceil(W / side))));
     v.gv = int(std::min(4096.0, std::max(1.0, std::ceil(H / side))));
@@ -1008,27 +994,35 @@ int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g)
     g.margin = margin;
     g.tol_max = 3.5f * scene_scale * 3.8146973e-6f;
     g.entries = int64_t(total);
+    g.per_leaf = per_leaf;
     g.valid = true;
     return AGWN_OK;
 }
 
 template <class T>
-int integer_prepare(Context& ctx, const Bvh& bvh, const T* dir_host)
+int integer_prepare(Context& ctx, const Bvh& bvh, const T* dir_host, int64_t n)
 {
     if (bvh.n_tri == 0)
         return AGWN_OK;
     AGWN_TRY(ray_hierarchy<T>(ctx, bvh, dir_host));
     CellGrid& cg = ctx.ray_cache.cells;
-    if (ctx.integer_cells && bvh.n_tri > 1 && !cg.valid)
-        AGWN_TRY(build_cells(ctx, ctx.ray_cache.h, float(bvh.scene_scale), cg));
+    if (!ctx.integer_cells || bvh.n_tri <= 1)
+        return AGWN_OK;
+    // The fine grid costs about 1 ns per leaf more to build and saves 0.016 ns per query, so it comes once 32 queries
+    // per leaf have been asked for (in one call or over many); until then the coarse one.
+    cg.served += n;
+    int const per_leaf = cg.served / 32 >= bvh.n_tri ? kCellsFine : kCellsCoarse;
+    if (!cg.valid || cg.per_leaf < per_leaf)
+        AGWN_TRY(build_cells(ctx, ctx.ray_cache.h, float(bvh.scene_scale), cg, per_leaf));
     return AGWN_OK;
 }
 
-template int integer_prepare<double>(Context&, const Bvh&, const double*);
-template int integer_prepare<float>(Context&, const Bvh&, const float*);
+template int integer_prepare<double>(Context&, const Bvh&, const double*, int64_t);
+template int integer_prepare<float>(Context&, const Bvh&, const float*, int64_t);
 
 template <class T>
-int integer_run(Context& ctx, const Bvh& bvh, const T* d_pos, int64_t n, int32_t* d_counts, const T* dir_host)
+int integer_run(Context& ctx, const Bvh& bvh, const T* d_pos, int64_t n, int32_t* d_counts, const T* dir_host,
+                bool prepared)
 {
     if (n == 0)
         return AGWN_OK;
@@ -1037,7 +1031,8 @@ int integer_run(Context& ctx, const Bvh& bvh, const T* d_pos, int64_t n, int32_t
         AGWN_TRY_CUDA(cudaMemsetAsync(d_counts, 0, sizeof(int32_t) * n, ctx.stream));
         return AGWN_OK;
     }
-    AGWN_TRY(integer_prepare<T>(ctx, bvh, dir_host));
+    if (!prepared)
+        AGWN_TRY(integer_prepare<T>(ctx, bvh, dir_host, n));
     Frame32 f;
     for (int k = 0; k < 9; ++k)
         f.r[k] = ctx.ray_cache.h.frame[k];
@@ -1065,8 +1060,8 @@ int integer_run(Context& ctx, const Bvh& bvh, const T* d_pos, int64_t n, int32_t
     return ctx.launch_end(AGWN_K_INTEGER);
 }
 
-template int integer_run<double>(Context&, const Bvh&, const double*, int64_t, int32_t*, const double*);
-template int integer_run<float>(Context&, const Bvh&, const float*, int64_t, int32_t*, const float*);
+template int integer_run<double>(Context&, const Bvh&, const double*, int64_t, int32_t*, const double*, bool);
+template int integer_run<float>(Context&, const Bvh&, const float*, int64_t, int32_t*, const float*, bool);
 
 namespace
 {
