@@ -8,8 +8,7 @@
 // `left + right` summation (post-order).  Two arithmetic forms:
 //  * exact -- the integrand and the G7/K15 sums in FP64, unfused, in the reference's order (k_param_exact): the
 //    result equals the CPU reference bit for bit.
-//  * mixed -- double-float arithmetic on the FP32 pipe (k_param_gk15), curves staged in shared memory by
-//    cp.async.bulk.
+//  * mixed -- double-float arithmetic on the FP32 pipe (k_param_gk15).
 //
 // Proposal hook: a per-(query, curve) start depth s (from the learned proposal; 0 for the plain method).  Panels
 // above depth s are split without being evaluated; every panel at depth >= s is evaluated and accepted or split by
@@ -20,7 +19,6 @@
 #include "df32.cuh"
 #include "hier.cuh"
 #include "mlp.cuh"
-#include "tma.cuh"
 
 #include <cmath>
 
@@ -30,12 +28,6 @@ namespace
 {
 constexpr int kParamMaxDepth = 24; // deepest panel the integrator can reach (2^24 panels per curve)
 constexpr int kParamBlock = 128;
-// The double-float form stages 384 curves (36 KB, room for the per-panel network's weights beside them), so that
-// six blocks reside per SM, the number its 80 registers allow.  Measured on 256 bicubic patches at tol 1e-10:
-// 40K queries, 768 was 10% faster than 1024 and flat down to 128; 250K queries (one work item per query block),
-// 384 is 1.7% faster than 768 (three blocks per SM) and 256 1.4%.
-constexpr int kParamTileDF = 384;
-
 // G7-K15 abscissae and weights: the published Gauss-Kronrod constants at the precision the reference carries
 // (integrate_gk15.hh:13-36); identical doubles make the sums identical.
 __constant__ double kGkX[8] = {0.0,
@@ -528,20 +520,18 @@ __global__ void k_param_sum(const double* __restrict__ vals, int nq, int nc, boo
     out[i] = last ? (sum / (rd(4.0) * rd(3.141592653589793238462643383279502884))).v : sum.v;
 }
 
-// out[q] = (sum over curves of the curve integral) / (4 pi).
+// Pair integrals in the double-float form: vals[k * nq + i] for the curves c0 + k and the queries q0 + i.
 //
-// The double-float form.  The cost of one (query, curve) integral is heavy-tailed, so the work is shared out by pair,
-// not by query.  A block owns up to kParamBlock
-// queries and, for each shared-memory tile of curves, the pool of (query, curve) pairs of that tile; a lane that
-// finishes its pair takes the next one from the pool (one shared-memory atomic per warp).  Each lane walks its
-// pair's panel tree as a team of the exact form does.  A finished pair's integral goes to the block's slab of `pair_vals`; after the tile each thread
-// adds its query's row in curve order.  Every sum is the reference's (post-order left + right within a curve,
-// curves in order), so the result does not depend on how the pairs were shared out.
+// The FMA pipe's chains bound it (a lane per pair: some 320 dependent FP32 operations a node, 15 nodes a panel).  The
+// cost of one (query, curve) integral is heavy-tailed, so the lanes of the whole grid draw their pairs from one counter
+// (a warp takes `take`, 32 or 64, at a time) and walk their panel trees as a team of the exact form does; k_param_sum adds a
+// query's integrals in curve order.  With blocks of 128 queries x 128 curves as the unit, 20,000 queries x 1,024 curves
+// made 1.4 waves of them and each block waited for its deepest pair: the whole call 34.5 -> 31.5 ms.
 //
 // start_depth: per (query, curve), row-major [n][n_curves], nullable = all 0.  stats (nullable): per (query,
-// curve) packed as leaves | shallowest leaf depth << 16 | deepest leaf depth << 24.  nodes_total (nullable):
-// panels evaluated per query.  pair_vals: gridDim.x * kParamBlock * tile doubles.
-// The per-panel network's shared memory, after the curve tile.
+// curve) packed as leaves | shallowest leaf depth << 16 | deepest leaf depth << 24.  nodes_total (nullable, zeroed):
+// panels evaluated per query.
+// The per-panel network's shared memory.
 struct PanelSmem
 {
     WeightsSmem w;
@@ -550,284 +540,240 @@ struct PanelSmem
 };
 
 // PANEL: the per-panel network runs (its code and shared memory are compiled only into this instance, so the other
-// instance keeps its registers).  n_groups > 1: the curve tiles
-// of a query block are split into n_groups consecutive groups, one work item each, and each item writes its raw
-// partial sum to partial[g * n + i] (a later kernel adds the groups in order) and adds its panel counts to
-// nodes_total[i] (zeroed first).
+// instance keeps its registers).
 template <bool PANEL>
 constexpr int param_min_blocks()
 {
     return !PANEL ? 6 : 1; // the double-float panels in 80 registers (no spills), six blocks per SM
 }
 template <bool PANEL>
-__global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>()) k_param_gk15(const df* __restrict__ pos, int64_t n,
-                                                            double* __restrict__ out, FrameDF F,
-                                                            const CurveDF* __restrict__ curves,
-                                                            int64_t n_curves, int tile, int min_depth, int max_depth,
-                                                            double tol, const uint8_t* __restrict__ start_depth,
-                                                            uint32_t* __restrict__ stats,
-                                                            int32_t* __restrict__ nodes_total,
-                                                            double* __restrict__ pair_vals, int* flags,
-                                                            ParamExtras ex, int n_groups, double* __restrict__ partial)
+__global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>())
+    k_param_gk15(const df* __restrict__ pos, int64_t q0, int nq, FrameDF F, const CurveDF* __restrict__ curves,
+                 int64_t n_curves, int64_t c0, int nc, int min_depth, int max_depth, double tol,
+                 const uint8_t* __restrict__ start_depth, uint32_t* __restrict__ stats,
+                 int32_t* __restrict__ nodes_total, double* __restrict__ vals, int* __restrict__ next, int take,
+                 ParamExtras ex)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ __align__(8) uint64_t bar;
-    __shared__ int s_next;
-    __shared__ int s_nodes[kParamBlock];
-    CurveDF* const buf = reinterpret_cast<CurveDF*>(smem);
-    PanelSmem* const ps = reinterpret_cast<PanelSmem*>(smem + size_t(tile) * sizeof(CurveDF));
+    __shared__ double tol_at[kParamMaxDepth + 1];
+    PanelSmem* const ps = reinterpret_cast<PanelSmem*>(smem);
     bool const use_panel = PANEL && ex.pwb != nullptr;
     unsigned long long skips = 0;
-    double* const slab = pair_vals + size_t(blockIdx.x) * kParamBlock * tile;
-    int64_t const n_blocks_q = (n + kParamBlock - 1) / kParamBlock;
-    int const n_tiles = int((n_curves + tile - 1) / tile);
-    int const tiles_per_group = (n_tiles + n_groups - 1) / n_groups;
-    int64_t const n_items = n_blocks_q * n_groups;
     unsigned const lane = threadIdx.x & 31u;
-    // tol * 2^-depth by repeated halving, as the recursion computes it (exact unless it reaches subnormals)
-    double tol_at[kParamMaxDepth + 1];
-    tol_at[0] = tol;
-    for (int l = 1; l <= kParamMaxDepth; ++l)
-        tol_at[l] = __dmul_rn(tol_at[l - 1], 0.5);
+    if (threadIdx.x == 0)
+    {
+        // tol * 2^-depth by repeated halving, as the recursion computes it (exact unless it reaches subnormals)
+        tol_at[0] = tol;
+        for (int l = 1; l <= kParamMaxDepth; ++l)
+            tol_at[l] = __dmul_rn(tol_at[l - 1], 0.5);
+    }
     if (use_panel)
         load_weights(ps->w, ex.pwb, ex.pparams);
     float3 const x0f = make_float3(0.f, 0.f, F.len.hi);
     int const warp = int(threadIdx.x >> 5);
-    if (threadIdx.x == 0)
-    {
-        mbar_init(&bar, 1);
-        fence_barrier_init();
-    }
     __syncthreads();
-    unsigned phase = 0;
-    for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x)
+    int const total = nc * nq; // curve-major
+    int taken = 0, end = 0;    // this warp's pairs not yet given to a lane: [taken, end)
+    int pi = -1;                // this lane's pair, -1 = needs one
+    bool drained = false;
+    int k = 0, ql = 0, s = 0, d = 0, leaves = 0, dmin = 0, dmax = 0, pnodes = 0;
+    uint32_t j = 0;
+    df cp[12]; // this pair's curve minus its query, as power coefficients about t = 1/2
+    double pending[kParamMaxDepth + 1];
+    for (;;)
     {
-        int64_t const qb = item / n_groups;
-        int const grp = int(item - qb * n_groups);
-        int const t_begin = grp * tiles_per_group;
-        int const t_end = min(n_tiles, t_begin + tiles_per_group);
-        int64_t const q0 = qb * kParamBlock;
-        int const nq = int(n - q0 < kParamBlock ? n - q0 : int64_t(kParamBlock));
-        rd sum = rd(0.0);
-        s_nodes[threadIdx.x] = 0;
-        for (int t = t_begin; t < t_end; ++t)
+        unsigned const want = __ballot_sync(0xffffffffu, pi < 0 && !drained);
+        if (want)
         {
-            int64_t const c0 = int64_t(t) * tile;
-            int const cnt = int(n_curves - c0 < tile ? n_curves - c0 : int64_t(tile));
-            __syncthreads(); // the tile buffer and the slab are free
-            if (threadIdx.x == 0)
+            int const need = __popc(want), left = end - taken, rank = __popc(want & ((1u << lane) - 1u));
+            int fresh = 0;
+            if (left < need)
             {
-                s_next = 0;
-                unsigned const bytes = unsigned(cnt) * unsigned(sizeof(CurveDF));
-                mbar_arrive_expect_tx(&bar, bytes);
-                bulk_copy_g2s(buf, curves + c0, bytes, &bar);
+                if (lane == 0)
+                    fresh = atomicAdd(next, take);
+                fresh = __shfl_sync(0xffffffffu, fresh, 0);
             }
-            if (!mbar_wait_bounded(&bar, phase, flags, 4))
-                return; // every thread of the block times out on the same barrier
-            phase ^= 1u;
-
-            int const total = cnt * nq; // pairs in this tile's pool, curve-major
-            int pi = -1;                // this lane's pair, -1 = needs one
-            bool drained = false;
-            int k = 0, ql = 0, s = 0, d = 0, leaves = 0, dmin = 0, dmax = 0, pnodes = 0;
-            uint32_t j = 0;
-            df cp[12]; // this pair's curve minus its query, as power coefficients about t = 1/2
-            double pending[kParamMaxDepth + 1];
-            for (;;)
+            if (want & (1u << lane))
             {
-                unsigned const want = __ballot_sync(0xffffffffu, pi < 0 && !drained);
-                if (want)
+                int const mine = rank < left ? taken + rank : fresh + rank - left;
+                if (mine < total)
                 {
-                    int base = 0;
-                    unsigned const leader = __ffs(want) - 1;
-                    if (lane == leader)
-                        base = atomicAdd(&s_next, __popc(want));
-                    base = __shfl_sync(0xffffffffu, base, leader);
-                    if (want & (1u << lane))
-                    {
-                        int const mine = base + __popc(want & ((1u << lane) - 1u));
-                        if (mine < total)
-                        {
-                            pi = mine;
-                            k = mine / nq;
-                            ql = mine - k * nq;
-                            int64_t const q = q0 + ql;
-                            df const pd[3] = {pos[3 * q], pos[3 * q + 1], pos[3 * q + 2]};
-                            CurveDF const& cv = buf[k];
+                    pi = mine;
+                    k = mine / nq;
+                    ql = mine - k * nq;
+                    int64_t const q = q0 + ql;
+                    df const pd[3] = {pos[3 * q], pos[3 * q + 1], pos[3 * q + 2]};
+                    CurveDF const& cv = curves[c0 + k];
 #pragma unroll
-                            for (int e = 0; e < 12; ++e)
-                                cp[e] = e < 3 ? cv.c[e] - pd[e] : cv.c[e];
-                            s = start_depth ? min(int(start_depth[q * n_curves + c0 + k]), max_depth) : 0;
-                            d = s;
-                            j = 0;
-                            leaves = 0;
-                            dmin = 255;
-                            dmax = 0;
-                            pnodes = 0;
-                        }
-                        else
-                            drained = true;
-                    }
+                    for (int e = 0; e < 12; ++e)
+                        cp[e] = e < 3 ? cv.c[e] - pd[e] : cv.c[e];
+                    s = start_depth ? min(int(start_depth[q * n_curves + c0 + k]), max_depth) : 0;
+                    d = s;
+                    j = 0;
+                    leaves = 0;
+                    dmin = 255;
+                    dmax = 0;
+                    pnodes = 0;
                 }
-                if (!__any_sync(0xffffffffu, pi >= 0))
-                    break;
-                // the per-panel network: up to four rounds of "split it without evaluating", all lanes together
-                for (int round = 0; PANEL && use_panel && round < 4; ++round)
-                {
-                    bool const cand = pi >= 0 && d < max_depth;
-                    float f[kF];
-                    if (cand)
-                    {
-                        // the control points minus the query, as the network was trained on them: a0 -+ a1/2 + a2/4
-                        // -+ a3/8 at the ends, a0 -+ a1/6 - a2/12 +- a3/8 between
-                        float cpf[12];
-#pragma unroll
-                        for (int e = 0; e < 3; ++e)
-                        {
-                            df const o1 = df_mulf(cp[3 + e], 1.f / 6.f), e2 = df_mulf(cp[6 + e], 1.f / 12.f);
-                            df const end = cp[e] + df_scale(cp[6 + e], 0.25f), mid = cp[e] - e2;
-                            df const a3 = df_scale(cp[9 + e], 0.125f), odd = df_scale(cp[3 + e], 0.5f) + a3;
-                            cpf[e] = (end - odd).hi;
-                            cpf[3 + e] = (mid - o1 + a3).hi;
-                            cpf[6 + e] = (mid + o1 - a3).hi;
-                            cpf[9 + e] = (end + odd).hi;
-                        }
-                        panel_features(cpf, d, j, x0f, ex.log10_tol, f);
-                    }
-                    else
-                    {
-#pragma unroll
-                        for (int e = 0; e < kF; ++e)
-                            f[e] = 0.f;
-                    }
-                    uint32_t* const row = ps->feat[warp][lane];
-#pragma unroll
-                    for (int e = 0; e < kF / 2; ++e)
-                        row[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
-                    row[6] = 0u;
-                    row[7] = 0u;
-                    __syncwarp();
-                    int const g = int(lane >> 2), tig = int(lane & 3u);
-#pragma unroll
-                    for (int mt = 0; mt < 2; ++mt)
-                    {
-                        uint32_t a0[4] = {ps->feat[warp][mt * 16 + g][tig], ps->feat[warp][mt * 16 + g + 8][tig],
-                                          ps->feat[warp][mt * 16 + g][4 + tig],
-                                          ps->feat[warp][mt * 16 + g + 8][4 + tig]};
-                        float z1[8][4], z2[8][4], z3[2][4];
-                        mlp_forward(ps->w, a0, z1, z2, z3);
-                        if (tig == 0) // columns 0 and 1: the split and accept logits
-                        {
-                            ps->logit[warp][mt * 16 + g][0] = z3[0][0];
-                            ps->logit[warp][mt * 16 + g][1] = z3[0][1];
-                            ps->logit[warp][mt * 16 + g + 8][0] = z3[0][2];
-                            ps->logit[warp][mt * 16 + g + 8][1] = z3[0][3];
-                        }
-                    }
-                    __syncwarp();
-                    bool const skip =
-                        cand && (ps->logit[warp][lane][1] - ps->logit[warp][lane][0]) < ex.skip_logit;
-                    __syncwarp();
-                    if (!__any_sync(0xffffffffu, skip))
-                        break;
-                    if (skip)
-                    {
-                        ++d; // split without evaluating: left child next
-                        j <<= 1;
-                        ++skips;
-                    }
-                }
-                if (pi < 0)
-                    continue;
-                float e32;
-                double v = gk15_panel_df(cp, F, d, j, &e32);
-                double const err = double(e32);
-                ++pnodes;
-                bool const accept = d >= max_depth || (d >= min_depth && err <= tol_at[d]);
-                if (ex.panel_log && d < max_depth)
-                {
-                    unsigned long long const slot = atomicAdd(ex.log_count, 1ull);
-                    if ((long long)slot < ex.log_cap)
-                    {
-                        ex.panel_log[2 * slot] = uint32_t((q0 + ql) * n_curves + c0 + k);
-                        ex.panel_log[2 * slot + 1] = (uint32_t(d) << 25) | (j << 1) | (accept ? 1u : 0u);
-                    }
-                }
-                if (!accept)
-                {
-                    ++d; // split: left child next
-                    j <<= 1;
-                    continue;
-                }
-                ++leaves;
-                dmin = min(dmin, d);
-                dmax = max(dmax, d);
-                while (d > 0 && (j & 1u))
-                {
-                    v = __dadd_rn(pending[d], v); // left + right
-                    --d;
-                    j >>= 1;
-                }
-                if (d > 0)
-                {
-                    pending[d] = v; // a finished left child: its right sibling is next
-                    ++j;
-                    while (d < s)
-                    {
-                        ++d;
-                        j <<= 1;
-                    }
-                    continue;
-                }
-                // the root is done: v is this pair's integral
-                slab[size_t(k) * kParamBlock + ql] = v;
-                if (stats)
-                    stats[(q0 + ql) * n_curves + c0 + k] = uint32_t(min(leaves, 0xffff)) | (uint32_t(dmin) << 16) |
-                                                           (uint32_t(dmax) << 24);
-                atomicAdd(&s_nodes[ql], pnodes);
-                pi = -1;
+                else
+                    drained = true;
             }
-            __syncthreads(); // the slab is complete
-            if (int(threadIdx.x) < nq)
-                for (int kk = 0; kk < cnt; ++kk)
-                    sum = sum + rd(slab[size_t(kk) * kParamBlock + threadIdx.x]);
+            taken = left < need ? fresh + need - left : taken + need;
+            end = left < need ? fresh + take : end;
         }
-        __syncthreads(); // s_nodes is complete
-        if (int(threadIdx.x) < nq)
+        if (!__any_sync(0xffffffffu, pi >= 0))
+            break;
+        // the per-panel network: up to four rounds of "split it without evaluating", all lanes together
+        for (int round = 0; PANEL && use_panel && round < 4; ++round)
         {
-            int64_t const i = q0 + threadIdx.x;
-            if (n_groups == 1)
+            bool const cand = pi >= 0 && d < max_depth;
+            float f[kF];
+            if (cand)
             {
-                out[i] = (sum / (rd(4.0) * rd(3.141592653589793238462643383279502884))).v;
-                if (nodes_total)
-                    nodes_total[i] = s_nodes[threadIdx.x];
+                // the control points minus the query, as the network was trained on them: a0 -+ a1/2 + a2/4
+                // -+ a3/8 at the ends, a0 -+ a1/6 - a2/12 +- a3/8 between
+                float cpf[12];
+#pragma unroll
+                for (int e = 0; e < 3; ++e)
+                {
+                    df const o1 = df_mulf(cp[3 + e], 1.f / 6.f), e2 = df_mulf(cp[6 + e], 1.f / 12.f);
+                    df const end = cp[e] + df_scale(cp[6 + e], 0.25f), mid = cp[e] - e2;
+                    df const a3 = df_scale(cp[9 + e], 0.125f), odd = df_scale(cp[3 + e], 0.5f) + a3;
+                    cpf[e] = (end - odd).hi;
+                    cpf[3 + e] = (mid - o1 + a3).hi;
+                    cpf[6 + e] = (mid + o1 - a3).hi;
+                    cpf[9 + e] = (end + odd).hi;
+                }
+                panel_features(cpf, d, j, x0f, ex.log10_tol, f);
             }
             else
             {
-                partial[int64_t(grp) * n + i] = sum.v;
-                if (nodes_total)
-                    atomicAdd(&nodes_total[i], s_nodes[threadIdx.x]);
+#pragma unroll
+                for (int e = 0; e < kF; ++e)
+                    f[e] = 0.f;
+            }
+            uint32_t* const row = ps->feat[warp][lane];
+#pragma unroll
+            for (int e = 0; e < kF / 2; ++e)
+                row[e] = pack_bf16(f[2 * e], f[2 * e + 1]);
+            row[6] = 0u;
+            row[7] = 0u;
+            __syncwarp();
+            int const g = int(lane >> 2), tig = int(lane & 3u);
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+            {
+                uint32_t a0[4] = {ps->feat[warp][mt * 16 + g][tig], ps->feat[warp][mt * 16 + g + 8][tig],
+                                  ps->feat[warp][mt * 16 + g][4 + tig],
+                                  ps->feat[warp][mt * 16 + g + 8][4 + tig]};
+                float z1[8][4], z2[8][4], z3[2][4];
+                mlp_forward(ps->w, a0, z1, z2, z3);
+                if (tig == 0) // columns 0 and 1: the split and accept logits
+                {
+                    ps->logit[warp][mt * 16 + g][0] = z3[0][0];
+                    ps->logit[warp][mt * 16 + g][1] = z3[0][1];
+                    ps->logit[warp][mt * 16 + g + 8][0] = z3[0][2];
+                    ps->logit[warp][mt * 16 + g + 8][1] = z3[0][3];
+                }
+            }
+            __syncwarp();
+            bool const skip =
+                cand && (ps->logit[warp][lane][1] - ps->logit[warp][lane][0]) < ex.skip_logit;
+            __syncwarp();
+            if (!__any_sync(0xffffffffu, skip))
+                break;
+            if (skip)
+            {
+                ++d; // split without evaluating: left child next
+                j <<= 1;
+                ++skips;
             }
         }
+        if (pi < 0)
+            continue;
+        float e32;
+        double v = gk15_panel_df(cp, F, d, j, &e32);
+        double const err = double(e32);
+        ++pnodes;
+        bool const accept = d >= max_depth || (d >= min_depth && err <= tol_at[d]);
+        if (ex.panel_log && d < max_depth)
+        {
+            unsigned long long const slot = atomicAdd(ex.log_count, 1ull);
+            if ((long long)slot < ex.log_cap)
+            {
+                ex.panel_log[2 * slot] = uint32_t((q0 + ql) * n_curves + c0 + k);
+                ex.panel_log[2 * slot + 1] = (uint32_t(d) << 25) | (j << 1) | (accept ? 1u : 0u);
+            }
+        }
+        if (!accept)
+        {
+            ++d; // split: left child next
+            j <<= 1;
+            continue;
+        }
+        ++leaves;
+        dmin = min(dmin, d);
+        dmax = max(dmax, d);
+        while (d > 0 && (j & 1u))
+        {
+            v = __dadd_rn(pending[d], v); // left + right
+            --d;
+            j >>= 1;
+        }
+        if (d > 0)
+        {
+            pending[d] = v; // a finished left child: its right sibling is next
+            ++j;
+            while (d < s)
+            {
+                ++d;
+                j <<= 1;
+            }
+            continue;
+        }
+        // the root is done: v is this pair's integral
+        vals[int64_t(k) * nq + ql] = v;
+        if (stats)
+            stats[(q0 + ql) * n_curves + c0 + k] = uint32_t(min(leaves, 0xffff)) | (uint32_t(dmin) << 16) |
+                                                   (uint32_t(dmax) << 24);
+        if (nodes_total)
+            atomicAdd(nodes_total + q0 + ql, pnodes);
+        pi = -1;
     }
     if (ex.skip_count && skips)
         atomicAdd(ex.skip_count, skips);
 }
 
-// The groups' partial sums of each query added in group order (so in curve order by tiles), then normalised.
-__global__ void k_param_groups(const double* __restrict__ partial, int n_groups, int64_t n, double* __restrict__ out)
+// The pair integrals and their sums over chunks of at most `most` pairs: queries first, and curves where one query has
+// more.  launch(q0, nq, c0, nc, vals, next) integrates a chunk's pairs.
+template <class Launch>
+int param_chunks(Context& ctx, int64_t n, int64_t n_curves, int64_t most, double* d_out, int32_t* d_nodes, Launch launch)
 {
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-    {
-        rd sum = rd(0.0);
-        for (int g = 0; g < n_groups; ++g)
-            sum = sum + rd(partial[int64_t(g) * n + i]);
-        out[i] = (sum / (rd(4.0) * rd(3.141592653589793238462643383279502884))).v;
-    }
+    int64_t const nc_max = std::min(n_curves, most);
+    int64_t const nq_max = std::min(n, std::max<int64_t>(1, most / nc_max));
+    double* vals = nullptr;
+    int* next = nullptr;
+    AGWN_TRY(ctx.scratch_reserve(S_SEGS_RAW, sizeof(double) * size_t(nc_max) * size_t(nq_max),
+                                 reinterpret_cast<void**>(&vals)));
+    AGWN_TRY(ctx.scratch_reserve(S_PARTIAL, sizeof(int), reinterpret_cast<void**>(&next)));
+    if (d_nodes)
+        AGWN_TRY_CUDA(cudaMemsetAsync(d_nodes, 0, sizeof(int32_t) * n, ctx.stream));
+    for (int64_t q0 = 0; q0 < n; q0 += nq_max)
+        for (int64_t c0 = 0; c0 < n_curves; c0 += nc_max)
+        {
+            int const nq = int(std::min(nq_max, n - q0)), nc = int(std::min(nc_max, n_curves - c0));
+            AGWN_TRY_CUDA(cudaMemsetAsync(next, 0, sizeof(int), ctx.stream));
+            AGWN_TRY(ctx.launch_begin(AGWN_K_PARAMETRIC));
+            launch(q0, nq, c0, nc, vals, next);
+            AGWN_TRY(ctx.launch_end(AGWN_K_PARAMETRIC));
+            AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
+            k_param_sum<<<div_up(nq, 64), 64, 0, ctx.stream>>>(vals, nq, nc, c0 == 0, c0 + nc == n_curves, d_out + q0);
+            AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
+        }
+    return AGWN_OK;
 }
 
-// The exact form over chunks of at most 2^25 pairs (268 MB of pair integrals): queries first, and curves where one
-// query has more.
+// The exact form, 2^25 pairs (268 MB of integrals) at a time.
 int param_run_exact(Context& ctx, const double* d_pos, int64_t n, double* d_out, const double* x0, const double* d_curves,
                     int64_t n_curves, int min_depth, int max_depth, double tol, const uint8_t* d_start,
                     uint32_t* d_stats, int32_t* d_nodes, ParamExtras const& ex)
@@ -839,37 +785,19 @@ int param_run_exact(Context& ctx, const double* d_pos, int64_t n, double* d_out,
         k_bernstein<<<div_up(kBernPanels * kTeam, 256), 256, 0, ctx.stream>>>(static_cast<double2*>(ctx.bernstein.ptr));
         AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
     }
-    constexpr int64_t most = int64_t(1) << 25;
-    int64_t const nc_max = std::min(n_curves, most);
-    int64_t const nq_max = std::min(n, std::max<int64_t>(1, most / nc_max));
-    double* vals = nullptr;
-    int* next = nullptr;
-    AGWN_TRY(ctx.scratch_reserve(S_SEGS_RAW, sizeof(double) * size_t(nc_max) * size_t(nq_max),
-                                 reinterpret_cast<void**>(&vals)));
-    AGWN_TRY(ctx.scratch_reserve(S_PARTIAL, sizeof(int), reinterpret_cast<void**>(&next)));
-    if (d_nodes)
-        AGWN_TRY_CUDA(cudaMemsetAsync(d_nodes, 0, sizeof(int32_t) * n, ctx.stream));
     int per_sm = 0;
     AGWN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_param_exact, kParamBlock, 0));
+    int64_t const full = int64_t(std::max(per_sm, 1)) * ctx.sm_count;
     ev3<rd> const x0v{rd(x0[0]), rd(x0[1]), rd(x0[2])};
-    for (int64_t q0 = 0; q0 < n; q0 += nq_max)
-        for (int64_t c0 = 0; c0 < n_curves; c0 += nc_max)
-        {
-            int const nq = int(std::min(nq_max, n - q0)), nc = int(std::min(nc_max, n_curves - c0));
-            int const grid = int(std::min<int64_t>(div_up(int64_t(nq) * nc, kParamBlock / kTeam),
-                                                   int64_t(std::max(per_sm, 1)) * ctx.sm_count));
-            AGWN_TRY_CUDA(cudaMemsetAsync(next, 0, sizeof(int), ctx.stream));
-            AGWN_TRY(ctx.launch_begin(AGWN_K_PARAMETRIC));
-            k_param_exact<<<grid, kParamBlock, 0, ctx.stream>>>(d_pos, q0, nq, x0v, d_curves, n_curves, c0, nc,
-                                                                min_depth, max_depth, tol, d_start, d_stats, d_nodes,
-                                                                vals, next,
-                                                                static_cast<const double2*>(ctx.bernstein.ptr), ex);
-            AGWN_TRY(ctx.launch_end(AGWN_K_PARAMETRIC));
-            AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-            k_param_sum<<<div_up(nq, 64), 64, 0, ctx.stream>>>(vals, nq, nc, c0 == 0, c0 + nc == n_curves, d_out + q0);
-            AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
-        }
-    return AGWN_OK;
+    return param_chunks(ctx, n, n_curves, int64_t(1) << 25, d_out, d_nodes,
+                        [&](int64_t q0, int nq, int64_t c0, int nc, double* vals, int* next)
+                        {
+                            int const grid =
+                                int(std::min<int64_t>(div_up(int64_t(nq) * nc, kParamBlock / kTeam), full));
+                            k_param_exact<<<grid, kParamBlock, 0, ctx.stream>>>(
+                                d_pos, q0, nq, x0v, d_curves, n_curves, c0, nc, min_depth, max_depth, tol, d_start,
+                                d_stats, d_nodes, vals, next, static_cast<const double2*>(ctx.bernstein.ptr), ex);
+                        });
 }
 } // namespace
 
@@ -906,51 +834,13 @@ int param_run(Context& ctx, const double* d_pos, int64_t n, double* d_out, const
         return param_run_exact(ctx, d_pos, n, d_out, x0, d_curves, n_curves, min_depth, max_depth, tol, d_start,
                                d_stats, d_nodes, ex);
     auto const kern = panel ? k_param_gk15<true> : k_param_gk15<false>;
-    int tile = int(std::min<int64_t>(kParamTileDF, n_curves));
-    size_t smem = 0;
+    size_t const smem = panel ? sizeof(PanelSmem) : 0;
+    AGWN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     int per_sm = 0;
-    auto shape = [&](int t) -> int
-    {
-        smem = size_t(t) * sizeof(CurveDF) + (panel ? sizeof(PanelSmem) : 0);
-        AGWN_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        AGWN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kParamBlock, smem));
-        if (per_sm < 1)
-            return fail(AGWN_ERR_UNSUPPORTED, "parametric kernel does not fit on an SM");
-        return AGWN_OK;
-    };
-    AGWN_TRY(shape(tile));
-    int64_t const n_blocks_q = (n + kParamBlock - 1) / kParamBlock;
-    int n_groups = 1;
-    // two waves of work items; tiles of at least 128 curves (measured: more waves or other tiles change <1%)
-    int64_t const waves = 2, min_tile = 128;
-    if (n_blocks_q < waves * int64_t(per_sm) * ctx.sm_count)
-    {
-        // Few query blocks (a sample of queries, or many curves per query): the curves of each block are split
-        // into groups of tiles, one work item each, so that every SM gets work.  Smaller tiles cost the
-        // double-float kernel nothing (measured flat from 768 down to 128 curves) and let more blocks reside.
-        int64_t const want = div_up(waves * int64_t(per_sm) * ctx.sm_count, n_blocks_q);
-        int64_t const t = div_up(div_up(n_curves, want), 32) * 32;
-        tile = int(std::max<int64_t>(std::min<int64_t>(t, tile), std::min<int64_t>(min_tile, n_curves)));
-        AGWN_TRY(shape(tile));
-        int const n_tiles = int(div_up(n_curves, tile));
-        int64_t const groups =
-            std::min<int64_t>(n_tiles, div_up(waves * int64_t(per_sm) * ctx.sm_count, n_blocks_q));
-        int const tpg = int(div_up(n_tiles, groups));
-        n_groups = int(div_up(n_tiles, tpg));
-    }
-    int64_t const n_items = n_blocks_q * n_groups;
-    int const grid = int(std::max<int64_t>(1, std::min<int64_t>(n_items, int64_t(per_sm) * ctx.sm_count)));
-    double* pair_vals = nullptr;
-    AGWN_TRY(ctx.scratch_reserve(S_SEGS_RAW, sizeof(double) * size_t(grid) * kParamBlock * tile,
-                                 reinterpret_cast<void**>(&pair_vals)));
-    double* partial = nullptr;
-    if (n_groups > 1)
-    {
-        AGWN_TRY(ctx.scratch_reserve(S_PARTIAL, sizeof(double) * size_t(n_groups) * size_t(n),
-                                     reinterpret_cast<void**>(&partial)));
-        if (d_nodes)
-            AGWN_TRY_CUDA(cudaMemsetAsync(d_nodes, 0, sizeof(int32_t) * n, ctx.stream));
-    }
+    AGWN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kParamBlock, smem));
+    if (per_sm < 1)
+        return fail(AGWN_ERR_UNSUPPORTED, "parametric kernel does not fit on an SM");
+    int64_t const full = int64_t(per_sm) * ctx.sm_count;
     // curves and queries in the frame of x0, as double-floats
     FrameDF F;
     {
@@ -974,17 +864,17 @@ int param_run(Context& ctx, const double* d_pos, int64_t n, double* d_out, const
     AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
     k_queries_df<<<int(std::min<int64_t>(div_up(n, 256), 4 * ctx.sm_count)), 256, 0, ctx.stream>>>(d_pos, n, F, qdf);
     AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
-    AGWN_TRY(ctx.launch_begin(AGWN_K_PARAMETRIC));
-    kern<<<grid, kParamBlock, smem, ctx.stream>>>(qdf, n, d_out, F, cdf, n_curves, tile,
-                                                 min_depth, max_depth, tol, d_start, d_stats, d_nodes, pair_vals,
-                                                 ctx.d_flags, ex, n_groups, partial);
-    AGWN_TRY(ctx.launch_end(AGWN_K_PARAMETRIC));
-    if (n_groups == 1)
-        return AGWN_OK;
-    AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-    k_param_groups<<<int(std::min<int64_t>(div_up(n, 256), 8 * ctx.sm_count)), 256, 0, ctx.stream>>>(partial, n_groups,
-                                                                                                     n, d_out);
-    return ctx.launch_end(AGWN_K_OTHER);
+    // 2^26 pairs (537 MB of integrals) at a time: a chunk ends with its deepest pairs, half a millisecond or so
+    return param_chunks(ctx, n, n_curves, int64_t(1) << 26, d_out, d_nodes,
+                        [&](int64_t q0, int nq, int64_t c0, int nc, double* vals, int* next)
+                        {
+                            int64_t const pairs = int64_t(nq) * nc;
+                            int const grid = int(std::min<int64_t>(div_up(pairs, kParamBlock), full));
+                            int const take = pairs >= 8 * full * kParamBlock ? 64 : 32;
+                            kern<<<grid, kParamBlock, smem, ctx.stream>>>(qdf, q0, nq, F, cdf, n_curves, c0, nc,
+                                                                         min_depth, max_depth, tol, d_start, d_stats,
+                                                                         d_nodes, vals, next, take, ex);
+                        });
 }
 } // namespace agwn
 
@@ -1022,15 +912,6 @@ int param_entry(agwn_context* ctx, const agwn_mlp* mlp, int n_classes, float alp
         AGWN_TRY(stage_out(*ctx, pair_stats, sizeof(uint32_t) * size_t(n) * n_curves, S_MISC2, &dstats, &h_stats));
     if (nodes_per_query)
         AGWN_TRY(stage_out(*ctx, nodes_per_query, sizeof(int32_t) * n, S_COUNTS, &dnodes, &h_nodes));
-    // curves must be 16-byte aligned for the bulk copy; a host array was staged into aligned scratch
-    if (reinterpret_cast<uintptr_t>(dcur) % 16 != 0)
-    {
-        void* aligned = nullptr;
-        AGWN_TRY(ctx->scratch_reserve(S_SEGS, sizeof(double) * 12 * n_curves, &aligned));
-        AGWN_TRY_CUDA(cudaMemcpyAsync(aligned, dcur, sizeof(double) * 12 * n_curves, cudaMemcpyDeviceToDevice,
-                                      ctx->stream));
-        dcur = aligned;
-    }
     if (mlp && n_curves > 0)
     {
         void* proposed = nullptr;
@@ -1109,14 +990,6 @@ extern "C" int agwn_param_panel_log_bezier3_f64(agwn_context* ctx, const double*
     bool h_log = false;
     AGWN_TRY(stage_in(*ctx, positions, sizeof(double) * 3 * n, S_QUERIES, &dpos));
     AGWN_TRY(stage_in(*ctx, curves, sizeof(double) * 12 * n_curves, S_MISC0, &dcur));
-    if (reinterpret_cast<uintptr_t>(dcur) % 16 != 0)
-    {
-        void* aligned = nullptr;
-        AGWN_TRY(ctx->scratch_reserve(S_SEGS, sizeof(double) * 12 * n_curves, &aligned));
-        AGWN_TRY_CUDA(cudaMemcpyAsync(aligned, dcur, sizeof(double) * 12 * n_curves, cudaMemcpyDeviceToDevice,
-                                      ctx->stream));
-        dcur = aligned;
-    }
     AGWN_TRY(ctx->scratch_reserve(S_OUT, sizeof(double) * n, &dout));
     if (capacity > 0)
         AGWN_TRY(stage_out(*ctx, log, sizeof(uint32_t) * 2 * size_t(capacity), S_MISC2, &dlog, &h_log));
