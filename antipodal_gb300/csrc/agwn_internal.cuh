@@ -306,6 +306,19 @@ struct rd
     __device__ __forceinline__ friend rd operator/(rd a, rd b) { return rd(div_rn_int(a.v, b.v)); }
     __device__ __forceinline__ friend rd operator-(rd a) { return rd(-a.v); }
 };
+// The same values with the products on the integer pipe too (mul_rn_int), for kernels with warps enough to hide its
+// longer chain: sums and products then issue side by side.
+struct rdi
+{
+    double v;
+    rdi() = default;
+    __host__ __device__ __forceinline__ constexpr rdi(double x) : v(x) {}
+    __device__ __forceinline__ friend rdi operator+(rdi a, rdi b) { return rdi(__dadd_rn(a.v, b.v)); }
+    __device__ __forceinline__ friend rdi operator-(rdi a, rdi b) { return rdi(__dsub_rn(a.v, b.v)); }
+    __device__ __forceinline__ friend rdi operator*(rdi a, rdi b) { return rdi(mul_rn_int(a.v, b.v)); }
+    __device__ __forceinline__ friend rdi operator/(rdi a, rdi b) { return rdi(div_rn_int(a.v, b.v)); }
+    __device__ __forceinline__ friend rdi operator-(rdi a) { return rdi(-a.v); }
+};
 struct rf
 {
     float v;
@@ -330,15 +343,34 @@ struct exact_of<float>
     using type = rf;
 };
 
+template <class T>
+struct exact_int_of
+{
+    using type = rf;
+};
+template <>
+struct exact_int_of<double>
+{
+    using type = rdi;
+};
+
 __device__ __forceinline__ rd ex_sqrt(rd a)
 {
     return rd(sqrt_rn_int(a.v));
+}
+__device__ __forceinline__ rdi ex_sqrt(rdi a)
+{
+    return rdi(sqrt_rn_int(a.v));
 }
 __device__ __forceinline__ rf ex_sqrt(rf a)
 {
     return rf(__fsqrt_rn(a.v));
 }
 __device__ __forceinline__ double ex_atan2(rd y, rd x)
+{
+    return atan2_int(y.v, x.v);
+}
+__device__ __forceinline__ double ex_atan2(rdi y, rdi x)
 {
     return atan2_int(y.v, x.v);
 }

@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(256) k_frac_exact(const T* __restrict__ pos, i
                                                     const SegX<T>* __restrict__ seg, int64_t n_seg, int tile,
                                                     int* flags)
 {
-    using S = typename exact_of<T>::type;
+    using S = typename exact_int_of<T>::type;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t bars[2];
     __shared__ int abort_cta;
@@ -178,7 +178,8 @@ __global__ void __launch_bounds__(256) k_frac_exact(const T* __restrict__ pos, i
                 {
                     ev3<S> const v0 = a - p[k];
                     ev3<S> const v1 = c - p[k];
-                    area[k] = area[k] + w * S(vos_exact(x1, v0, v1));
+                    S const term = S(vos_exact(x1, v0, v1));
+                    area[k] = area[k] + (g.w == T(1) ? term : w * term); // the same for a weight of 1
                 }
             }
             if (!pipe.single)

@@ -47,7 +47,12 @@ __device__ __forceinline__ uint32_t bits_of_float(float f)
 {
     return __float_as_uint(f);
 }
-// out of line: the cases they serve are rare, and their registers stay out of the callers
+// out of line: the cases they serve are rare, and their registers and FP64 instructions stay out of the callers
+// (inlined, the multiplication would be issued for every operand and then selected)
+static __device__ __noinline__ double mul_general(double a, double b)
+{
+    return __dmul_rn(a, b);
+}
 static __device__ __noinline__ double div_general(double a, double b)
 {
     return __ddiv_rn(a, b);
@@ -84,6 +89,10 @@ inline float float_of_bits(uint32_t b)
 inline uint32_t bits_of_float(float f)
 {
     return copy_bits<uint32_t>(f);
+}
+inline double mul_general(double a, double b)
+{
+    return a * b;
 }
 inline double div_general(double a, double b)
 {
@@ -140,6 +149,34 @@ AGWN_FN double double_of_53(int64_t v)
     uint32_t const h = uint32_t(m >> 32), z = h ? leading_zeros(h) : 32 + leading_zeros(uint32_t(m));
     uint64_t const t = m << (z & 63u); // the leading one at bit 63
     return of_bits(m ? (t >> 11) + (uint64_t(1085u - z) << 52) + (uint64_t(v) & 0x8000000000000000ull) : 0ull);
+}
+
+// a b, rounded to nearest even: the significands' 128-bit product by 32-bit halves, for operands within 2^+-511 (so
+// the product is normal); the FP64 instruction for the others.  Some 40 integer instructions, which leave the FP64
+// pipe to the sums: the mesh functions' exact form (27 products and 38 other FP64 instructions per term) went from 3.53
+// to 2.25 ms on 261,632 queries x 102 segments, FP64 75% and integer pipe 62% busy.  For kernels with warps enough to
+// hide its longer chain, and few enough copies for the instruction cache.
+AGWN_FN double mul_rn_int(double a, double b)
+{
+    uint64_t const ab = bits_of(a), bb = bits_of(b);
+    uint32_t const ah = uint32_t(ab >> 32), bh = uint32_t(bb >> 32), al = uint32_t(ab), bl = uint32_t(bb);
+    if (2 * ah - (512u << 21) >= (1023u << 21) || 2 * bh - (512u << 21) >= (1023u << 21))
+        return mul_general(a, b);
+    // significands in [2^63, 2^64)
+    uint32_t const a1 = (ah << 11) | (al >> 21) | 0x80000000u, a0 = al << 11;
+    uint32_t const b1 = (bh << 11) | (bl >> 21) | 0x80000000u, b0 = bl << 11;
+    uint64_t const ll = uint64_t(a0) * b0;
+    uint64_t const m1 = uint64_t(a1) * b0 + (ll >> 32);
+    uint64_t const m2 = uint64_t(a0) * b1 + uint32_t(m1);
+    uint64_t h = uint64_t(a1) * b1 + (m1 >> 32) + (m2 >> 32);
+    uint32_t const sticky = (uint32_t(m2) | uint32_t(ll)) ? 1u : 0u;
+    uint32_t const top = uint32_t(h >> 63); // 0: the product is below 2^127, one bit less
+    h = top ? h : h + h;
+    uint64_t const M = h >> 11;
+    uint32_t const rest = (uint32_t(h) & 0x7ffu) | sticky; // half is 0x400
+    uint32_t const up = rest + (uint32_t(M) & 1u) > 0x400u ? 1u : 0u;
+    uint32_t const e = (ah & 0x7ff00000u) + (bh & 0x7ff00000u) - ((1024u - top) << 20);
+    return of_bits((uint64_t(e | ((ah ^ bh) & 0x80000000u)) << 32) + M + up);
 }
 
 // a / b, rounded to nearest even.

@@ -103,12 +103,27 @@ __device__ __forceinline__ double integrand(const double (&c)[12], Bernstein con
     Gp.z = (dr.z - G.z * s1) * inv_s;
     rd const a = edot(x0, G);
     rd const ap = edot(x0, Gp);
-    ev3<rd> const X = x0 - ev3<rd>{G.x * a, G.y * a, G.z * a};
-    ev3<rd> const Xp = ev3<rd>{G.x * -ap, G.y * -ap, G.z * -ap} - ev3<rd>{Gp.x * a, Gp.y * a, Gp.z * a};
-    rd const d_eta = edot(G, ecross(X, Xp)) / edot(X, X);
-    ev3<rd> const v = G - ev3<rd>{x0.x * a, x0.y * a, x0.z * a};
-    ev3<rd> const vp = Gp - ev3<rd>{x0.x * ap, x0.y * ap, x0.z * ap};
-    rd const w = -(edot(x0, ecross(v, vp)) / edot(v, v));
+    // The products from here on take the integer pipe, beside the sums.  The two quotients have one form,
+    // axis . (A x A') / |A|^2, and share their code (inlined twice, the products overflow the instruction cache).
+    auto const i3 = [](ev3<rd> const& u) { return ev3<rdi>{rdi(u.x.v), rdi(u.y.v), rdi(u.z.v)}; };
+    ev3<rdi> const g = i3(G), gp = i3(Gp), z = i3(x0);
+    rdi const ai = rdi(a.v), api = rdi(ap.v);
+    ev3<rdi> A = g - ev3<rdi>{z.x * ai, z.y * ai, z.z * ai};
+    ev3<rdi> Ap = gp - ev3<rdi>{z.x * api, z.y * api, z.z * api};
+    ev3<rdi> axis = z;
+    ev3<rdi> const X = z - ev3<rdi>{g.x * ai, g.y * ai, g.z * ai};
+    ev3<rdi> const Xp = ev3<rdi>{g.x * -api, g.y * -api, g.z * -api} - ev3<rdi>{gp.x * ai, gp.y * ai, gp.z * ai};
+    rd w = rd(0.0), d_eta = rd(0.0);
+#pragma unroll 1
+    for (int term = 0; term < 2; ++term)
+    {
+        rd const quotient = rd((edot(axis, ecross(A, Ap)) / edot(A, A)).v);
+        w = d_eta;
+        d_eta = term == 0 ? -quotient : quotient; // first -x0 . (v x v') / |v|^2 = w, then G . (X x X') / |X|^2
+        A = X;
+        Ap = Xp;
+        axis = g;
+    }
     return (w - d_eta).v;
 }
 

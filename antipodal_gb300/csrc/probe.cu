@@ -166,37 +166,40 @@ namespace agwn
 namespace
 {
 __global__ void k_math_f64(const double* __restrict__ a, const double* __restrict__ b, int64_t n,
-                           double* __restrict__ quotient, double* __restrict__ root, double* __restrict__ angle)
+                           double* __restrict__ quotient, double* __restrict__ root, double* __restrict__ angle,
+                           double* __restrict__ product)
 {
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     {
         quotient[i] = div_rn_int(a[i], b[i]);
         root[i] = sqrt_rn_int(a[i]);
         angle[i] = atan2_int(a[i], b[i]);
+        product[i] = mul_rn_int(a[i], b[i]);
     }
 }
 } // namespace
 } // namespace agwn
 
 extern "C" int agwn_probe_math_f64(agwn_context* ctx, const double* a, const double* b, int64_t n, double* quotient,
-                                   double* root, double* angle)
+                                   double* root, double* angle, double* product)
 {
-    AGWN_CHECK_ARG(ctx && n >= 0 && (n == 0 || (a && b && quotient && root && angle)), "bad arguments");
+    AGWN_CHECK_ARG(ctx && n >= 0 && (n == 0 || (a && b && quotient && root && angle && product)), "bad arguments");
     AGWN_TRY_CUDA(cudaSetDevice(ctx->device));
     if (n == 0)
         return AGWN_OK;
     const void *da = nullptr, *db = nullptr;
-    void *dq = nullptr, *dr = nullptr, *dt = nullptr;
-    bool h[3] = {};
+    void *dq = nullptr, *dr = nullptr, *dt = nullptr, *dp = nullptr;
+    bool h[4] = {};
     size_t const bytes = sizeof(double) * size_t(n);
     AGWN_TRY(stage_in(*ctx, a, bytes, S_MISC0, &da));
     AGWN_TRY(stage_in(*ctx, b, bytes, S_MISC1, &db));
     AGWN_TRY(stage_out(*ctx, quotient, bytes, S_MISC2, &dq, &h[0]));
     AGWN_TRY(stage_out(*ctx, root, bytes, S_MISC3, &dr, &h[1]));
     AGWN_TRY(stage_out(*ctx, angle, bytes, S_OUT, &dt, &h[2]));
+    AGWN_TRY(stage_out(*ctx, product, bytes, S_QUERIES, &dp, &h[3]));
     k_math_f64<<<int(std::min<int64_t>(div_up(n, 256), 4 * ctx->sm_count)), 256, 0, ctx->stream>>>(
         static_cast<const double*>(da), static_cast<const double*>(db), n, static_cast<double*>(dq),
-        static_cast<double*>(dr), static_cast<double*>(dt));
+        static_cast<double*>(dr), static_cast<double*>(dt), static_cast<double*>(dp));
     AGWN_TRY_CUDA(cudaGetLastError());
     if (h[0])
         AGWN_TRY_CUDA(cudaMemcpyAsync(quotient, dq, bytes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -204,6 +207,8 @@ extern "C" int agwn_probe_math_f64(agwn_context* ctx, const double* a, const dou
         AGWN_TRY_CUDA(cudaMemcpyAsync(root, dr, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     if (h[2])
         AGWN_TRY_CUDA(cudaMemcpyAsync(angle, dt, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    if (h[3])
+        AGWN_TRY_CUDA(cudaMemcpyAsync(product, dp, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     AGWN_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
     return AGWN_OK;
 }

@@ -442,9 +442,10 @@ int agwn_probe_fp64_peak(agwn_context* ctx, double* tflops);
 /* The mixed kernel's own float atan2 and CUDA's atan2f on the same n inputs (host or device arrays), for testing
  * the former's error.  No reference counterpart. */
 int agwn_probe_atan2(agwn_context* ctx, const float* y, const float* x, int64_t n, float* ours, float* cuda_ref);
-/* The exact forms' double-precision division, square root and atan2 (csrc/intfp.cuh): a / b, sqrt(a), atan2(a, b). */
+/* The exact forms' double-precision division, square root, atan2 and product (csrc/intfp.cuh): a / b, sqrt(a),
+ * atan2(a, b), a b. */
 int agwn_probe_math_f64(agwn_context* ctx, const double* a, const double* b, int64_t n, double* quotient, double* root,
-                        double* angle);
+                        double* angle, double* product);
 
 #ifdef __cplusplus
 }

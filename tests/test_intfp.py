@@ -1,5 +1,5 @@
-"""The exact forms' division, square root and atan2 on the integer pipe (csrc/intfp.cuh): bit for bit IEEE division and
-square root, and atan2 within 3 ulp, on the host build of the same source (CPU) and on the device."""
+"""The exact forms' division, square root, product and atan2 on the integer pipe (csrc/intfp.cuh): bit for bit IEEE
+division, square root and product, and atan2 within 3 ulp, on the host build of the same source (CPU) and on the device."""
 
 import os
 import re
@@ -41,6 +41,10 @@ def pairs(kind: str, n: int = 40_000):
             a.append(float(((m >> s) + k % 3 - 1)) * 2.0 ** s)
             b.append(float(y))
         return np.array([a, b])
+    if kind == "short":  # few significant bits: exact products, ties, and products next to ties
+        a = rng.integers(1, 1 << 27, n) * 2 + 1
+        b = rng.integers(1, 1 << 27, n) * 2 + 1
+        return np.stack([a * 2.0 ** rng.integers(-400, 400, n).astype(float), -b.astype(float)])
     angles = rng.uniform(-np.pi, np.pi, n)  # "angles": the circle, the multiples of 1/64 and 1/128 and tiny ratios
     y, x = np.sin(angles), np.cos(angles)
     k = rng.integers(0, 129, n) / 128.0
@@ -49,15 +53,16 @@ def pairs(kind: str, n: int = 40_000):
     return np.stack([y, x]) * 2.0 ** rng.integers(-300, 300, n).astype(float)
 
 
-KINDS = ["any bits", "specials", "near one", "halfway", "angles"]
+KINDS = ["any bits", "specials", "near one", "halfway", "short", "angles"]
 
 
-def check(a, b, quotient, root, angle):
+def check(a, b, quotient, root, angle, product):
     with np.errstate(all="ignore"):
         want_q, want_r = a / b, np.sqrt(a)
         same = lambda u, v: (u.view(np.uint64) == v.view(np.uint64)) | (np.isnan(u) & np.isnan(v))  # noqa: E731
         assert same(quotient, want_q).all(), (a[~same(quotient, want_q)][:3], b[~same(quotient, want_q)][:3])
         assert same(root, want_r).all(), a[~same(root, want_r)][:3]
+        assert same(product, a * b).all(), (a[~same(product, a * b)][:3], b[~same(product, a * b)][:3])
         want = np.arctan2(a.astype(np.longdouble), b.astype(np.longdouble))
         assert (np.isnan(angle) == np.isnan(want)).all()
         ok = ~np.isnan(angle)
@@ -83,8 +88,8 @@ def test_host_build(host_build, kind):
     a, b = pairs(kind)
     r = subprocess.run([host_build], input=np.ascontiguousarray(np.stack([a, b], 1)).tobytes(), stdout=subprocess.PIPE,
                        check=True)
-    out = np.frombuffer(r.stdout, np.float64).reshape(-1, 3)
-    check(a, b, *(np.ascontiguousarray(out[:, k]) for k in range(3)))
+    out = np.frombuffer(r.stdout, np.float64).reshape(-1, 4)
+    check(a, b, *(np.ascontiguousarray(out[:, k]) for k in range(4)))
 
 
 def test_table():
@@ -108,7 +113,7 @@ def test_table():
 def test_device(kind):
     import antipodal_gb300 as ag
     a, b = (np.ascontiguousarray(v) for v in pairs(kind))
-    out = [np.empty_like(a) for _ in range(3)]
+    out = [np.empty_like(a) for _ in range(4)]
     with ag.CudaDispatcher() as disp:
         assert ag.library().agwn_probe_math_f64(disp.handle, a.ctypes.data, b.ctypes.data, len(a),
                                                 *(o.ctypes.data for o in out)) == 0
