@@ -131,7 +131,7 @@ struct CellGrid
     float tol_max = 0; // queries whose own tolerance exceeds this take the hierarchy walk
     int64_t entries = 0;
     int per_leaf = 0;   // cells per leaf it was built with
-    int64_t served = 0; // queries prepared for on this hierarchy so far
+    int64_t calls = 0;  // calls prepared for on this hierarchy so far
     bool valid = false;
     void release()
     {

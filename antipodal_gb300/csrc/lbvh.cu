@@ -323,6 +323,15 @@ __global__ void k_depth(int n, const int* __restrict__ parent_node, const int* _
 
 // ---- traversal ----------------------------------------------------------------------------------------------
 // Moller-Trumbore sign with NaiveIntersector's arithmetic and early rejections, in unfused precision S.
+// 1 / x by the FP64 instructions: the exact tests are rare, and a few warps' worth of them wait for the shorter chain.
+__device__ __forceinline__ rd recip_rare(rd x)
+{
+    return rd(__ddiv_rn(1.0, x.v));
+}
+__device__ __forceinline__ rf recip_rare(rf x)
+{
+    return rf(1.f) / x;
+}
 template <class S>
 __device__ __forceinline__ int mt_sign(ev3<S> p, ev3<S> dir, ev3<S> a, ev3<S> b, ev3<S> c, bool* tie = nullptr)
 {
@@ -332,7 +341,7 @@ __device__ __forceinline__ int mt_sign(ev3<S> p, ev3<S> dir, ev3<S> a, ev3<S> b,
     S const det = edot(e1, h);
     if (det.v == 0)
         return 0;
-    S const inv = S(1) / det;
+    S const inv = recip_rare(det);
     ev3<S> const s = p - a;
     S const u = inv * edot(s, h);
     if (u.v < 0 || u.v > 1)
@@ -910,7 +919,7 @@ int ray_hierarchy(Context& ctx, const Bvh& bvh, const T* dir_host)
         return AGWN_OK;
     rc.generation = 0; // invalid until the build completes
     rc.cells.valid = false;
-    rc.cells.served = 0;
+    rc.cells.calls = 0;
     AGWN_TRY(build_hier<T>(ctx, static_cast<const T*>(bvh.tri), bvh.n_tri, dir, rc.h, nullptr));
     std::memcpy(rc.dir, dir, sizeof(dir));
     rc.scalar_bytes = bvh.scalar_bytes;
@@ -923,9 +932,9 @@ int ray_hierarchy(Context& ctx, const Bvh& bvh, const T* dir_host)
 // The cell grid of the cached hierarchy (its leaves' float (u, v) corners), about per_leaf cells per leaf over the
 // widened boxes' extent (at most 2^22 cells).  Finer cells hold fewer leaves, so a query reads fewer list entries:
 // on a 76,496-triangle icosphere with 256^3 grid queries 2 cells per leaf read 5.06 entries per query (1.09 ms),
-// 16 read 3.49 (0.83 ms); 32 and 64 gained no more.  But a fine grid takes longer to build (two passes of 40 us against 16
-// there), so a mesh starts with 2 and takes 16 when its queries so far could repay it (integer_prepare).  Leaf boxes are widened by 4 * 2^-18 of the scene scale; a
-// query takes the grid while its own tolerance (qmax + scene) * 2^-18 stays below 3.5 * 2^-18 of the scene scale
+// 16 read 3.49 (0.83 ms); 32 and 64 gained no more.  But a fine grid takes longer to build (two passes of
+// 40 us against 16 there), so a mesh that is new on every call gets the coarse one (integer_prepare).  Leaf boxes are widened by
+// 4 * 2^-18 of the scene scale; a query takes the grid while its own tolerance (qmax + scene) * 2^-18 stays below 3.5 * 2^-18 of the scene scale
 // (qmax <= 2.5 * scene), which leaves room for the one-ulp difference between the corners and the walk's
 // outward-rounded boxes.
 int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g, int per_leaf)
@@ -1008,10 +1017,10 @@ int integer_prepare(Context& ctx, const Bvh& bvh, const T* dir_host, int64_t n)
     CellGrid& cg = ctx.ray_cache.cells;
     if (!ctx.integer_cells || bvh.n_tri <= 1)
         return AGWN_OK;
-    // The fine grid costs about 1 ns per leaf more to build and saves 0.016 ns per query, so it comes once 32 queries
-    // per leaf have been asked for (in one call or over many); until then the coarse one.
-    cg.served += n;
-    int const per_leaf = cg.served / 32 >= bvh.n_tri ? kCellsFine : kCellsCoarse;
+    // The fine grid costs about 1 ns per leaf more to build, and saves 0.016 ns per query and 1.5 us of a small call's
+    // latency: a mesh's first call takes it with 32 queries per leaf or more, and any later call on the mesh takes it.
+    ++cg.calls;
+    int const per_leaf = cg.calls > 1 || n / 32 >= bvh.n_tri ? kCellsFine : kCellsCoarse;
     if (!cg.valid || cg.per_leaf < per_leaf)
         AGWN_TRY(build_cells(ctx, ctx.ray_cache.h, float(bvh.scene_scale), cg, per_leaf));
     return AGWN_OK;
