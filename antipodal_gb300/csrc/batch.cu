@@ -27,7 +27,8 @@ struct agwn_batch
     int64_t total_queries = 0;
     double total_pairs = 0;
     agwn::DevBuf meshes, items, sample, head;
-    int n_items = 0, n_sample = 0;
+    // the work list cut for each number of queries a block takes at once, one list after the other in `items`
+    int n_items[3] = {0, 0, 0}, item0[3] = {0, 0, 0}, n_sample = 0;
     agwn::BConf conf{128, 1, 512, 64};
     bool tuned = false;
     cudaStream_t cap = nullptr;
@@ -71,6 +72,12 @@ size_t smem_of(const agwn_batch& b, const BConf& c, bool mixed)
 {
     // two tiles of segments, or of chain entries in the mixed form
     return 2 * size_t(c.seg_tile) * std::max(ops_of(b.policy).seg_bytes, mixed ? sizeof(RChain) : size_t(0));
+}
+
+// The list of work items for a configuration (128, 256 or 512 queries a block at once).
+int items_of(const BConf& c)
+{
+    return c.block * c.k / 256;
 }
 
 int grid_of(const agwn_batch& b, const Context& ctx, const BConf& c, int* grid)
@@ -179,38 +186,49 @@ extern "C" int agwn_batch_create(agwn_context* ctx, const agwn_robust* const* me
     }
     AGWN_CHECK_ARG(max_depth < 64, "hierarchy depth %d exceeds the traversal stack", max_depth);
 
-    // work items: every item carries about the same number of pairs; enough items for ~8 per CTA slot
+    // Work items: every item carries about the same number of pairs; enough items for ~16 per CTA slot, in whole
+    // blocks' worths of queries (block * queries per thread: a list for each of 128, 256 and 512).  A block's queries
+    // all run at once, so where the batch is small an item is one such unit.  With no item below 2^18 pairs and 512
+    // queries most SMs of a small batch had none, and blocks ran four units in turn (mixed, 16,864 queries on 4 meshes:
+    // 779 us, now 72; 536,007 on 6: 1069 us, now 415).  16 per slot against 8: 3.1e6 queries on 16, 1639 -> 1597 us.
     double total_cost = 0;
     for (auto const& m : hm)
         total_cost += double(m.n_q) * query_cost(m);
-    double const target = std::max(total_cost / (double(ctx->sm_count) * 4.0 * 8.0), double(1 << 18));
-    constexpr int64_t kQuantum = 512; // largest block * queries per thread
-    std::vector<BItem> items;
-    std::vector<double> cost;
+    double const target = total_cost / (double(ctx->sm_count) * 4.0 * 16.0);
+    constexpr int64_t kSample = 2048;
     std::vector<BItem> sample;
+    std::vector<BItem> sorted;
+    int item0[3], n_items[3];
     for (int i = 0; i < n_meshes; ++i)
+        if (hm[i].n_q > 0)
+            sample.push_back({i, 0, 0, std::min<int64_t>(hm[i].n_q, kSample)});
+    for (int u = 0; u < 3; ++u)
     {
-        BMesh const& m = hm[i];
-        if (m.n_q == 0)
-            continue;
-        double const c = query_cost(m);
-        int64_t nq = int64_t(std::ceil(target / c));
-        nq = std::max<int64_t>(kQuantum, (nq + kQuantum - 1) / kQuantum * kQuantum);
-        for (int64_t q0 = 0; q0 < m.n_q; q0 += nq)
+        int64_t const unit = int64_t(128) << u;
+        std::vector<BItem> items;
+        std::vector<double> cost;
+        for (int i = 0; i < n_meshes; ++i)
         {
-            items.push_back({i, 0, q0, std::min(m.n_q, q0 + nq)});
-            cost.push_back(double(items.back().q1 - q0) * c);
+            BMesh const& m = hm[i];
+            double const c = query_cost(m);
+            int64_t nq = int64_t(std::ceil(target / c));
+            nq = std::max<int64_t>(unit, (nq + unit - 1) / unit * unit);
+            for (int64_t q0 = 0; q0 < m.n_q; q0 += nq)
+            {
+                items.push_back({i, 0, q0, std::min(m.n_q, q0 + nq)});
+                cost.push_back(double(items.back().q1 - q0) * c);
+            }
         }
-        sample.push_back({i, 0, 0, std::min<int64_t>(m.n_q, 4 * kQuantum)});
+        AGWN_CHECK_ARG(items.size() < (size_t(1) << 28), "too many work items");
+        std::vector<size_t> order(items.size());
+        for (size_t j = 0; j < order.size(); ++j)
+            order[j] = j;
+        std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return cost[a] > cost[b]; });
+        item0[u] = int(sorted.size());
+        n_items[u] = int(items.size());
+        for (size_t const j : order)
+            sorted.push_back(items[j]);
     }
-    AGWN_CHECK_ARG(items.size() < (size_t(1) << 30), "too many work items");
-    std::vector<size_t> order(items.size());
-    for (size_t j = 0; j < order.size(); ++j)
-        order[j] = j;
-    std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return cost[a] > cost[b]; });
-    std::vector<BItem> sorted(items.size());
-    for (size_t j = 0; j < order.size(); ++j)
-        sorted[j] = items[order[j]];
 
     auto* b = new agwn_batch;
     b->device = ctx->device;
@@ -221,7 +239,11 @@ extern "C" int agwn_batch_create(agwn_context* ctx, const agwn_robust* const* me
     b->max_segments = max_segments;
     b->total_queries = total_q;
     b->total_pairs = total_cost;
-    b->n_items = int(sorted.size());
+    for (int u = 0; u < 3; ++u)
+    {
+        b->item0[u] = item0[u];
+        b->n_items[u] = n_items[u];
+    }
     b->n_sample = int(sample.size());
     int st = AGWN_OK;
     if ((st = b->meshes.reserve(sizeof(BMesh) * hm.size())) != AGWN_OK ||
@@ -253,7 +275,12 @@ extern "C" int agwn_batch_create(agwn_context* ctx, const agwn_robust* const* me
                 for (int stack : {32, 64})
                     if (stack == 64 || max_depth < 32)
                         b->candidates.push_back({block, k, tile, stack});
-    b->conf = {128, 1, 512, max_depth < 32 ? 32 : 64};
+    // Untuned: 128 threads, so that a small batch spreads over the SMs, and 256 where the int64_grid form has blocks to
+    // spare, since twice the queries then share a staged tile (mixed, 16,864 queries on 4 meshes: 73 us with 128 threads
+    // against 80; 175,645 on 8: 154 against 165; 536,007 on 6: 421 against 415; 2,055,880 on 12: 927 against 874).  The
+    // other policies are bound by FP64 and never faster with 256 (int128_grid, 2,055,880: 19.6 ms against 19.7).
+    int const block = ops_of(policy).has_mixed && total_q >= int64_t(1) << 19 ? 256 : 128;
+    b->conf = {block, 1, 512, max_depth < 32 ? 32 : 64};
     *plan = b;
     return AGWN_OK;
 }
@@ -306,7 +333,7 @@ extern "C" int agwn_batch_info(const agwn_batch* plan, int32_t* config, int32_t*
                 tune_ms[i] = plan->tune_ms[i];
     }
     if (n_items)
-        *n_items = plan->n_items;
+        *n_items = plan->n_items[items_of(plan->conf)];
     if (total_queries)
         *total_queries = plan->total_queries;
     if (total_pairs)
@@ -375,16 +402,17 @@ extern "C" int agwn_batch_run(agwn_context* ctx, agwn_batch* plan, int32_t use_g
     AGWN_CHECK_ARG(ctx->device == plan->device, "plan and context are on different devices");
     clear_message();
     AGWN_TRY_CUDA(cudaSetDevice(ctx->device));
-    if (plan->n_items == 0)
+    if (plan->total_queries == 0)
         return AGWN_OK;
     BConf const c = plan->conf;
+    int const list = items_of(c), n_items = plan->n_items[list];
     int grid = 0;
     AGWN_TRY(grid_of(*plan, *ctx, c, &grid));
-    const BItem* items = static_cast<const BItem*>(plan->items.ptr);
+    const BItem* items = static_cast<const BItem*>(plan->items.ptr) + plan->item0[list];
     if (!use_graph)
     {
         AGWN_TRY(ctx->launch_begin(AGWN_K_ROBUST));
-        AGWN_TRY(launch(*plan, *ctx, ctx->stream, c, grid, items, plan->n_items));
+        AGWN_TRY(launch(*plan, *ctx, ctx->stream, c, grid, items, n_items));
         return ctx->launch_end(AGWN_K_ROBUST);
     }
     bool const mixed = mixed_of(*plan, *ctx);
@@ -396,7 +424,7 @@ extern "C" int agwn_batch_run(agwn_context* ctx, agwn_batch* plan, int32_t use_g
     {
         drop_graph(*plan);
         AGWN_TRY_CUDA(cudaStreamBeginCapture(plan->cap, cudaStreamCaptureModeThreadLocal));
-        int const s = launch(*plan, *ctx, plan->cap, c, grid, items, plan->n_items);
+        int const s = launch(*plan, *ctx, plan->cap, c, grid, items, n_items);
         cudaGraph_t g = nullptr;
         cudaError_t const e = cudaStreamEndCapture(plan->cap, &g);
         AGWN_TRY(s);
