@@ -216,12 +216,14 @@ int fractional_launch(Context& ctx, const FracPlan<T>& p, const T* d_pos, int64_
         return fractional_split<T>(ctx, p, d_pos, n, d_out, d_counts);
     if (!p.mixed)
     {
-        // Doubles below 2^20 queries: one query per thread in blocks of 64.  The FP64 pipe is full from 8 warps, and
-        // the SMs' shares then differ by a small block (100,000 queries x 4 segments: 78 -> 73 us).  In float, two
-        // queries per thread hide the chain of one (884,736 queries x 102 segments: 412 us with one, 393 with two).
-        bool const small = sizeof(T) == 8 && n < int64_t(1) << 20;
-        int const K = small ? 1 : ctx.queries_per_thread;
-        int const block = ctx.frac_block ? ctx.frac_block : (small ? 64 : 128);
+        // Doubles: one query per thread in blocks of 64.  The FP64 and integer pipes are full from 8 warps, the SMs'
+        // shares differ by a small block (100,000 queries x 4 segments: 78 -> 73 us), and the state of a second query
+        // takes the registers that warps need (3,000,000 queries x 212 segments: 46.2 ms with one, 59.7 with two, 70.6
+        // with four).  In float, two queries per thread hide the chain of one (884,736 queries x 102 segments: 412 us
+        // with one, 393 with two).
+        constexpr bool kDouble = sizeof(T) == 8;
+        int const K = kDouble ? 1 : ctx.queries_per_thread;
+        int const block = ctx.frac_block ? ctx.frac_block : (kDouble ? 64 : 128);
         int64_t const per_tile = int64_t(block) * K;
         int64_t const n_qtiles = (n + per_tile - 1) / per_tile;
         size_t const smem = size_t(p.nbuf) * p.tile * sizeof(SegX<T>);
@@ -234,17 +236,21 @@ int fractional_launch(Context& ctx, const FracPlan<T>& p, const T* d_pos, int64_
                                                     p.n_seg, p.tile, ctx.d_flags);
             return ctx.launch_end(AGWN_K_FRACTIONAL);
         };
-        switch (K)
+        if constexpr (!kDouble)
         {
-        case 1:
-            return launch(k_frac_exact<T, 1>);
-        case 2:
-            return launch(k_frac_exact<T, 2>);
-        case 4:
-            return launch(k_frac_exact<T, 4>);
-        default:
-            return launch(k_frac_exact<T, 8>);
+            switch (K)
+            {
+            case 1:
+                break;
+            case 2:
+                return launch(k_frac_exact<T, 2>);
+            case 4:
+                return launch(k_frac_exact<T, 4>);
+            default:
+                return launch(k_frac_exact<T, 8>);
+            }
         }
+        return launch(k_frac_exact<T, 1>);
     }
     return fractional_launch_mixed(ctx, p, reinterpret_cast<const double*>(d_pos), n, reinterpret_cast<double*>(d_out),
                                    d_counts, MeshFallback{p.seg64});
