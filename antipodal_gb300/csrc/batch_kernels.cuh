@@ -146,6 +146,7 @@ __global__ void __launch_bounds__(256) k_batch(const BMesh* __restrict__ meshes,
             qv3<C> q[K];
             int cnt[K];
             double half[K];
+            RobustTerms<P> terms_of[K];
             using LV = typename RLanes<K>::V;
             LV acc[RLanes<K>::NP], comp[RLanes<K>::NP];
             int64_t idx[K];
@@ -194,7 +195,7 @@ __global__ void __launch_bounds__(256) k_batch(const BMesh* __restrict__ meshes,
                         Seg const sgm = sb[s];
 #pragma unroll
                         for (int k = 0; k < K; ++k)
-                            half[k] = __dadd_rn(half[k], __dmul_rn(sgm.w, robust_contrib<P>(q[k], sgm)));
+                            half[k] = __dadd_rn(half[k], terms_of[k].term(q[k], sgm));
                     }
                 }
                 if (!single)

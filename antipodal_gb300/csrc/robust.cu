@@ -122,15 +122,20 @@ int robust_build(Context& ctx, const T* vertices, int64_t nv, const int32_t* ind
         AGWN_TRY_CUDA(cudaStreamSynchronize(st));
     }
     AGWN_TRY_CUDA(cudaMalloc(&out->seg, sizeof(RSeg<C>) * std::max<int64_t>(1, n_seg)));
+    // int64_grid: the segments as they come, which k_robust_chain below puts in chain order
+    bool const chains = std::is_same_v<P, P64> && n_seg > 0 && n_seg < (int64_t(1) << 24);
+    Tmp unsorted(ctx);
+    if (chains)
+        AGWN_TRY(unsorted.alloc(sizeof(RSeg<C>) * n_seg));
     if (n_seg > 0)
     {
         AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
         k_robust_segs<T, P><<<g, 256, 0, st>>>(static_cast<const T*>(db), n_seg, qz,
-                                              static_cast<RSeg<C>*>(out->seg));
+                                              static_cast<RSeg<C>*>(chains ? unsorted.p : out->seg));
         AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
     }
     if constexpr (std::is_same_v<P, P64>)
-        if (n_seg > 0 && n_seg < (int64_t(1) << 24))
+        if (chains)
         {
             // the chains of the mixed form's FP32 pairs
             AGWN_TRY_CUDA(cudaMalloc(&out->chain, sizeof(RChain) * 2 * size_t(n_seg)));
@@ -138,7 +143,8 @@ int robust_build(Context& ctx, const T* vertices, int64_t nv, const int32_t* ind
             AGWN_TRY(order.alloc(sizeof(int) * std::max<int64_t>(1, chain_scratch_ints(n_seg))));
             AGWN_TRY(cnt.alloc(sizeof(long long)));
             AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-            k_robust_chain<<<1, kChainBlock, 0, st>>>(static_cast<const RSeg<int32_t>*>(out->seg), n_seg,
+            k_robust_chain<<<1, kChainBlock, 0, st>>>(static_cast<const RSeg<int32_t>*>(unsorted.p), n_seg,
+                                               static_cast<RSeg<int32_t>*>(out->seg),
                                                static_cast<RChain*>(out->chain), static_cast<long long*>(cnt.p),
                                                static_cast<int*>(order.p));
             AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));

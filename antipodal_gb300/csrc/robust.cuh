@@ -393,13 +393,16 @@ __global__ void k_robust_segs(const T* __restrict__ raw, int64_t n_seg, Quant qz
     }
 }
 
-// One block: the vertex chains of an int64_grid boundary (block_chains on the RSeg endpoints), then the entries;
-// boundaries above kChainMax segments take one chain per segment.  *n_entries receives the count.  order:
-// chain_scratch_ints(n_seg) ints of scratch.
+// One block: the vertex chains of an int64_grid boundary (block_chains on the RSeg endpoints), then the entries, and the
+// segments in the entries' order (seg_out), so that a segment mostly starts where the one before it ends and the exact
+// form keeps that end (robust_term).  Boundaries above kChainMax segments take one chain per segment and keep their
+// order.  *n_entries receives the count.  order: chain_scratch_ints(n_seg) ints of scratch.
 __global__ void __launch_bounds__(kChainBlock) k_robust_chain(const RSeg<int32_t>* __restrict__ seg, int64_t n_seg,
-                                                       RChain* __restrict__ out, long long* __restrict__ n_entries,
-                                                       int* __restrict__ order)
+                                                       RSeg<int32_t>* __restrict__ seg_out, RChain* __restrict__ out,
+                                                       long long* __restrict__ n_entries, int* __restrict__ order)
 {
+    __shared__ int s_starts[kChainBlock / 32];
+    int starts = 0; // chain starts before the current round's entries
     __shared__ int s_succ[kChainMax], s_pred[kChainMax];
     __shared__ unsigned char s_seen[kChainMax];
     __shared__ int s_m;
@@ -412,28 +415,41 @@ __global__ void __launch_bounds__(kChainBlock) k_robust_chain(const RSeg<int32_t
     int const m = chain ? mc : int(2 * n_seg);
     if (threadIdx.x == 0)
         *n_entries = m;
-    for (int e = threadIdx.x; e < m; e += blockDim.x)
+    int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int e0 = 0; e0 < m; e0 += kChainBlock)
     {
-        int si;
-        bool start;
-        if (chain)
+        int const e = e0 + int(threadIdx.x);
+        int si = -1;
+        bool start = false;
+        if (e < m)
         {
-            int const o = order[e];
+            int const o = chain ? order[e] : ((e & 1) == 0 ? ~(e >> 1) : e >> 1);
             start = o < 0;
             si = start ? ~o : o;
         }
-        else
+        unsigned const vote = __ballot_sync(0xffffffffu, start);
+        if (lane == 0)
+            s_starts[warp] = __popc(vote);
+        __syncthreads();
+        int before = starts + __popc(vote & ((1u << lane) - 1u));
+        for (int w = 0; w < kChainBlock / 32; ++w)
         {
-            si = e >> 1;
-            start = (e & 1) == 0;
+            before += w < warp ? s_starts[w] : 0;
+            starts += s_starts[w];
         }
+        __syncthreads();
+        if (e >= m)
+            continue; // the last round's tail: no barrier follows for it
         RSeg<int32_t> const g = seg[si];
+        int const place = e - before;
         RChain r{};
         for (int k = 0; k < 3; ++k)
             r.p[k] = start ? g.p0[k] : g.p1[k];
-        r.s = start ? -1 : si;
+        r.s = start ? -1 : place;
         r.w = start ? 0.f : __double2float_rn(g.w);
         out[e] = r;
+        if (!start)
+            seg_out[place] = g;
     }
 }
 
@@ -581,53 +597,73 @@ __device__ __forceinline__ double l_plus_x_small(int32_t x, int64_t yz)
     return x >= 0 ? __dadd_rn(l, vx) : div_rn_int(double_of_53(yz), __dsub_rn(l, vx));
 }
 
-// Half-area contribution of one boundary segment.  gwn_mesh_robust.hh:272-321.
 template <class P>
-__device__ __forceinline__ double robust_contrib(qv3<typename P::C> q, RSeg<typename P::C> const& s)
+__device__ __forceinline__ qv3<typename P::C> seg_diff(const typename P::C* p, qv3<typename P::C> q)
+{
+    using C = typename P::C;
+    if constexpr (P::grid)
+        return {C(p[0] - q.x), C(p[1] - q.y), C(p[2] - q.z)};
+    else
+        return {__dsub_rn(p[0], q.x), __dsub_rn(p[1], q.y), __dsub_rn(p[2], q.z)};
+}
+
+// int64_grid differences below 2^24 (every query within 16 grid extents of the mesh): all products and sums up to |v|
+// are exact integers, so they run on the integer pipe, conversions included, and 13 FP64 instructions of a term are left
+// of about 40 (150,000 queries x 41 segments: call 972 -> 536 us).
+template <class P>
+__device__ __forceinline__ bool small_diff(qv3<typename P::C> v)
+{
+    if constexpr (std::is_same_v<P, P64>)
+    {
+        unsigned const off = 1u << 24, lim = 1u << 25;
+        return unsigned(v.x) + off < lim && unsigned(v.y) + off < lim && unsigned(v.z) + off < lim;
+    }
+    else
+        return false;
+}
+
+// |v| + v.x of one end of a segment (the same bits on either path)
+template <class P>
+__device__ __forceinline__ double robust_end_general(qv3<typename P::C> v)
+{
+    ev3<rd> const d{rd(P::cdbl(v.x)), rd(P::cdbl(v.y)), rd(P::cdbl(v.z))};
+    return l_plus_x<P>(v, ex_sqrt(edot(d, d)).v);
+}
+template <class P>
+__device__ __forceinline__ double robust_end(qv3<typename P::C> v)
+{
+    if constexpr (std::is_same_v<P, P64>)
+        if (small_diff<P>(v))
+            return l_plus_x_small(v.x, int64_t(v.y) * v.y + int64_t(v.z) * v.z);
+    return robust_end_general<P>(v);
+}
+
+// Half-area contribution of one boundary segment from its ends' b = |v| + v.x.  gwn_mesh_robust.hh:272-321.
+template <class P>
+__device__ __forceinline__ double robust_contrib(qv3<typename P::C> q, RSeg<typename P::C> const& s, double b0,
+                                                 double b1)
 {
     using C = typename P::C;
     constexpr double pi = 3.141592653589793238462643383279502884;
     qv3<C> const p0{s.p0[0], s.p0[1], s.p0[2]}, p1{s.p1[0], s.p1[1], s.p1[2]};
-    qv3<C> v0, v1;
-    if constexpr (P::grid)
-    {
-        v0 = {C(p0.x - q.x), C(p0.y - q.y), C(p0.z - q.z)};
-        v1 = {C(p1.x - q.x), C(p1.y - q.y), C(p1.z - q.z)};
-    }
-    else
-    {
-        v0 = {__dsub_rn(p0.x, q.x), __dsub_rn(p0.y, q.y), __dsub_rn(p0.z, q.z)};
-        v1 = {__dsub_rn(p1.x, q.x), __dsub_rn(p1.y, q.y), __dsub_rn(p1.z, q.z)};
-    }
+    qv3<C> const v0 = seg_diff<P>(s.p0, q), v1 = seg_diff<P>(s.p1, q);
+    double const bb = __dmul_rn(b0, b1);
     double den;
-    bool small = false;
-    if constexpr (std::is_same_v<P, P64>)
+    bool const small = small_diff<P>(v0) && small_diff<P>(v1);
+    if (small)
     {
-        // Differences below 2^24 (every query within 16 grid extents of the mesh): all products and sums up to l are
-        // exact integers, so they run on the integer pipe, conversions included, and 13 FP64 instructions are left
-        // of about 40 (150,000 queries x 41 segments: call 972 -> 536 us).
-        unsigned const off = 1u << 24, lim = 1u << 25;
-        small = unsigned(v0.x) + off < lim && unsigned(v0.y) + off < lim && unsigned(v0.z) + off < lim &&
-                unsigned(v1.x) + off < lim && unsigned(v1.y) + off < lim && unsigned(v1.z) + off < lim;
-        if (small)
+        if constexpr (std::is_same_v<P, P64>)
         {
             int64_t const n = int64_t(v0.z) * v1.y - int64_t(v0.y) * v1.z;
-            double const b0 = l_plus_x_small(v0.x, int64_t(v0.y) * v0.y + int64_t(v0.z) * v0.z);
-            double const b1 = l_plus_x_small(v1.x, int64_t(v1.y) * v1.y + int64_t(v1.z) * v1.z);
-            den = __dadd_rn(__dmul_rn(b0, b1), double_of_53(int64_t(v0.y) * v1.y + int64_t(v0.z) * v1.z));
+            den = __dadd_rn(bb, double_of_53(int64_t(v0.y) * v1.y + int64_t(v0.z) * v1.z));
             if (n != 0)
                 return atan2_int(double_of_53(n), den);
         }
     }
-    if (!small)
+    else
     {
-        ev3<rd> const d0{rd(P::cdbl(v0.x)), rd(P::cdbl(v0.y)), rd(P::cdbl(v0.z))};
-        ev3<rd> const d1{rd(P::cdbl(v1.x)), rd(P::cdbl(v1.y)), rd(P::cdbl(v1.z))};
-        double const l0 = ex_sqrt(edot(d0, d0)).v;
-        double const l1 = ex_sqrt(edot(d1, d1)).v;
         auto const num = atan2_num<P>(q, p0, p1);
-        double const yz = dot_yz<P>(v0, v1);
-        den = __dadd_rn(__dmul_rn(l_plus_x<P>(v0, l0), l_plus_x<P>(v1, l1)), yz);
+        den = __dadd_rn(bb, dot_yz<P>(v0, v1));
         if (P::sgn(num) != 0)
             return atan2_int(P::dbl(num), den);
     }
@@ -638,6 +674,42 @@ __device__ __forceinline__ double robust_contrib(qv3<typename P::C> q, RSeg<type
     int const sg = -edge_sign<P>(q, p0, p1);
     return den < 0.0 ? double(sg) * pi : 0.0;
 }
+template <class P>
+__device__ __forceinline__ double robust_contrib(qv3<typename P::C> q, RSeg<typename P::C> const& s)
+{
+    return robust_contrib<P>(q, s, robust_end<P>(seg_diff<P>(s.p0, q)), robust_end<P>(seg_diff<P>(s.p1, q)));
+}
+
+__device__ __forceinline__ bool same_coord(int32_t a, int32_t b) { return a == b; }
+__device__ __forceinline__ bool same_coord(int64_t a, int64_t b) { return a == b; }
+__device__ __forceinline__ bool same_coord(double a, double b)
+{
+    return __double_as_longlong(a) == __double_as_longlong(b);
+}
+
+// The weighted contributions of a run of segments in order: the end of the segment before is kept, and a segment that
+// starts there (most do in chain order, k_robust_chain) works out one end instead of two.
+template <class P>
+struct RobustTerms
+{
+    using C = typename P::C;
+    C last[3];
+    double b = 0.0;
+    bool any = false;
+
+    __device__ __forceinline__ double term(qv3<C> q, RSeg<C> const& s)
+    {
+        // (the same for every query of a block)
+        if (!any || !same_coord(s.p0[0], last[0]) || !same_coord(s.p0[1], last[1]) || !same_coord(s.p0[2], last[2]))
+            b = robust_end<P>(seg_diff<P>(s.p0, q));
+        any = true;
+        for (int k = 0; k < 3; ++k)
+            last[k] = s.p1[k];
+        double const b0 = b;
+        b = robust_end<P>(seg_diff<P>(s.p1, q));
+        return __dmul_rn(s.w, robust_contrib<P>(q, s, b0, b));
+    }
+};
 
 // ---- mixed precision (int64_grid) -------------------------------------------------------------------------------
 // Per-warp queue of the pairs the FP32 path turned down, evaluated in FP64 32 at a time (one per lane), so
@@ -889,10 +961,11 @@ __global__ void __launch_bounds__(32 * kSplitWarps)
     int const i = int(blockIdx.x) * 32 + lane, ii = min(i, n - 1);
     auto const q = quantize<P>(double(pos[3 * ii]), double(pos[3 * ii + 1]), double(pos[3 * ii + 2]), qz);
     int const s0 = min((int(blockIdx.y) * kSplitWarps + warp) * g, n_seg), s1 = min(s0 + g, n_seg);
+    RobustTerms<P> terms_of;
     for (int s = s0; s < s1; ++s)
     {
         RSeg<typename P::C> const sg = seg[s];
-        double const term = __dmul_rn(sg.w, robust_contrib<P>(q, sg));
+        double const term = terms_of.term(q, sg);
         if (i < n)
             terms[size_t(s) * n + i] = term;
     }
@@ -984,6 +1057,7 @@ __global__ void __launch_bounds__(kRobBlock) k_robust_frac(const T* __restrict__
         int64_t const ii = i < n ? i : n - 1;
         auto const q = quantize<P>(double(pos[3 * ii]), double(pos[3 * ii + 1]), double(pos[3 * ii + 2]), qz);
         double half = 0.0;
+        RobustTerms<P> terms_of;
         float acc[1] = {0.f}, comp[1] = {0.f};
         decltype(q) qarr[1] = {q};
         double harr[1] = {0.0};
@@ -1016,7 +1090,7 @@ __global__ void __launch_bounds__(kRobBlock) k_robust_frac(const T* __restrict__
                 for (int s = 0; s < cnt; ++s)
                 {
                     Seg const sgm = sb[s];
-                    half = __dadd_rn(half, __dmul_rn(sgm.w, robust_contrib<P>(q, sgm)));
+                    half = __dadd_rn(half, terms_of.term(q, sgm));
                 }
             }
             if (!pipe.single)
