@@ -219,8 +219,8 @@ int fractional_launch(Context& ctx, const FracPlan<T>& p, const T* d_pos, int64_
         // Doubles: one query per thread in blocks of 64.  The FP64 and integer pipes are full from 8 warps, the SMs'
         // shares differ by a small block (100,000 queries x 4 segments: 78 -> 73 us), and the state of a second query
         // takes the registers that warps need (3,000,000 queries x 212 segments: 46.2 ms with one, 59.7 with two, 70.6
-        // with four).  In float, two queries per thread hide the chain of one (884,736 queries x 102 segments: 412 us
-        // with one, 393 with two).
+        // with four).  In float, two queries per thread make a packed pair (900,000 queries x 102 segments: 326 us with
+        // one, 270 with two, 285 with four).
         constexpr bool kDouble = sizeof(T) == 8;
         int const K = kDouble ? 1 : ctx.queries_per_thread;
         int const block = ctx.frac_block ? ctx.frac_block : (kDouble ? 64 : 128);

@@ -104,6 +104,291 @@ __global__ void k_prep_exact(const T* __restrict__ raw, int64_t n_seg, SegX<T>* 
     }
 }
 
+// The same operations on a lane vector: one query (float) or a packed pair of queries (float2, the paired add /
+// multiply / FMA instructions of sm_100 and later, one instruction for both).  Each lane is rounded as the scalar
+// operation would be, so code written over a lane vector gives bit-identical lanes for one query per thread and
+// for two.
+__device__ __forceinline__ float lv_add(float a, float b)
+{
+    return __fadd_rn(a, b);
+}
+__device__ __forceinline__ float lv_mul(float a, float b)
+{
+    return __fmul_rn(a, b);
+}
+__device__ __forceinline__ float lv_fma(float a, float b, float c)
+{
+    return __fmaf_rn(a, b, c);
+}
+__device__ __forceinline__ float2 lv_add(float2 a, float2 b)
+{
+    return __fadd2_rn(a, b);
+}
+__device__ __forceinline__ float2 lv_mul(float2 a, float2 b)
+{
+    return __fmul2_rn(a, b);
+}
+__device__ __forceinline__ float2 lv_fma(float2 a, float2 b, float2 c)
+{
+    return __ffma2_rn(a, b, c);
+}
+template <class V>
+__device__ __forceinline__ V lv_set(float x)
+{
+    if constexpr (std::is_same_v<V, float>)
+        return x;
+    else
+        return make_float2(x, x);
+}
+// a - b, rounded once
+template <class V>
+__device__ __forceinline__ V lv_sub(V a, V b)
+{
+    return lv_fma(b, lv_set<V>(-1.f), a);
+}
+// lane h of a lane vector
+__device__ __forceinline__ float& ln(float& v, int)
+{
+    return v;
+}
+__device__ __forceinline__ float ln(float const& v, int)
+{
+    return v;
+}
+__device__ __forceinline__ float& ln(float2& v, int h)
+{
+    return h ? v.y : v.x;
+}
+__device__ __forceinline__ float ln(float2 const& v, int h)
+{
+    return h ? v.y : v.x;
+}
+// -a by its sign bits (the integer pipe has room where the FMA pipe is full)
+__device__ __forceinline__ float lv_flip(float a)
+{
+    return __uint_as_float(__float_as_uint(a) ^ 0x80000000u);
+}
+__device__ __forceinline__ float2 lv_flip(float2 a)
+{
+    return make_float2(lv_flip(a.x), lv_flip(a.y));
+}
+
+// ---- the float form on lane vectors: one query (float) or a pair of them (float2, packed FP32 instructions) ----
+// Every product and sum of the reference's float arithmetic, each rounded by itself and in its order.  The square root
+// is correctly rounded, the arctangent the fit below; either vector gives a query the same bits.
+//
+// What bounds it: the FMA pipe (74% busy).  As scalar code with the library's square root and atan2f a term took 120
+// instructions at 90% of the issue slots; now 69 (884,736 queries x 102 segments: kernel 328 -> 270 us).
+
+// Whether x is outside [2^-100, 2^100): zeros, subnormals, infinities and NaN too.
+__device__ __forceinline__ bool off_range(float x)
+{
+    return __float_as_uint(x) - 0x0d800000u >= 0x64000000u;
+}
+
+// sqrt(a), a sum of squares: one correction of the approximate root by its exact residual (Markstein 1990)
+template <class V>
+__device__ __forceinline__ V sqrt_lv(V a)
+{
+    constexpr int W = sizeof(V) / sizeof(float);
+    V y;
+    bool odd = false;
+#pragma unroll
+    for (int h = 0; h < W; ++h)
+    {
+        ln(y, h) = rsqrt_approx(ln(a, h));
+        odd |= off_range(ln(a, h));
+    }
+    V const g = lv_mul(a, y), hy = lv_mul(y, lv_set<V>(0.5f));
+    V const e = lv_fma(lv_flip(g), g, a);
+    V r = lv_fma(e, hy, g);
+    if (odd)
+    {
+#pragma unroll
+        for (int h = 0; h < W; ++h)
+            if (off_range(ln(a, h)))
+                ln(r, h) = __fsqrt_rn(ln(a, h));
+    }
+    return r;
+}
+
+// atan2(n, d): with q = min / max of the magnitudes and its exact residual r in units of the quotient, atan(q + r) =
+// q + (q^3 Q(q^2) + r / (1 + q^2)), Q of degree 7 (a minimax fit, relative error of atan 1.7e-8) and 1 / (1 + q^2) by a
+// line (4% is near enough for r), then +-atan + {0, pi/2, pi} in one FMA: pi/2 is 1.8663789 x 0.84162778 to 1.6e-14.
+// Against 64 bits over 4,194,304 random and skewed arguments: mean error 0.26 ulp, largest 1.38 (the library's atan2f:
+// 0.28 and 1.79).
+template <class V>
+__device__ __forceinline__ V atan2_lv(V n, V d)
+{
+    constexpr int W = sizeof(V) / sizeof(float);
+    V mn, mx, rc, base, a;
+    uint32_t flip[W];
+    bool odd = false;
+#pragma unroll
+    for (int h = 0; h < W; ++h)
+    {
+        float const an = fabsf(ln(n, h)), ad = fabsf(ln(d, h));
+        bool const swap = an > ad, neg = ln(d, h) < 0.f;
+        ln(mx, h) = swap ? an : ad; // a NaN ends up in mx, or in mn and so in t
+        ln(mn, h) = swap ? ad : an;
+        odd |= off_range(ln(mx, h));
+        ln(rc, h) = rcp_approx(ln(mx, h));
+        ln(base, h) = swap ? 1.8663789033889771f : (neg ? 3.7327578067779541f : 0.f);
+        flip[h] = swap != neg ? 0x80000000u : 0u;
+    }
+    V const q = lv_mul(mn, rc);
+    V const rem = lv_mul(lv_fma(lv_flip(q), mx, mn), rc);
+    V const s = lv_mul(q, q);
+    V const slope = lv_fma(lv_set<V>(-0.5f), s, lv_set<V>(0.95710678f));
+    V p = lv_set<V>(0.002920688595622778f);
+    p = lv_fma(p, s, lv_set<V>(-0.016367914155125618f));
+    p = lv_fma(p, s, lv_set<V>(0.043211836367845535f));
+    p = lv_fma(p, s, lv_set<V>(-0.07552212476730347f));
+    p = lv_fma(p, s, lv_set<V>(0.10666003823280334f));
+    p = lv_fma(p, s, lv_set<V>(-0.14211055636405945f));
+    p = lv_fma(p, s, lv_set<V>(0.19993773102760315f));
+    p = lv_fma(p, s, lv_set<V>(-0.33333152532577515f));
+    a = lv_add(q, lv_fma(lv_mul(q, s), p, lv_mul(rem, slope)));
+#pragma unroll
+    for (int h = 0; h < W; ++h)
+        ln(a, h) = __uint_as_float(__float_as_uint(ln(a, h)) ^ flip[h]);
+    V r = lv_fma(base, lv_set<V>(0.84162777662277222f), a);
+#pragma unroll
+    for (int h = 0; h < W; ++h)
+        ln(r, h) = copysignf(ln(r, h), ln(n, h));
+    if (odd)
+    {
+#pragma unroll
+        for (int h = 0; h < W; ++h)
+            if (off_range(ln(mx, h)))
+                ln(r, h) = atan2f(ln(n, h), ln(d, h));
+    }
+    return r;
+}
+
+template <class V>
+struct LV3
+{
+    V x, y, z;
+};
+// The compiler fuses a packed product and the packed sum that reads it into one FMA, which rounds once (a third of
+// 1,048,576 random dot products differed).  So no sum below reads a product: every one is a difference from a product
+// with one factor negated, and a difference is an FMA itself (lv_sub).
+// a . b from b and nb = -b
+template <class V>
+__device__ __forceinline__ V lv_dot(LV3<V> const& a, LV3<V> const& b, LV3<V> const& nb)
+{
+    return lv_sub(lv_sub(lv_mul(a.x, b.x), lv_mul(a.y, nb.y)), lv_mul(a.z, nb.z));
+}
+template <class V>
+__device__ __forceinline__ LV3<V> lv_neg(LV3<V> const& a)
+{
+    return {lv_flip(a.x), lv_flip(a.y), lv_flip(a.z)};
+}
+template <class V>
+__device__ __forceinline__ V lv_det(V a, V b, V c, V d)
+{
+    return lv_sub(lv_mul(a, b), lv_mul(c, d));
+}
+template <class V>
+__device__ __forceinline__ LV3<V> lv_splat(float x, float y, float z)
+{
+    return {lv_set<V>(x), lv_set<V>(y), lv_set<V>(z)};
+}
+// vos_exact in float of a segment from v0 to v1; nx1 = -x1
+template <class V>
+__device__ __forceinline__ V vos_float(LV3<V> const& x1, LV3<V> const& nx1, LV3<V> const& v0, LV3<V> const& v1)
+{
+    LV3<V> const n0 = lv_neg(v0), n1 = lv_neg(v1);
+    V const l0 = sqrt_lv(lv_dot(v0, v0, n0)), l1 = sqrt_lv(lv_dot(v1, v1, n1));
+    LV3<V> const c{lv_det(v0.y, v1.z, v0.z, v1.y), lv_det(v0.z, v1.x, v0.x, v1.z), lv_det(v0.x, v1.y, v0.y, v1.x)};
+    V const nd0 = lv_dot(v0, nx1, x1), nd1 = lv_dot(v1, nx1, x1); // -x1 . v0, -x1 . v1
+    V const den = lv_add(lv_sub(lv_sub(lv_mul(l0, l1), lv_mul(l1, nd0)), lv_mul(l0, nd1)), lv_dot(v0, v1, n1));
+    return atan2_lv(lv_dot(c, x1, nx1), den);
+}
+
+// A thread's K queries in the exact form: their running sums over the segments.
+template <class T, int K>
+struct ExactSums
+{
+    using S = typename exact_int_of<T>::type;
+    ev3<S> p[K];
+    S area[K];
+    End<S> e0[K], e1[K];
+
+    __device__ __forceinline__ void load(int k, const T* q)
+    {
+        p[k] = {S(q[0]), S(q[1]), S(q[2])};
+        area[k] = S(T(0));
+    }
+    __device__ __forceinline__ T sum(int k) const
+    {
+        return area[k].v;
+    }
+    __device__ __forceinline__ void add(SegX<T> const& g, const T* x)
+    {
+        ev3<S> const x1{S(x[0]), S(x[1]), S(x[2])};
+        ev3<S> const a{S(g.p0x), S(g.p0y), S(g.p0z)};
+        ev3<S> const c{S(g.p1x), S(g.p1y), S(g.p1z)};
+        // The ends of the segment before are at hand, and one that is shared is not worked out again (44% of an
+        // icosphere's boundary segments share one: 261,632 queries x 102 segments, 2249 -> 2096 us; a cube's four,
+        // 57 -> 52).
+        bool const back = g.shared == T(2);
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+        {
+            if (g.shared == T(0))
+                e0[k] = end_exact(x1, a - p[k]);
+            else if (!back)
+                e0[k] = e1[k];
+            else
+                e1[k] = e0[k];
+            End<S> const e = end_exact(x1, (back ? a : c) - p[k]);
+            if (back)
+                e0[k] = e;
+            else
+                e1[k] = e;
+            S const term = S(vos_ends(x1, e0[k], e1[k]));
+            area[k] = area[k] + (g.w == T(1) ? term : S(g.w) * term); // the same for a weight of 1
+        }
+    }
+};
+// In float both ends are worked out: a kept one costs registers and a branch (884,736 queries x 102 segments: kernel 270
+// -> 316 us).
+template <int K>
+struct ExactSums<float, K>
+{
+    using V = std::conditional_t<K == 1, float, float2>;
+    static constexpr int W = K == 1 ? 1 : 2, NP = K / W;
+    LV3<V> p[NP];
+    V area[NP];
+
+    __device__ __forceinline__ void load(int k, const float* q)
+    {
+        ln(p[k / W].x, k % W) = q[0];
+        ln(p[k / W].y, k % W) = q[1];
+        ln(p[k / W].z, k % W) = q[2];
+        ln(area[k / W], k % W) = 0.f;
+    }
+    __device__ __forceinline__ float sum(int k) const
+    {
+        return ln(area[k / W], k % W);
+    }
+    __device__ __forceinline__ void add(SegX<float> const& g, const float* x)
+    {
+        LV3<V> const x1 = lv_splat<V>(x[0], x[1], x[2]), nx1 = lv_splat<V>(-x[0], -x[1], -x[2]);
+        LV3<V> const a = lv_splat<V>(g.p0x, g.p0y, g.p0z), c = lv_splat<V>(g.p1x, g.p1y, g.p1z);
+        V const nw = lv_set<V>(-g.w);
+#pragma unroll
+        for (int k = 0; k < NP; ++k)
+        {
+            LV3<V> const v0{lv_sub(a.x, p[k].x), lv_sub(a.y, p[k].y), lv_sub(a.z, p[k].z)};
+            LV3<V> const v1{lv_sub(c.x, p[k].x), lv_sub(c.y, p[k].y), lv_sub(c.z, p[k].z)};
+            area[k] = lv_sub(area[k], lv_mul(nw, vos_float(x1, nx1, v0, v1)));
+        }
+    }
+};
+
 // Shared skeleton of both fractional kernels: persistent CTAs over query tiles, segment tiles in shared memory.
 // Policy provides: Seg type, per-thread state init (load), per-segment accumulate, and finish (store).
 template <class Seg>
@@ -172,24 +457,19 @@ __global__ void __launch_bounds__(256) k_frac_exact(const T* __restrict__ pos, i
     }
     __syncthreads();
 
-    S const x1x = S(-x0x), x1y = S(-x0y), x1z = S(-x0z);
-    ev3<S> const x1{x1x, x1y, x1z};
+    T const x1[3] = {-x0x, -x0y, -x0z};
     T const two_pi = T(2) * kPi<T>;
 
     int it = 0;
     for (int j = 0; j < my_qtiles; ++j)
     {
         int64_t const base = (blockIdx.x + int64_t(j) * gridDim.x) * per_tile + threadIdx.x;
-        ev3<S> p[K];
-        S area[K];
-        End<S> e0[K], e1[K];
+        ExactSums<T, K> sums;
 #pragma unroll
         for (int k = 0; k < K; ++k)
         {
             int64_t const i = base + int64_t(k) * blockDim.x;
-            int64_t const ii = i < n ? i : n - 1;
-            p[k] = {S(pos[3 * ii]), S(pos[3 * ii + 1]), S(pos[3 * ii + 2])};
-            area[k] = S(T(0));
+            sums.load(k, pos + 3 * (i < n ? i : n - 1));
         }
         for (int st = 0; st < pipe.n_tiles; ++st)
         {
@@ -206,33 +486,7 @@ __global__ void __launch_bounds__(256) k_frac_exact(const T* __restrict__ pos, i
             SegX<T> const* sb = pipe.buf[b];
             int const cnt = pipe.tile_count(st);
             for (int s = 0; s < cnt; ++s)
-            {
-                SegX<T> const g = sb[s];
-                ev3<S> const a{S(g.p0x), S(g.p0y), S(g.p0z)};
-                ev3<S> const c{S(g.p1x), S(g.p1y), S(g.p1z)};
-                S const w = S(g.w);
-                // Doubles: the ends of the segment before are at hand, and one that is shared is not worked out again
-                // (44% of an icosphere's boundary segments share one: 261,632 queries x 102 segments, 2249 ->
-                // 2096 us; a cube's four, 57 -> 52).  In float the branch costs more than the end (394 -> 426 us).
-                bool const keep = sizeof(T) == 8, back = keep && g.shared == T(2);
-#pragma unroll
-                for (int k = 0; k < K; ++k)
-                {
-                    if (!keep || g.shared == T(0))
-                        e0[k] = end_exact(x1, a - p[k]);
-                    else if (!back)
-                        e0[k] = e1[k];
-                    else
-                        e1[k] = e0[k];
-                    End<S> const e = end_exact(x1, (back ? a : c) - p[k]);
-                    if (back)
-                        e0[k] = e;
-                    else
-                        e1[k] = e;
-                    S const term = S(vos_ends(x1, e0[k], e1[k]));
-                    area[k] = area[k] + (g.w == T(1) ? term : w * term); // the same for a weight of 1
-                }
-            }
+                sums.add(sb[s], x1);
             if (!pipe.single)
             {
                 __syncthreads();
@@ -247,7 +501,7 @@ __global__ void __launch_bounds__(256) k_frac_exact(const T* __restrict__ pos, i
             int64_t const i = base + int64_t(k) * blockDim.x;
             if (i < n)
             {
-                S v = area[k] / S(two_pi);
+                S v = S(sums.sum(k)) / S(two_pi);
                 if (counts)
                     v = v + S(T(counts[i]));
                 out[i] = v.v;
@@ -281,9 +535,21 @@ __global__ void __launch_bounds__(32 * kSplitWarps)
     for (int s = s0; s < s1; ++s)
     {
         const T* const r = raw + 7 * size_t(s);
-        ev3<S> const v0 = ev3<S>{S(__ldg(r)), S(__ldg(r + 1)), S(__ldg(r + 2))} - p;
-        ev3<S> const v1 = ev3<S>{S(__ldg(r + 3)), S(__ldg(r + 4)), S(__ldg(r + 5))} - p;
-        S const term = S(__ldg(r + 6)) * S(vos_exact(x1, v0, v1));
+        S term;
+        if constexpr (sizeof(T) == 4)
+        {
+            LV3<float> const v0{__fsub_rn(__ldg(r), p.x.v), __fsub_rn(__ldg(r + 1), p.y.v),
+                                __fsub_rn(__ldg(r + 2), p.z.v)};
+            LV3<float> const v1{__fsub_rn(__ldg(r + 3), p.x.v), __fsub_rn(__ldg(r + 4), p.y.v),
+                                __fsub_rn(__ldg(r + 5), p.z.v)};
+            term = S(__ldg(r + 6)) * S(vos_float({x1.x.v, x1.y.v, x1.z.v}, {-x1.x.v, -x1.y.v, -x1.z.v}, v0, v1));
+        }
+        else
+        {
+            ev3<S> const v0 = ev3<S>{S(__ldg(r)), S(__ldg(r + 1)), S(__ldg(r + 2))} - p;
+            ev3<S> const v1 = ev3<S>{S(__ldg(r + 3)), S(__ldg(r + 4)), S(__ldg(r + 5))} - p;
+            term = S(__ldg(r + 6)) * S(vos_exact(x1, v0, v1));
+        }
         if (i < n)
             terms[size_t(s) * n + i] = term.v;
     }
@@ -786,65 +1052,6 @@ __device__ __forceinline__ void fp64_flush(Fp64Queue<K>& q, unsigned c, int lane
     q.head += c;
 }
 
-// The same operations on a lane vector: one query (float) or a packed pair of queries (float2, the paired add /
-// multiply / FMA instructions of sm_100 and later, one instruction for both).  Each lane is rounded as the scalar
-// operation would be, so code written over a lane vector gives bit-identical lanes for one query per thread and
-// for two.
-__device__ __forceinline__ float lv_add(float a, float b)
-{
-    return __fadd_rn(a, b);
-}
-__device__ __forceinline__ float lv_mul(float a, float b)
-{
-    return __fmul_rn(a, b);
-}
-__device__ __forceinline__ float lv_fma(float a, float b, float c)
-{
-    return __fmaf_rn(a, b, c);
-}
-__device__ __forceinline__ float2 lv_add(float2 a, float2 b)
-{
-    return __fadd2_rn(a, b);
-}
-__device__ __forceinline__ float2 lv_mul(float2 a, float2 b)
-{
-    return __fmul2_rn(a, b);
-}
-__device__ __forceinline__ float2 lv_fma(float2 a, float2 b, float2 c)
-{
-    return __ffma2_rn(a, b, c);
-}
-template <class V>
-__device__ __forceinline__ V lv_set(float x)
-{
-    if constexpr (std::is_same_v<V, float>)
-        return x;
-    else
-        return make_float2(x, x);
-}
-// a - b, rounded once
-template <class V>
-__device__ __forceinline__ V lv_sub(V a, V b)
-{
-    return lv_fma(b, lv_set<V>(-1.f), a);
-}
-// lane h of a lane vector
-__device__ __forceinline__ float& ln(float& v, int)
-{
-    return v;
-}
-__device__ __forceinline__ float ln(float const& v, int)
-{
-    return v;
-}
-__device__ __forceinline__ float& ln(float2& v, int h)
-{
-    return h ? v.y : v.x;
-}
-__device__ __forceinline__ float ln(float2 const& v, int h)
-{
-    return h ? v.y : v.x;
-}
 // Compensated accumulation: acc + x by TwoSum (Knuth), its exact rounding error added to comp.  The pair
 // (acc, comp) carries the sum to well below float's rounding, independently of the order of the terms.
 template <class V>
