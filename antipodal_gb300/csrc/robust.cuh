@@ -810,6 +810,9 @@ struct RVState
 // the reference takes its exact branches), a difference of 2^24 or more and ill-conditioned pairs go to FP64 with
 // the reference's formula.  The arithmetic runs on lane vectors (RLanes), so one query per thread and packed
 // pairs give the same bits; selects and comparisons per lane.
+// The inputs of the reciprocal and its root are normal or zero, so they are the bare instructions (approx.cuh); without
+// the library forms' subnormal handling the batch kernel also takes 64 registers where it took 80 (16 meshes of up to
+// 20,000 triangles, 72^3 grids: 1516 -> 1294 us).
 template <int K>
 __device__ __forceinline__ void robust_chain_entry(RChain const& e, qv3<int32_t> const (&q)[K],
                                                    RVState<typename RLanes<K>::V> (&pv)[RLanes<K>::NP],
@@ -841,7 +844,7 @@ __device__ __forceinline__ void robust_chain_entry(RChain const& e, qv3<int32_t>
         V rs;
 #pragma unroll
         for (int h = 0; h < L::W; ++h)
-            ln(rs, h) = rsqrtf(ln(sq, h));
+            ln(rs, h) = rsqrt_approx(ln(sq, h));
         V const l = lv_mul(sq, rs);
         V const lpx = lv_add(l, c.x), lmx = lv_sub(l, c.x);
 #pragma unroll
@@ -854,18 +857,17 @@ __device__ __forceinline__ void robust_chain_entry(RChain const& e, qv3<int32_t>
     }
     if (e.s < 0)
         return; // a chain start: its vertex only
-    V const m1 = lv_set<V>(-1.f);
 #pragma unroll
     for (int p = 0; p < L::NP; ++p)
     {
         RVState<V> const& a = pv[p];
         RVState<V> const& b = cv[p];
         V const pn = lv_mul(a.y, b.z);
-        V const npn = lv_mul(pn, m1);
+        V const npn = lv_flip(pn);
         V const en = lv_fma(a.y, b.z, npn);
         V const numf = lv_sub(lv_fma(a.z, b.y, npn), en);
         V const pz = lv_mul(a.z, b.z);
-        V const ez = lv_fma(a.z, b.z, lv_mul(pz, m1));
+        V const ez = lv_fma(a.z, b.z, lv_flip(pz));
         V const yzf = lv_add(lv_fma(a.y, b.y, pz), ez);
         V const D = lv_mul(a.d, b.d), ab = lv_mul(a.n, b.n), yzs = lv_mul(yzf, D);
         V const num_s = lv_mul(numf, D), den_s = lv_add(ab, yzs);
@@ -878,7 +880,7 @@ __device__ __forceinline__ void robust_chain_entry(RChain const& e, qv3<int32_t>
             swap[h] = anh > adh;
             ln(an, h) = anh;
             ln(ad, h) = adh;
-            ln(inv, h) = __fdividef(1.f, fmaxf(swap[h] ? anh : adh, 1e-37f));
+            ln(inv, h) = rcp_approx(fmaxf(swap[h] ? anh : adh, 1e-37f));
             ln(sab, h) = __fadd_rn(fabsf(ln(ab, h)), fabsf(ln(yzs, h)));
         }
         V const an1 = lv_mul(an, inv), ad1 = lv_mul(ad, inv);
