@@ -616,7 +616,7 @@ __device__ __forceinline__ bool small_diff(qv3<typename P::C> v)
     if constexpr (std::is_same_v<P, P64>)
     {
         unsigned const off = 1u << 24, lim = 1u << 25;
-        return unsigned(v.x) + off < lim && unsigned(v.y) + off < lim && unsigned(v.z) + off < lim;
+        return ((unsigned(v.x) + off) | (unsigned(v.y) + off) | (unsigned(v.z) + off)) < lim; // 2^25
     }
     else
         return false;
@@ -834,7 +834,7 @@ __device__ __forceinline__ void robust_chain_entry(RChain const& e, qv3<int32_t>
         {
             int const k = p * L::W + h;
             int32_t const vx = e.p[0] - q[k].x, vy = e.p[1] - q[k].y, vz = e.p[2] - q[k].z;
-            small[h] = unsigned(vx) + off < lim && unsigned(vy) + off < lim && unsigned(vz) + off < lim;
+            small[h] = ((unsigned(vx) + off) | (unsigned(vy) + off) | (unsigned(vz) + off)) < lim; // 2^25
             ln(c.x, h) = float(vx);
             ln(c.y, h) = float(vy);
             ln(c.z, h) = float(vz);
