@@ -132,6 +132,7 @@ struct CellGrid
     int64_t entries = 0;
     int per_leaf = 0;   // cells per leaf it was built with
     int64_t calls = 0;  // calls prepared for on this hierarchy so far
+    bool pinned = false; // a captured call reads it: its buffers stay as they are
     bool valid = false;
     void release()
     {
@@ -211,11 +212,11 @@ struct Context
 
     // Whether a mixed-mode call of `pairs` (query, segment) pairs over a boundary of n_seg segments runs the mixed
     // kernels: at least mixed_min_pairs pairs over at least kMixedMinSegments segments, or always with the minimum 0.
-    // The exact kernel's time follows the boundary's length (each thread's chain of FP64 terms), the mixed kernel's
-    // has a fixed part (the boundary's preparation) and, over long segments, many pairs within the near distance
-    // that go to FP64 anyway: on a GB300 the exact kernels were faster below 32 segments at every query count tried
-    // (2,000 to 200,000 random queries; 4 segments and 2e5 queries: 202 against 297 us), the mixed ones from 64
-    // segments at every count (64 segments and 2,000 queries: 293 against 537 us; 128: 198 against 1,065 us).
+    // The mixed kernel has a fixed part (the boundary's preparation) and, over long segments, many pairs within the near
+    // distance that go to FP64 anyway.  The line was drawn where the two met when the exact kernels took 8 us a segment:
+    // faster below 32 segments at every query count tried (2,000 to 200,000 random queries).  They take less now (257
+    // queries x 24 segments 55 us, 261,632 x 102 2.1 ms), but the two forms' values differ by up to 6e-8 a term, so the
+    // line stays where calls expect it.
     static constexpr int64_t kMixedMinSegments = 32;
     bool use_mixed(double pairs, int64_t n_seg) const
     {

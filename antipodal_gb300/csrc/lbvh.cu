@@ -920,6 +920,7 @@ int ray_hierarchy(Context& ctx, const Bvh& bvh, const T* dir_host)
     rc.generation = 0; // invalid until the build completes
     rc.cells.valid = false;
     rc.cells.calls = 0;
+    rc.cells.pinned = false;
     AGWN_TRY(build_hier<T>(ctx, static_cast<const T*>(bvh.tri), bvh.n_tri, dir, rc.h, nullptr));
     std::memcpy(rc.dir, dir, sizeof(dir));
     rc.scalar_bytes = bvh.scalar_bytes;
@@ -932,11 +933,11 @@ int ray_hierarchy(Context& ctx, const Bvh& bvh, const T* dir_host)
 // The cell grid of the cached hierarchy (its leaves' float (u, v) corners), about per_leaf cells per leaf over the
 // widened boxes' extent (at most 2^22 cells).  Finer cells hold fewer leaves, so a query reads fewer list entries:
 // on a 76,496-triangle icosphere with 256^3 grid queries 2 cells per leaf read 5.06 entries per query (1.09 ms),
-// 16 read 3.49 (0.83 ms); 32 and 64 gained no more.  But a fine grid takes longer to build (two passes of
-// 40 us against 16 there), so a mesh that is new on every call gets the coarse one (integer_prepare).  Leaf boxes are widened by
-// 4 * 2^-18 of the scene scale; a query takes the grid while its own tolerance (qmax + scene) * 2^-18 stays below 3.5 * 2^-18 of the scene scale
-// (qmax <= 2.5 * scene), which leaves room for the one-ulp difference between the corners and the walk's
-// outward-rounded boxes.
+// 16 read 3.49 (0.83 ms); 32 and 64 gained no more.  But a fine grid takes longer to build (two passes of 40 us against
+// 16 there), so a mesh that is new on every call gets the coarse one (integer_prepare).  Leaf boxes are widened by
+// 4 * 2^-18 of the scene scale; a query takes the grid while its own tolerance (qmax + scene) * 2^-18 stays below
+// 3.5 * 2^-18 of the scene scale (qmax <= 2.5 * scene), which leaves room for the one-ulp difference between the corners
+// and the walk's outward-rounded boxes.
 int build_cells(Context& ctx, const Hier& h, float scene_scale, CellGrid& g, int per_leaf)
 {
     g.valid = false;
@@ -1021,7 +1022,14 @@ int integer_prepare(Context& ctx, const Bvh& bvh, const T* dir_host, int64_t n)
     // latency: a mesh's first call takes it with 32 queries per leaf or more, and any later call on the mesh takes it.
     ++cg.calls;
     int const per_leaf = cg.calls > 1 || n / 32 >= bvh.n_tri ? kCellsFine : kCellsCoarse;
-    if (!cg.valid || cg.per_leaf < per_leaf)
+    if (cg.valid && cg.per_leaf < per_leaf && !cg.pinned)
+    {
+        // a build allocates and synchronises, and a graph that is being captured will read the grid there is
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        AGWN_TRY_CUDA(cudaStreamIsCapturing(ctx.stream, &status));
+        cg.pinned = status != cudaStreamCaptureStatusNone;
+    }
+    if (!cg.valid || (cg.per_leaf < per_leaf && !cg.pinned))
         AGWN_TRY(build_cells(ctx, ctx.ray_cache.h, float(bvh.scene_scale), cg, per_leaf));
     return AGWN_OK;
 }
