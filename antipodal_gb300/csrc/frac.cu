@@ -459,18 +459,18 @@ int mesh_batch_pipelined(Context& ctx, const agwn_bvh* bvh, const T* positions, 
     return ctx.check_flags();
 }
 
-// Device queries and device results of the full GWN: the batch runs in 4 chunks (of 2^20 queries at least) whose
-// kernels alternate between the context's stream and a second compute stream, as the host-array pipeline's do, so
-// that the next chunk's integer and fractional kernels fill the SMs that the end of the current chunk's fractional
-// kernel leaves idle.  Each chunk reads and writes its own slices (queries, counts, results), so no chunk waits for
-// another; the boundary, the hierarchy and its cell grid are prepared once on the context's stream before either
+// Device queries and device results of the full GWN: the batch runs in 4 chunks (of 2^20 queries at least; two halves
+// below 2^21) whose kernels alternate between the context's stream and a second compute stream, as the host-array
+// pipeline's do, so that the next chunk's integer and fractional kernels fill the SMs that the end of the current chunk's
+// fractional kernel leaves idle.  Each chunk reads and writes its own slices (queries, counts, results), so no chunk waits
+// for another; the boundary, the hierarchy and its cell grid are prepared once on the context's stream before either
 // stream starts.  (On 256^3 queries of a 212-segment boundary: 4 chunks 7.18 ms, 8 chunks 7.25, 16 chunks 7.57.)
 template <class T>
 int mesh_batch_chunked(Context& ctx, const agwn_bvh* bvh, const T* dpos, int64_t n, T* dout, const T* x0,
                        const T* dseg, int64_t n_seg)
 {
     AGWN_TRY(ctx.ensure_pipeline());
-    int64_t chunk = std::max<int64_t>(int64_t(1) << 20, (n + 3) / 4);
+    int64_t chunk = n < int64_t(1) << 21 ? (n + 1) / 2 : std::max<int64_t>(int64_t(1) << 20, (n + 3) / 4);
     chunk = (chunk + 1023) / 1024 * 1024;
     bool const with_int = bvh && bvh->n_tri > 0;
     int32_t* dcounts = nullptr;
@@ -584,7 +584,10 @@ int mesh_batch(agwn_context* ctx, const agwn_bvh* bvh, const T* positions, int64
             }
         }
     }
-    if (n >= (int64_t(1) << 21) && want_frac && bvh && bvh->n_tri > 0 && is_device_pointer(positions) &&
+    // From 2^21 queries; in float, whose counts take a good part of a call, from 3 x 2^18 (float, 102 segments, in one
+    // piece against halves: 500,000 queries 202 us against 206, 884,736 342 against 316, 1,815,848 659 against 610; double,
+    // 884,736: 6608 against 6592).
+    if (n >= (sizeof(T) == 4 ? int64_t(3) << 18 : int64_t(1) << 21) && want_frac && bvh && bvh->n_tri > 0 && is_device_pointer(positions) &&
         is_device_pointer(out))
     {
         AGWN_TRY(stage_in(*ctx, boundary, sizeof(T) * 7 * n_seg, S_MISC0, &dseg));
