@@ -201,11 +201,33 @@ int robust_count_chunk(void* user, Context& ctx, const double* d_pos, int64_t m,
     return ctx.launch_end(AGWN_K_ROBUST);
 }
 
-// The evaluator's cell grid, complete on return: other contexts may use the evaluator next.
-int robust_cells(Context& ctx, const Robust& r)
+// Whether the counts take the evaluator's cell grid, building it at the first call.  The build goes into a grid of its
+// own and is waited for before it becomes the evaluator's: another thread's context, on another stream, finds either no
+// grid or a complete one, and a second thread's first call waits here for the first one's build.
+int robust_cells(Context& ctx, const Robust& r, bool* usable)
 {
-    AGWN_TRY(build_cells(ctx, r.hier, float(r.hier.scale), r.cells));
-    AGWN_TRY_CUDA(cudaStreamSynchronize(ctx.stream));
+    *usable = false;
+    if (!ctx.integer_cells || r.n_tri <= 1)
+        return AGWN_OK;
+    std::lock_guard<std::mutex> lock(r.cells_mutex);
+    if (!r.cells.valid)
+    {
+        CellGrid g;
+        int s = build_cells(ctx, r.hier, float(r.hier.scale), g);
+        if (s == AGWN_OK)
+        {
+            cudaError_t const e = cudaStreamSynchronize(ctx.stream);
+            if (e != cudaSuccess)
+                s = fail(AGWN_ERR_CUDA, "cell grid build: %s", cudaGetErrorString(e));
+        }
+        if (s != AGWN_OK || !g.valid)
+        {
+            g.release();
+            return s;
+        }
+        r.cells = g;
+    }
+    *usable = true;
     return AGWN_OK;
 }
 
@@ -224,9 +246,9 @@ int robust_run(Context& ctx, const Robust& r, const T* d_pos, int64_t n, T* d_ou
             ctx.robust_mode == AGWN_ROBUST_MIXED && r.n_seg > 0 && r.n_seg < (int64_t(1) << 24) &&
             ctx.use_mixed(double(n) * double(r.n_seg), r.n_seg))
         {
-            if (!r.cells.valid)
-                AGWN_TRY(robust_cells(ctx, r));
-            if (r.cells.valid)
+            bool cells = false;
+            AGWN_TRY(robust_cells(ctx, r, &cells));
+            if (cells)
             {
                 double* raw = nullptr;
                 AGWN_TRY(ctx.scratch_reserve(S_MISC2, sizeof(double) * 7 * size_t(r.n_seg),
@@ -253,9 +275,9 @@ int robust_run(Context& ctx, const Robust& r, const T* d_pos, int64_t n, T* d_ou
         for (int k = 0; k < 9; ++k)
             f.r[k] = r.hier.frame[k];
         int const grid = int(std::min<int64_t>(div_up(n, kRobBlock), int64_t(ctx.sm_count) * 16));
-        if (ctx.integer_cells && r.n_tri > 1 && !r.cells.valid)
-            AGWN_TRY(robust_cells(ctx, r));
-        if (ctx.integer_cells && r.n_tri > 1 && r.cells.valid)
+        bool cells = false;
+        AGWN_TRY(robust_cells(ctx, r, &cells));
+        if (cells)
         {
             AGWN_TRY(ctx.launch_begin(AGWN_K_ROBUST));
             k_robust_cells<T, P><<<grid, kRobBlock, 0, st>>>(

@@ -4,6 +4,8 @@
 
 #include "agwn_internal.cuh"
 
+#include <mutex>
+
 namespace agwn
 {
 // The int64_grid boundary as vertex chains for the FP32 pairs (k_robust_chain, robust.cuh): per chain a start
@@ -31,7 +33,10 @@ struct Robust
     void* chain = nullptr; // int64_grid: the segments as vertex chains (RChain) for the FP32 pairs
     int64_t n_entries = 0;
     Hier hier;
-    mutable CellGrid cells; // the integer term's cell grid over hier, built on first use
+    // The integer term's cell grid over hier, built on first use.  Contexts on several threads may share the evaluator:
+    // it is built and published under the mutex, complete on the device, and never changes after (robust_cells).
+    mutable CellGrid cells;
+    mutable std::mutex cells_mutex;
 };
 } // namespace agwn
 
