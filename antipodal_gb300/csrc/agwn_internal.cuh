@@ -169,6 +169,7 @@ struct Context
     int sm_count = 0;
     RayCache ray_cache;
     DevBuf bernstein; // the exact parametric integrator's node bases (param.cu), filled on first use
+    bool bernstein_filled = false;
     // host-array pipeline (mesh batch): upload and download streams and their events, created on first use
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
     cudaStream_t compute2 = nullptr; // the host-array pipeline runs alternate chunks' kernels here

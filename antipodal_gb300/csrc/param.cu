@@ -793,12 +793,16 @@ int param_run_exact(Context& ctx, const double* d_pos, int64_t n, double* d_out,
                     int64_t n_curves, int min_depth, int max_depth, double tol, const uint8_t* d_start,
                     uint32_t* d_stats, int32_t* d_nodes, ParamExtras const& ex)
 {
-    if (!ctx.bernstein.ptr)
+    if (!ctx.bernstein_filled)
     {
         AGWN_TRY(ctx.bernstein.reserve(sizeof(double2) * 4 * kTeam * kBernPanels));
         AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
         k_bernstein<<<div_up(kBernPanels * kTeam, 256), 256, 0, ctx.stream>>>(static_cast<double2*>(ctx.bernstein.ptr));
         AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
+        // a launch that is being captured fills the table when the graph runs, not now
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        AGWN_TRY_CUDA(cudaStreamIsCapturing(ctx.stream, &status));
+        ctx.bernstein_filled = status == cudaStreamCaptureStatusNone;
     }
     int per_sm = 0;
     AGWN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_param_exact, kParamBlock, 0));
