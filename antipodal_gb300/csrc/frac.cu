@@ -271,25 +271,34 @@ int fractional_launch_mixed(Context& ctx, const FracPlan<T>& p, const double* d_
     // (34.9 ms against 40.5 on 1,066 segments), since more queries share each staged tile and its barriers
     int const block = ctx.frac_block ? ctx.frac_block : (p.nbuf > 1 || p.tile > 512 ? 256 : 128);
     int64_t const n_qtiles = (n + int64_t(block) * K - 1) / (int64_t(block) * K);
-    auto launch = [&](auto kern, size_t smem) -> int
+    // Two buffers of the largest tiles, their groups and the queues of 8 queries per thread in blocks of 256 exceed an
+    // SM's 227 KB from 1,984 entries: the tile is cut to what fits (the values do not depend on it).
+    int tile = p.tile;
+    auto const smem_of = [&] { return K == 2   ? mixed_smem<2>(p.nbuf, tile, block)
+                                      : K == 4 ? mixed_smem<4>(p.nbuf, tile, block)
+                                               : mixed_smem<8>(p.nbuf, tile, block); };
+    constexpr size_t kMixedStatic = 256; // the kernel's static shared memory, rounded up
+    while (tile > 32 && smem_of() > size_t(227) * 1024 - kMixedStatic)
+        tile -= 32;
+    size_t const smem = smem_of();
+    auto launch = [&](auto kern) -> int
     {
         int grid = 0;
         AGWN_TRY(launch_persistent(ctx, kern, block, smem, n_qtiles, &grid));
         AGWN_TRY(ctx.launch_begin(AGWN_K_FRACTIONAL));
         kern<<<grid, block, smem, ctx.stream>>>(d_pos, n, d_out, d_counts, p.x0d[0], p.x0d[1], p.x0d[2], p.rot,
                                                 p.frame, int(ctx.mixed_certify), float(ctx.mixed_term_err), p.segm, fb,
-                                                p.n_seg, p.tile,
-                                                ctx.d_flags, ctx.d_counters, ctx.timing);
+                                                p.n_seg, tile, ctx.d_flags, ctx.d_counters, ctx.timing);
         return ctx.launch_end(AGWN_K_FRACTIONAL);
     };
     switch (K)
     {
     case 2:
-        return launch(k_frac_mixed<2, FB>, mixed_smem<2>(p.nbuf, p.tile, block));
+        return launch(k_frac_mixed<2, FB>);
     case 4:
-        return launch(k_frac_mixed<4, FB>, mixed_smem<4>(p.nbuf, p.tile, block));
+        return launch(k_frac_mixed<4, FB>);
     default:
-        return launch(k_frac_mixed<8, FB>, mixed_smem<8>(p.nbuf, p.tile, block));
+        return launch(k_frac_mixed<8, FB>);
     }
 }
 
