@@ -21,7 +21,7 @@ STATUS = {0: "ok", 1: "invalid argument", 2: "CUDA runtime error", 3: "out of de
 
 OPT_FRAC_MODE, OPT_MIXED_TAU, OPT_QUERIES_PER_THREAD, OPT_FRAC_BLOCK, OPT_TIMING, OPT_SEG_TILE, \
     OPT_MIXED_TERM_ERR, OPT_ROBUST_MODE, OPT_ROBUST_TERM_ERR, OPT_PARAM_MODE, OPT_INTEGER_CELLS, \
-    OPT_MIXED_MIN_PAIRS, OPT_MIXED_CERTIFY = range(13)
+    OPT_MIXED_MIN_PAIRS, OPT_MIXED_CERTIFY, OPT_SCRATCH_LIMIT = range(14)
 ROBUST_EXACT, ROBUST_MIXED = 0, 1
 PARAM_EXACT, PARAM_MIXED = 0, 1
 FRAC_EXACT, FRAC_MIXED = 0, 1

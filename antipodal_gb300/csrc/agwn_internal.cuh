@@ -60,7 +60,8 @@ struct DevBuf
 {
     void* ptr = nullptr;
     size_t cap = 0;
-    int reserve(size_t bytes);
+    // Room for `bytes`, with a quarter more while that stays within `most` and there is memory for it.
+    int reserve(size_t bytes, size_t most = SIZE_MAX);
     void release();
 };
 
@@ -93,7 +94,7 @@ enum scratch_slot
     S_MISC1 = 7,
     S_MISC2 = 8,
     S_MISC3 = 9,
-    S_PARTIAL = 10, // the parametric integrator's per-group partial sums; the split exact kernel's terms
+    S_PARTIAL = 10, // the split exact kernels' terms; the parametric integrator's pair counter
     S_ORDER0 = 11,  // the spatial order of the queries: sort keys, indices, digit counters (order.cu)
     S_ORDER1 = 12,  // the queries in that order and their outputs
     S_COUNT = 13
@@ -201,6 +202,7 @@ struct Context
     int frac_block = 0; // 0: chosen per launch (frac.cu)
     int seg_tile = 512;
     int timing = 0;
+    size_t scratch_limit = SIZE_MAX; // the largest scratch buffer of a call
 
     // statistics
     double kernel_ms[AGWN_K_COUNT] = {};
@@ -225,6 +227,8 @@ struct Context
     }
 
     int scratch_reserve(int slot, size_t bytes, void** out);
+    // scratch_reserve of fixed + unit * *units bytes; *units is halved, down to 1, while there is no memory for them
+    int scratch_reserve_units(int slot, size_t fixed, size_t unit, int64_t* units, void** out);
     // Brackets a launch with timing events when AGWN_OPT_TIMING is on; always counts the launch.
     int launch_begin(int kclass);
     int launch_end(int kclass);

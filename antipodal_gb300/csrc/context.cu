@@ -34,13 +34,19 @@ void clear_message()
     g_message[0] = 0;
 }
 
-int DevBuf::reserve(size_t bytes)
+int DevBuf::reserve(size_t bytes, size_t most)
 {
     if (bytes <= cap)
         return AGWN_OK;
     release();
-    size_t const want = bytes + bytes / 4 + 256;
-    cudaError_t const e = cudaMalloc(&ptr, want);
+    size_t want = std::max(bytes, std::min(bytes + bytes / 4 + 256, most));
+    cudaError_t e = cudaMalloc(&ptr, want);
+    if (e == cudaErrorMemoryAllocation && want > bytes)
+    {
+        cudaGetLastError();
+        want = bytes;
+        e = cudaMalloc(&ptr, want);
+    }
     if (e != cudaSuccess)
     {
         cudaGetLastError();
@@ -131,11 +137,25 @@ int Context::scratch_reserve(int slot, size_t bytes, void** out)
 {
     // Scratch is shared by calls on this context's stream; a growing reallocation must not free memory that
     // queued work may still read.
+    if (bytes > scratch_limit)
+        return fail(AGWN_ERR_NOMEM, "%zu bytes of scratch exceed the context's limit of %zu", bytes, scratch_limit);
     if (bytes > scratch[slot].cap)
         AGWN_TRY_CUDA(cudaStreamSynchronize(stream));
-    AGWN_TRY(scratch[slot].reserve(bytes == 0 ? 1 : bytes));
+    AGWN_TRY(scratch[slot].reserve(bytes == 0 ? 1 : bytes, scratch_limit));
     *out = scratch[slot].ptr;
     return AGWN_OK;
+}
+
+int Context::scratch_reserve_units(int slot, size_t fixed, size_t unit, int64_t* units, void** out)
+{
+    for (;;)
+    {
+        int const s = scratch_reserve(slot, fixed + unit * size_t(*units), out);
+        if (s != AGWN_ERR_NOMEM || *units <= 1)
+            return s;
+        clear_message();
+        *units /= 2;
+    }
 }
 
 int Context::launch_begin(int kclass)
@@ -449,6 +469,10 @@ int agwn_context_set_option(agwn_context* ctx, int option, double value)
         AGWN_CHECK_ARG(value == 0 || value == 1, "mixed certify must be 0 or 1");
         ctx->mixed_certify = value != 0.0;
         return AGWN_OK;
+    case AGWN_OPT_SCRATCH_LIMIT:
+        AGWN_CHECK_ARG(value >= 0.0 && value <= 1e15, "scratch limit must be 0 (none) or a number of bytes");
+        ctx->scratch_limit = value == 0.0 ? SIZE_MAX : size_t(value);
+        return AGWN_OK;
     default:
         return fail(AGWN_ERR_INVALID, "unknown option %d", option);
     }
@@ -497,6 +521,9 @@ int agwn_context_get_option(agwn_context* ctx, int option, double* value)
         return AGWN_OK;
     case AGWN_OPT_MIXED_CERTIFY:
         *value = ctx->mixed_certify ? 1.0 : 0.0;
+        return AGWN_OK;
+    case AGWN_OPT_SCRATCH_LIMIT:
+        *value = ctx->scratch_limit == SIZE_MAX ? 0.0 : double(ctx->scratch_limit);
         return AGWN_OK;
     default:
         return fail(AGWN_ERR_INVALID, "unknown option %d", option);

@@ -181,14 +181,14 @@ int fractional_launch_mixed(Context& ctx, const FracPlan<T>& p, const double* d_
                             const int32_t* d_counts, FB fb);
 
 // The exact form shared out by segment: units of g segments so that there are 16 warps per SM or more, in passes over
-// the boundary of at most 64 MB of terms.
+// the boundary of at most 64 MB of terms (fewer where there is no memory for them).
 template <class T>
 int fractional_split(Context& ctx, const FracPlan<T>& p, const T* d_pos, int64_t n, T* d_out, const int32_t* d_counts)
 {
     int64_t const groups = div_up(n, 32);
-    int64_t const pass = std::min<int64_t>(p.n_seg, std::max<int64_t>(1, (int64_t(1) << 26) / (n * int64_t(sizeof(T)))));
+    int64_t pass = std::min<int64_t>(p.n_seg, std::max<int64_t>(1, (int64_t(1) << 26) / (n * int64_t(sizeof(T)))));
     T* terms = nullptr;
-    AGWN_TRY(ctx.scratch_reserve(S_PARTIAL, sizeof(T) * size_t(pass) * size_t(n), reinterpret_cast<void**>(&terms)));
+    AGWN_TRY(ctx.scratch_reserve_units(S_PARTIAL, 0, sizeof(T) * size_t(n), &pass, reinterpret_cast<void**>(&terms)));
     for (int64_t s0 = 0; s0 < p.n_seg; s0 += pass)
     {
         int const ns = int(std::min(pass, p.n_seg - s0));

@@ -535,7 +535,8 @@ __global__ void k_param_sum(const double* __restrict__ vals, int nq, int nc, boo
     out[i] = last ? (sum / (rd(4.0) * rd(3.141592653589793238462643383279502884))).v : sum.v;
 }
 
-// Pair integrals in the double-float form: vals[k * nq + i] for the curves c0 + k and the queries q0 + i.
+// Pair integrals in the double-float form: vals[k * nq + i] for the curves c0 + k and the queries q0 + i (pos: these
+// queries' coordinates).
 //
 // The FMA pipe's chains bound it (a lane per pair: some 320 dependent FP32 operations a node, 15 nodes a panel).  The
 // cost of one (query, curve) integral is heavy-tailed, so the lanes of the whole grid draw their pairs from one counter
@@ -617,7 +618,7 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>())
                     k = mine / nq;
                     ql = mine - k * nq;
                     int64_t const q = q0 + ql;
-                    df const pd[3] = {pos[3 * q], pos[3 * q + 1], pos[3 * q + 2]};
+                    df const pd[3] = {pos[3 * ql], pos[3 * ql + 1], pos[3 * ql + 2]};
                     CurveDF const& cv = curves[c0 + k];
 #pragma unroll
                     for (int e = 0; e < 12; ++e)
@@ -760,17 +761,35 @@ __global__ void __launch_bounds__(kParamBlock, param_min_blocks<PANEL>())
 }
 
 // The pair integrals and their sums over chunks of at most `most` pairs: queries first, and curves where one query has
-// more.  launch(q0, nq, c0, nc, vals, next) integrates a chunk's pairs.
-template <class Launch>
-int param_chunks(Context& ctx, int64_t n, int64_t n_curves, int64_t most, double* d_out, int32_t* d_nodes, Launch launch)
+// more.  launch(q0, nq, c0, nc, vals, next) integrates a chunk's pairs.  reserve(nq) takes what else a chunk of nq queries
+// needs.  Where there is no memory for a chunk, it is halved until there is.
+template <class Reserve, class Launch>
+int param_chunks(Context& ctx, int64_t n, int64_t n_curves, int64_t most, double* d_out, int32_t* d_nodes,
+                 Reserve reserve, Launch launch)
 {
-    int64_t const nc_max = std::min(n_curves, most);
-    int64_t const nq_max = std::min(n, std::max<int64_t>(1, most / nc_max));
+    int64_t nc_max = 0, nq_max = 0;
     double* vals = nullptr;
     int* next = nullptr;
-    AGWN_TRY(ctx.scratch_reserve(S_SEGS_RAW, sizeof(double) * size_t(nc_max) * size_t(nq_max),
-                                 reinterpret_cast<void**>(&vals)));
     AGWN_TRY(ctx.scratch_reserve(S_PARTIAL, sizeof(int), reinterpret_cast<void**>(&next)));
+    most = std::min<int64_t>(most, n > most / n_curves ? most : n * n_curves);
+    for (;; most /= 2)
+    {
+        nc_max = std::min(n_curves, most);
+        nq_max = std::min(n, std::max<int64_t>(1, most / nc_max));
+        int s = ctx.scratch_reserve(S_SEGS_RAW, sizeof(double) * size_t(nc_max) * size_t(nq_max),
+                                    reinterpret_cast<void**>(&vals));
+        if (s == AGWN_OK)
+            s = reserve(nq_max);
+        if (s == AGWN_OK)
+            break;
+        if (s != AGWN_ERR_NOMEM || most == 1)
+            return s;
+        // the larger buffers of this attempt or an earlier call make room
+        clear_message();
+        AGWN_TRY_CUDA(cudaStreamSynchronize(ctx.stream));
+        ctx.scratch[S_SEGS_RAW].release();
+        ctx.scratch[S_FRAME].release();
+    }
     if (d_nodes)
         AGWN_TRY_CUDA(cudaMemsetAsync(d_nodes, 0, sizeof(int32_t) * n, ctx.stream));
     for (int64_t q0 = 0; q0 < n; q0 += nq_max)
@@ -778,9 +797,7 @@ int param_chunks(Context& ctx, int64_t n, int64_t n_curves, int64_t most, double
         {
             int const nq = int(std::min(nq_max, n - q0)), nc = int(std::min(nc_max, n_curves - c0));
             AGWN_TRY_CUDA(cudaMemsetAsync(next, 0, sizeof(int), ctx.stream));
-            AGWN_TRY(ctx.launch_begin(AGWN_K_PARAMETRIC));
-            launch(q0, nq, c0, nc, vals, next);
-            AGWN_TRY(ctx.launch_end(AGWN_K_PARAMETRIC));
+            AGWN_TRY(launch(q0, nq, c0, nc, vals, next));
             AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
             k_param_sum<<<div_up(nq, 64), 64, 0, ctx.stream>>>(vals, nq, nc, c0 == 0, c0 + nc == n_curves, d_out + q0);
             AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
@@ -808,15 +825,17 @@ int param_run_exact(Context& ctx, const double* d_pos, int64_t n, double* d_out,
     AGWN_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_param_exact, kParamBlock, 0));
     int64_t const full = int64_t(std::max(per_sm, 1)) * ctx.sm_count;
     ev3<rd> const x0v{rd(x0[0]), rd(x0[1]), rd(x0[2])};
-    return param_chunks(ctx, n, n_curves, int64_t(1) << 25, d_out, d_nodes,
-                        [&](int64_t q0, int nq, int64_t c0, int nc, double* vals, int* next)
-                        {
-                            int const grid =
-                                int(std::min<int64_t>(div_up(int64_t(nq) * nc, kParamBlock / kTeam), full));
-                            k_param_exact<<<grid, kParamBlock, 0, ctx.stream>>>(
-                                d_pos, q0, nq, x0v, d_curves, n_curves, c0, nc, min_depth, max_depth, tol, d_start,
-                                d_stats, d_nodes, vals, next, static_cast<const double2*>(ctx.bernstein.ptr), ex);
-                        });
+    return param_chunks(
+        ctx, n, n_curves, int64_t(1) << 25, d_out, d_nodes, [](int64_t) { return int(AGWN_OK); },
+        [&](int64_t q0, int nq, int64_t c0, int nc, double* vals, int* next) -> int
+        {
+            int const grid = int(std::min<int64_t>(div_up(int64_t(nq) * nc, kParamBlock / kTeam), full));
+            AGWN_TRY(ctx.launch_begin(AGWN_K_PARAMETRIC));
+            k_param_exact<<<grid, kParamBlock, 0, ctx.stream>>>(d_pos, q0, nq, x0v, d_curves, n_curves, c0, nc, min_depth,
+                                                               max_depth, tol, d_start, d_stats, d_nodes, vals, next,
+                                                               static_cast<const double2*>(ctx.bernstein.ptr), ex);
+            return ctx.launch_end(AGWN_K_PARAMETRIC);
+        });
 }
 } // namespace
 
@@ -872,28 +891,43 @@ int param_run(Context& ctx, const double* d_pos, int64_t n, double* d_out, const
         F.scale = split((n2 - 2.0) * n2);
         F.unit = std::fabs(n2 - 1.0) <= 1e-15;
     }
+    // the curves, then a chunk's queries
     CurveDF* cdf = nullptr;
-    AGWN_TRY(ctx.scratch_reserve(S_FRAME, sizeof(CurveDF) * size_t(n_curves) + sizeof(df) * 3 * size_t(n),
-                                 reinterpret_cast<void**>(&cdf)));
-    df* const qdf = reinterpret_cast<df*>(cdf + n_curves);
-    AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-    k_curves_df<<<int(std::min<int64_t>(div_up(3 * n_curves, 256), 4 * ctx.sm_count)), 256, 0, ctx.stream>>>(
-        d_curves, n_curves, F, cdf);
-    AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
-    AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-    k_queries_df<<<int(std::min<int64_t>(div_up(n, 256), 4 * ctx.sm_count)), 256, 0, ctx.stream>>>(d_pos, n, F, qdf);
-    AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
+    auto const reserve = [&](int64_t nq)
+    {
+        return ctx.scratch_reserve(S_FRAME, sizeof(CurveDF) * size_t(n_curves) + sizeof(df) * 3 * size_t(nq),
+                                   reinterpret_cast<void**>(&cdf));
+    };
+    bool curves_done = false;
     // 2^26 pairs (537 MB of integrals) at a time: a chunk ends with its deepest pairs, half a millisecond or so
-    return param_chunks(ctx, n, n_curves, int64_t(1) << 26, d_out, d_nodes,
-                        [&](int64_t q0, int nq, int64_t c0, int nc, double* vals, int* next)
-                        {
-                            int64_t const pairs = int64_t(nq) * nc;
-                            int const grid = int(std::min<int64_t>(div_up(pairs, kParamBlock), full));
-                            int const take = pairs >= 8 * full * kParamBlock ? 64 : 32;
-                            kern<<<grid, kParamBlock, smem, ctx.stream>>>(qdf, q0, nq, F, cdf, n_curves, c0, nc,
-                                                                         min_depth, max_depth, tol, d_start, d_stats,
-                                                                         d_nodes, vals, next, take, ex);
-                        });
+    return param_chunks(
+        ctx, n, n_curves, int64_t(1) << 26, d_out, d_nodes, reserve,
+        [&](int64_t q0, int nq, int64_t c0, int nc, double* vals, int* next) -> int
+        {
+            df* const qdf = reinterpret_cast<df*>(cdf + n_curves);
+            if (!curves_done)
+            {
+                AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
+                k_curves_df<<<int(std::min<int64_t>(div_up(3 * n_curves, 256), 4 * ctx.sm_count)), 256, 0, ctx.stream>>>(
+                    d_curves, n_curves, F, cdf);
+                AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
+                curves_done = true;
+            }
+            if (c0 == 0)
+            {
+                AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
+                k_queries_df<<<int(std::min<int64_t>(div_up(nq, 256), 4 * ctx.sm_count)), 256, 0, ctx.stream>>>(
+                    d_pos + 3 * q0, nq, F, qdf);
+                AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
+            }
+            int64_t const pairs = int64_t(nq) * nc;
+            int const grid = int(std::min<int64_t>(div_up(pairs, kParamBlock), full));
+            int const take = pairs >= 8 * full * kParamBlock ? 64 : 32;
+            AGWN_TRY(ctx.launch_begin(AGWN_K_PARAMETRIC));
+            kern<<<grid, kParamBlock, smem, ctx.stream>>>(qdf, q0, nq, F, cdf, n_curves, c0, nc, min_depth, max_depth, tol,
+                                                         d_start, d_stats, d_nodes, vals, next, take, ex);
+            return ctx.launch_end(AGWN_K_PARAMETRIC);
+        });
 }
 } // namespace agwn
 

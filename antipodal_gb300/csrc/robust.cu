@@ -326,10 +326,10 @@ int robust_run(Context& ctx, const Robust& r, const T* d_pos, int64_t n, T* d_ou
         // fewer than 8 warps of queries per SM: shared out by segment, in units that give 16 warps per SM or more and
         // passes of at most 64 MB of terms (as the mesh functions' exact form, frac.cu)
         int64_t const groups = div_up(n, 32);
-        int64_t const pass = std::min<int64_t>(r.n_seg, std::max<int64_t>(1, (int64_t(1) << 26) / (n * 8)));
-        double* terms = nullptr;
-        AGWN_TRY(ctx.scratch_reserve(S_PARTIAL, sizeof(double) * size_t(pass + 1) * size_t(n),
-                                     reinterpret_cast<void**>(&terms)));
+        int64_t pass = std::min<int64_t>(r.n_seg, std::max<int64_t>(1, (int64_t(1) << 26) / (n * 8)));
+        double* terms = nullptr; // pass x n, then the running sums
+        size_t const row = sizeof(double) * size_t(n);
+        AGWN_TRY(ctx.scratch_reserve_units(S_PARTIAL, row, row, &pass, reinterpret_cast<void**>(&terms)));
         for (int64_t s0 = 0; s0 < r.n_seg; s0 += pass)
         {
             int const ns = int(std::min(pass, r.n_seg - s0));
