@@ -78,6 +78,7 @@ struct Arena
     };
     std::vector<Chunk> chunks;
     int depth = 0;
+    size_t limit = SIZE_MAX; // of all chunks together
     int take(size_t bytes, void** out);
     void release();
 };

@@ -45,7 +45,7 @@ __global__ void k_edge_keys(const int32_t* __restrict__ idx, int64_t n_tri, int6
 
 constexpr unsigned kBinMax = 512;
 
-// state[0]: an out-of-range index; state[1]: a bin above kBinMax; state[2]: the number of emitted edges.
+// state[0]: an out-of-range index; state[1]: a bin above kBinMax.
 // rank[i]: edge i's place in its lower vertex's bin (0xffffffff for an invalid edge).
 __global__ void k_edge_count(const int32_t* __restrict__ idx, int64_t n_tri, int64_t nv, unsigned* __restrict__ bins,
                              unsigned* __restrict__ rank, unsigned* __restrict__ state)
@@ -309,6 +309,52 @@ int boundary_radix(Context& ctx, const T* dv, int64_t nv, const int32_t* di, int
     return ctx.launch_end(AGWN_K_OTHER);
 }
 
+// The extraction by bins: *n_segments and the first `rows` rows into d_out, both set by rows_for(*n_segments); or *radix
+// and nothing else where a bin is above kBinMax.  Its buffers are given back before the radix sort takes its own.
+template <class T, class RowsFor>
+int boundary_bins(Context& ctx, const T* dv, int64_t nv, const int32_t* di, int64_t m, RowsFor rows_for, T* const& d_out,
+                  int64_t const& rows, int64_t* n_segments, bool* radix)
+{
+    cudaStream_t const st = ctx.stream;
+    ArenaScope scope(ctx);
+    Tmp bins(ctx), sums(ctx), rank(ctx), lo(ctx), hi(ctx), net(ctx);
+    // one counter per vertex and its end for the bins, the same for the emitted edges, and the state
+    size_t const n_cnt = size_t(nv) + 1;
+    AGWN_TRY(bins.alloc(sizeof(unsigned) * (2 * n_cnt + 2)));
+    AGWN_TRY(sums.alloc(sizeof(unsigned) * size_t(scan_sums_count(int64_t(n_cnt)))));
+    AGWN_TRY(rank.alloc(sizeof(unsigned) * m));
+    AGWN_TRY(lo.alloc(sizeof(int) * m));
+    AGWN_TRY(hi.alloc(sizeof(unsigned) * m));
+    AGWN_TRY(net.alloc(sizeof(int) * m));
+    unsigned* const bin = bins.as<unsigned>();
+    unsigned* const emitted = bin + n_cnt;
+    unsigned* const state = emitted + n_cnt;
+    int const grid = int(std::min<int64_t>(div_up(m, 256), 8 * ctx.sm_count));
+    AGWN_TRY_CUDA(cudaMemsetAsync(bin, 0, sizeof(unsigned) * (2 * n_cnt + 2), st));
+    AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
+    k_edge_count<<<grid, 256, 0, st>>>(di, m / 3, nv, bin, rank.as<unsigned>(), state);
+    scan_counters(st, bin, int64_t(n_cnt), sums.as<unsigned>());
+    k_edge_place<<<grid, 256, 0, st>>>(di, m / 3, bin, rank.as<unsigned>(), lo.as<int>(), hi.as<unsigned>());
+    k_edge_net<<<grid, 256, 0, st>>>(lo.as<int>(), hi.as<unsigned>(), m, bin, state, net.as<int>(), emitted);
+    scan_counters(st, emitted, int64_t(n_cnt), sums.as<unsigned>()); // its last counter: all emitted edges
+    AGWN_TRY(ctx.launch_end(AGWN_K_OTHER));
+    unsigned back[3] = {}; // the last counter and the state
+    AGWN_TRY_CUDA(cudaMemcpyAsync(back, emitted + nv, sizeof(back), cudaMemcpyDeviceToHost, st));
+    AGWN_TRY_CUDA(cudaStreamSynchronize(st));
+    if (back[1])
+        return fail(AGWN_ERR_INVALID, "triangle index out of range [0, %lld)", (long long)nv);
+    *radix = back[2] != 0;
+    if (*radix)
+        return AGWN_OK;
+    *n_segments = back[0];
+    AGWN_TRY(rows_for(int64_t(back[0])));
+    if (rows == 0)
+        return AGWN_OK;
+    AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
+    k_edge_rows<T><<<grid, 256, 0, st>>>(lo.as<int>(), hi.as<unsigned>(), m, bin, net.as<int>(), emitted, dv, rows, d_out);
+    return ctx.launch_end(AGWN_K_OTHER);
+}
+
 template <class T>
 int boundary_build(agwn_context* ctx, const T* vertices, int64_t nv, const int32_t* indices, int64_t n_idx, T* out,
                    int64_t capacity, int64_t* n_segments)
@@ -323,68 +369,40 @@ int boundary_build(agwn_context* ctx, const T* vertices, int64_t nv, const int32
     int64_t const m = n_idx; // one entry per triangle edge
     if (m == 0)
         return AGWN_OK;
-    cudaStream_t const st = ctx->stream;
     const void *dv = nullptr, *di = nullptr;
     AGWN_TRY(stage_in(*ctx, vertices, sizeof(T) * 3 * nv, S_MISC0, &dv));
     AGWN_TRY(stage_in(*ctx, indices, sizeof(int32_t) * n_idx, S_MISC1, &di));
-    ArenaScope scope(*ctx);
-    Tmp bins(*ctx), sums(*ctx), rank(*ctx), lo(*ctx), hi(*ctx), net(*ctx);
-    // one counter per vertex and its end for the bins, the same for the emitted edges, and the state
-    bool const sparse = nv > 16 * m + 65536;
-    size_t const n_cnt = sparse ? 1 : size_t(nv) + 1;
-    AGWN_TRY(bins.alloc(sizeof(unsigned) * (2 * n_cnt + 3)));
-    AGWN_TRY(sums.alloc(sizeof(unsigned) * size_t(scan_sums_count(int64_t(n_cnt)))));
-    AGWN_TRY(rank.alloc(sizeof(unsigned) * m));
-    AGWN_TRY(lo.alloc(sizeof(int) * m));
-    AGWN_TRY(hi.alloc(sizeof(unsigned) * m));
-    AGWN_TRY(net.alloc(sizeof(int) * m));
-    unsigned* const bin = bins.as<unsigned>();
-    unsigned* const emitted = bin + n_cnt;
-    unsigned* const state = emitted + n_cnt;
-    int const grid = int(std::min<int64_t>(div_up(m, 256), 8 * ctx->sm_count));
+    const T* const verts = static_cast<const T*>(dv);
     const int32_t* const ip = static_cast<const int32_t*>(di);
-    unsigned back[4] = {};
-    if (!sparse)
-    {
-        AGWN_TRY_CUDA(cudaMemsetAsync(bin, 0, sizeof(unsigned) * (2 * n_cnt + 3), st));
-        AGWN_TRY(ctx->launch_begin(AGWN_K_OTHER));
-        k_edge_count<<<grid, 256, 0, st>>>(ip, m / 3, nv, bin, rank.as<unsigned>(), state);
-        scan_counters(st, bin, int64_t(n_cnt), sums.as<unsigned>());
-        k_edge_place<<<grid, 256, 0, st>>>(ip, m / 3, bin, rank.as<unsigned>(), lo.as<int>(), hi.as<unsigned>());
-        k_edge_net<<<grid, 256, 0, st>>>(lo.as<int>(), hi.as<unsigned>(), m, bin, state, net.as<int>(), emitted);
-        scan_counters(st, emitted, int64_t(n_cnt), sums.as<unsigned>()); // its last counter: all emitted edges
-        AGWN_TRY(ctx->launch_end(AGWN_K_OTHER));
-        AGWN_TRY_CUDA(cudaMemcpyAsync(back, emitted + nv, sizeof(back), cudaMemcpyDeviceToHost, st));
-        AGWN_TRY_CUDA(cudaStreamSynchronize(st));
-        if (back[1])
-            return fail(AGWN_ERR_INVALID, "triangle index out of range [0, %lld)", (long long)nv);
-    }
-    bool const radix = sparse || back[2] != 0;
-    int64_t count = back[0];
     bool const host_out = out && !is_device_pointer(out);
-    int64_t rows = out ? std::min(capacity, radix ? m : count) : 0;
     T* d_out = out;
-    if (host_out && rows > 0)
+    int64_t count = 0, rows = 0;
+    // where `count` rows go on the device, at most the capacity
+    auto const rows_for = [&](int64_t most) -> int
     {
-        void* p = nullptr;
-        AGWN_TRY(ctx->scratch_reserve(S_MISC2, sizeof(T) * 7 * size_t(rows), &p));
-        d_out = static_cast<T*>(p);
-    }
+        rows = out ? std::min(capacity, most) : 0;
+        if (host_out && rows > 0)
+        {
+            void* p = nullptr;
+            AGWN_TRY(ctx->scratch_reserve(S_MISC2, sizeof(T) * 7 * size_t(rows), &p));
+            d_out = static_cast<T*>(p);
+        }
+        return AGWN_OK;
+    };
+    bool radix = nv > 16 * m + 65536;
+    if (!radix)
+        AGWN_TRY(boundary_bins<T>(*ctx, verts, nv, ip, m, rows_for, d_out, rows, &count, &radix));
     if (radix)
-        AGWN_TRY(boundary_radix<T>(*ctx, static_cast<const T*>(dv), nv, ip, m, d_out, rows, &count));
-    else if (rows > 0)
     {
-        AGWN_TRY(ctx->launch_begin(AGWN_K_OTHER));
-        k_edge_rows<T><<<grid, 256, 0, st>>>(lo.as<int>(), hi.as<unsigned>(), m, bin, net.as<int>(), emitted,
-                                             static_cast<const T*>(dv), rows, d_out);
-        AGWN_TRY(ctx->launch_end(AGWN_K_OTHER));
+        AGWN_TRY(rows_for(m));
+        AGWN_TRY(boundary_radix<T>(*ctx, verts, nv, ip, m, d_out, rows, &count));
     }
     *n_segments = count;
     rows = std::min(rows, count);
     if (rows == 0)
         return AGWN_OK;
     if (host_out)
-        AGWN_TRY_CUDA(cudaMemcpyAsync(out, d_out, sizeof(T) * 7 * size_t(rows), cudaMemcpyDeviceToHost, st));
+        AGWN_TRY_CUDA(cudaMemcpyAsync(out, d_out, sizeof(T) * 7 * size_t(rows), cudaMemcpyDeviceToHost, ctx->stream));
     return ctx->check_flags();
 }
 } // namespace

@@ -75,7 +75,11 @@ int Arena::take(size_t bytes, void** out)
         size_t total = 0;
         for (Chunk const& c : chunks)
             total += c.cap;
-        Chunk c{nullptr, std::max<size_t>({bytes, total, size_t(1) << 18}), 0};
+        size_t const room = limit - std::min(limit, total);
+        if (bytes > room)
+            return fail(AGWN_ERR_NOMEM, "%zu bytes of build temporaries beside %zu exceed the context's limit of %zu", bytes,
+                        total, limit);
+        Chunk c{nullptr, std::min(room, std::max<size_t>({bytes, total, size_t(1) << 18})), 0};
         cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&c.ptr), c.cap);
         if (e == cudaErrorMemoryAllocation && c.cap > bytes)
         {
@@ -472,6 +476,7 @@ int agwn_context_set_option(agwn_context* ctx, int option, double value)
     case AGWN_OPT_SCRATCH_LIMIT:
         AGWN_CHECK_ARG(value >= 0.0 && value <= 1e15, "scratch limit must be 0 (none) or a number of bytes");
         ctx->scratch_limit = value == 0.0 ? SIZE_MAX : size_t(value);
+        ctx->arena.limit = ctx->scratch_limit;
         return AGWN_OK;
     default:
         return fail(AGWN_ERR_INVALID, "unknown option %d", option);

@@ -112,9 +112,10 @@ enum agwn_option
        across the ray for its error bound to pass and its angle to lie in the first octant) without the per-pair
        bound and octant unfolding; 0 takes the per-pair path everywhere.  The results are the same bit for bit. */
     AGWN_OPT_MIXED_CERTIFY = 12,
-    /* The largest device scratch buffer in bytes, 0 (default): whatever a call takes.  Where it is less than a call
-       would take, or device memory is, the parametric integrals and the terms of the exact forms on few queries are
-       taken in smaller pieces, with the same values; other calls return AGWN_ERR_NOMEM. */
+    /* The largest device scratch buffer, and all temporaries of a build together, in bytes; 0 (default): whatever a
+       call takes.  Where it is less than a call would take, or device memory is, the parametric integrals and the
+       terms of the exact forms on few queries are taken in smaller pieces, with the same values; other calls return
+       AGWN_ERR_NOMEM. */
     AGWN_OPT_SCRATCH_LIMIT = 13
 };
 enum agwn_param_mode

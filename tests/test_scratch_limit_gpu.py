@@ -94,3 +94,19 @@ def test_calls_that_cannot_be_cut():
             ag.eval_gwnr_mesh_batch_fractional(d, np.zeros((500, 3)), np.empty(500), np.array([0.0, 0.0, 1.0]),
                                                np.ones((1, 7)))
         assert e.value.status == 3
+
+
+def test_boundary_fallback_takes_the_sort_alone():
+    """A vertex array far larger than its triangles use takes the radix sort (36 bytes per edge and its counters), without
+    the 16 bytes per edge of the bins."""
+    import antipodal_gb300 as ag
+    n_tri = 20_000
+    rng = np.random.default_rng(1)
+    v = rng.normal(size=(16 * 3 * n_tri + 70_000, 3))
+    idx = rng.integers(0, len(v), 3 * n_tri).astype(np.int32)
+    with ag.CudaDispatcher() as d:
+        want = ag.build_boundary_segments(d, v, idx)
+    vt, it = device(v), device(idx)
+    with limited(ag, 2_900_000) as d:
+        got = ag.build_boundary_segments(d, vt, it).cpu().numpy()
+    np.testing.assert_array_equal(got, want)
