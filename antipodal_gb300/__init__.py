@@ -465,7 +465,9 @@ def build_boundary_segments(dispatcher: CudaDispatcher, vertices, indices):
     i = _View(indices, np.int32, None, "indices")
     fn = getattr(library(), f"agwn_build_boundary_segments_{kind}")
     cnt = C.c_int64()
-    rows = 8192  # most boundaries fit; a longer one takes a second call with its count
+    # Most boundaries fit the first call's rows, and a longer one takes a second call with its count.  The result owns its
+    # rows alone: a slice would keep all 8,192 (458 KB) alive with every small boundary.
+    rows = 8192
     while True:
         out = _empty_like_input(vertices, (rows, 7), dt)
         o = _View(out, dt, None, "out", writable=True)
@@ -473,7 +475,9 @@ def build_boundary_segments(dispatcher: CudaDispatcher, vertices, indices):
         if cnt.value <= rows:
             break
         rows = cnt.value
-    return out[:cnt.value]
+    if cnt.value == rows:
+        return out
+    return out[:cnt.value].clone() if _is_torch(out) else out[:cnt.value].copy()
 
 
 class CudaRobustBatch:

@@ -567,6 +567,8 @@ template <class T>
     out.resize(static_cast<std::size_t>(n));
     if (more)
         run(out.data(), n, &n);
+    else
+        out.shrink_to_fit(); // the caller keeps its rows alone
     return out;
 }
 
