@@ -168,6 +168,10 @@ class CudaDispatcher:
     def synchronize(self):
         _check(library().agwn_context_synchronize(self.handle), "agwn_context_synchronize")
 
+    def trim(self):
+        """Waits for the work queued here, then frees the scratch memory and build temporaries kept for later calls."""
+        _check(library().agwn_context_trim(self.handle), "agwn_context_trim")
+
     def stats(self, reset: bool = False) -> dict:
         s = Stats()
         _check(library().agwn_context_get_stats(self.handle, C.byref(s), int(reset)), "agwn_context_get_stats")

@@ -44,6 +44,7 @@ SIGNATURES = {
     "agwn_context_create": (_I, [_I, _P, _PP]),
     "agwn_context_destroy": (_I, [_P]),
     "agwn_context_synchronize": (_I, [_P]),
+    "agwn_context_trim": (_I, [_P]),
     "agwn_context_set_option": (_I, [_P, _I, _D]),
     "agwn_context_get_option": (_I, [_P, _I, C.POINTER(_D)]),
     "agwn_context_get_stats": (_I, [_P, C.POINTER(Stats), _I]),

@@ -145,7 +145,16 @@ int Context::scratch_reserve(int slot, size_t bytes, void** out)
         return fail(AGWN_ERR_NOMEM, "%zu bytes of scratch exceed the context's limit of %zu", bytes, scratch_limit);
     if (bytes > scratch[slot].cap)
         AGWN_TRY_CUDA(cudaStreamSynchronize(stream));
-    AGWN_TRY(scratch[slot].reserve(bytes == 0 ? 1 : bytes, scratch_limit));
+    int s = scratch[slot].reserve(bytes == 0 ? 1 : bytes, scratch_limit);
+    if (s == AGWN_ERR_NOMEM && arena.depth == 0 && !arena.chunks.empty())
+    {
+        // the build temporaries kept for a next build make room
+        clear_message();
+        AGWN_TRY_CUDA(cudaStreamSynchronize(stream));
+        arena.release();
+        s = scratch[slot].reserve(bytes, scratch_limit);
+    }
+    AGWN_TRY(s);
     *out = scratch[slot].ptr;
     return AGWN_OK;
 }
@@ -413,6 +422,18 @@ int agwn_context_synchronize(agwn_context* ctx)
     AGWN_CHECK_ARG(ctx, "agwn_context_synchronize: null context");
     AGWN_TRY_CUDA(cudaSetDevice(ctx->device));
     return ctx->check_flags();
+}
+
+int agwn_context_trim(agwn_context* ctx)
+{
+    AGWN_CHECK_ARG(ctx, "agwn_context_trim: null context");
+    clear_message();
+    AGWN_TRY_CUDA(cudaSetDevice(ctx->device));
+    AGWN_TRY(ctx->check_flags()); // nothing queued reads what is freed below
+    ctx->arena.release();
+    for (DevBuf& b : ctx->scratch)
+        b.release();
+    return AGWN_OK;
 }
 
 int agwn_context_set_option(agwn_context* ctx, int option, double value)

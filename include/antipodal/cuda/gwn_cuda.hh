@@ -106,6 +106,8 @@ public:
         return v;
     }
     void synchronize() { check(agwn_context_synchronize(m_ctx), "agwn_context_synchronize"); }
+    // Waits, then frees the scratch memory and build temporaries kept for later calls.
+    void trim() { check(agwn_context_trim(m_ctx), "agwn_context_trim"); }
     [[nodiscard]] agwn_context* handle() const noexcept { return m_ctx; }
 
     // The reference's parallel_for runs arbitrary host callables; the GPU library has no form for them and no

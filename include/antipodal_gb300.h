@@ -60,6 +60,9 @@ int agwn_context_create(int device, void* stream, agwn_context** out);
 int agwn_context_destroy(agwn_context* ctx);
 /* Waits for all work of the context and reports device-side error flags raised since the last check. */
 int agwn_context_synchronize(agwn_context* ctx);
+/* Waits as above, then frees the scratch buffers and the build temporaries (up to 1 GB) that the context keeps for its
+ * next calls, which take them anew.  Graphs captured from calls on this context must not run after it. */
+int agwn_context_trim(agwn_context* ctx);
 
 enum agwn_option
 {
