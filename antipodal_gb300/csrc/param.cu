@@ -237,10 +237,10 @@ struct FrameDF
 // quotients.
 //
 // In the frame with x0 = |x0| z these are two-term forms: m = |x0| z, T = |x0| (x y' - y x'), |x0 x r|^2 = n (x^2 + y^2),
-// and z' is not needed.  With the fused chains of df32.cuh a node takes about 320 FP32 operations; with x0's three
-// coordinates and separate products and sums it took about 660 (20,000 queries x 1,024 curves at tol 1e-10: 57.9 -> 26.2
-// ms).  Errors against the exact form did not grow: p50 4.2e-15 -> 2.9e-15, p99 2.6e-11 -> 1.9e-11, p99.9 3.8e-10 ->
-// 2.7e-10 over 4 x 30,000 queries, 30% of them within 1e-3 of a curve.
+// and z' is not needed.  A node takes about 370 FP32 operations; with x0's three coordinates it took about 660.  Errors
+// against the exact form did not grow: p50 4.2e-15 -> 2.8e-15, p99 2.6e-11 -> 1.8e-11, p99.9 3.8e-10 -> 2.3e-10 over 4 x
+// 30,000 queries, 30% of them within 1e-3 of a curve.  (Products that go into their sums without being normalised first
+// would save 10% of the time, and lose half a bit of each.)
 // pc: the pair's curve minus its query as power coefficients about t = 1/2 (k_curves_df), dl = t - 1/2.
 __device__ __forceinline__ df integrand_df(const df (&pc)[12], FrameDF const& F, df dl)
 {
@@ -538,7 +538,7 @@ __global__ void k_param_sum(const double* __restrict__ vals, int nq, int nc, boo
 // Pair integrals in the double-float form: vals[k * nq + i] for the curves c0 + k and the queries q0 + i (pos: these
 // queries' coordinates).
 //
-// The FMA pipe's chains bound it (a lane per pair: some 320 dependent FP32 operations a node, 15 nodes a panel).  The
+// The FMA pipe's chains bound it (a lane per pair: some 370 dependent FP32 operations a node, 15 nodes a panel).  The
 // cost of one (query, curve) integral is heavy-tailed, so the lanes of the whole grid draw their pairs from one counter
 // (a warp takes `take`, 32 or 64, at a time) and walk their panel trees as a team of the exact form does; k_param_sum adds a
 // query's integrals in curve order.  With blocks of 128 queries x 128 curves as the unit, 20,000 queries x 1,024 curves
