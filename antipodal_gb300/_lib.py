@@ -69,6 +69,7 @@ SIGNATURES = {
     "agwn_probe_fp32_peak": (_I, [_P, C.POINTER(_D)]),
     "agwn_probe_atan2": (_I, [_P, _P, _P, _I64, _P, _P]),
     "agwn_probe_math_f64": (_I, [_P, _P, _P, _I64, _P, _P, _P, _P]),
+    "agwn_probe_math_f32": (_I, [_P, _P, _P, _I64, _P, _P, _P, _P]),
     "agwn_probe_fp64_peak": (_I, [_P, _P]),
     "agwn_robust_predicates": (_I, [_P, _I, _P, _P, _P, _P, _I64, _P, _P, _P, _P]),
     "agwn_probe_i128_mul_sub": (_I, [_P, _P, _P, _P, _P, _I64, _P, _P, _P]),

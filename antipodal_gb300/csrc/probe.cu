@@ -212,3 +212,59 @@ extern "C" int agwn_probe_math_f64(agwn_context* ctx, const double* a, const dou
     AGWN_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
     return AGWN_OK;
 }
+
+namespace agwn
+{
+namespace
+{
+// One thread: elements 2 i and 2 i + 1, each by itself and as a packed pair (the last one of an odd number twice).
+__global__ void k_math_f32(const float* __restrict__ a, const float* __restrict__ b, int64_t n,
+                           float* __restrict__ root, float* __restrict__ root2, float* __restrict__ angle,
+                           float* __restrict__ angle2)
+{
+    int64_t const pairs = (n + 1) / 2;
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < pairs; i += int64_t(gridDim.x) * blockDim.x)
+    {
+        int64_t const e0 = 2 * i, e1 = 2 * i + 1 < n ? 2 * i + 1 : e0;
+        float2 const u = make_float2(a[e0], a[e1]), v = make_float2(b[e0], b[e1]);
+        float2 const r2 = sqrt_lv(u), t2 = atan2_lv(u, v);
+        root2[e0] = r2.x;
+        root2[e1] = r2.y;
+        angle2[e0] = t2.x;
+        angle2[e1] = t2.y;
+        root[e0] = sqrt_lv(u.x);
+        root[e1] = sqrt_lv(u.y);
+        angle[e0] = atan2_lv(u.x, v.x);
+        angle[e1] = atan2_lv(u.y, v.y);
+    }
+}
+} // namespace
+} // namespace agwn
+
+extern "C" int agwn_probe_math_f32(agwn_context* ctx, const float* a, const float* b, int64_t n, float* root, float* root2,
+                                   float* angle, float* angle2)
+{
+    AGWN_CHECK_ARG(ctx && n >= 0 && (n == 0 || (a && b && root && root2 && angle && angle2)), "bad arguments");
+    AGWN_TRY_CUDA(cudaSetDevice(ctx->device));
+    if (n == 0)
+        return AGWN_OK;
+    const void *da = nullptr, *db = nullptr;
+    void* d[4] = {};
+    float* const host[4] = {root, root2, angle, angle2};
+    int const slot[4] = {S_MISC2, S_MISC3, S_OUT, S_QUERIES};
+    bool h[4] = {};
+    size_t const bytes = sizeof(float) * size_t(n);
+    AGWN_TRY(stage_in(*ctx, a, bytes, S_MISC0, &da));
+    AGWN_TRY(stage_in(*ctx, b, bytes, S_MISC1, &db));
+    for (int k = 0; k < 4; ++k)
+        AGWN_TRY(stage_out(*ctx, host[k], bytes, slot[k], &d[k], &h[k]));
+    k_math_f32<<<int(std::min<int64_t>(div_up(n, 256), 16 * ctx->sm_count)), 256, 0, ctx->stream>>>(
+        static_cast<const float*>(da), static_cast<const float*>(db), n, static_cast<float*>(d[0]),
+        static_cast<float*>(d[1]), static_cast<float*>(d[2]), static_cast<float*>(d[3]));
+    AGWN_TRY_CUDA(cudaGetLastError());
+    for (int k = 0; k < 4; ++k)
+        if (h[k])
+            AGWN_TRY_CUDA(cudaMemcpyAsync(host[k], d[k], bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    AGWN_TRY_CUDA(cudaStreamSynchronize(ctx->stream));
+    return AGWN_OK;
+}

@@ -454,6 +454,10 @@ int agwn_probe_atan2(agwn_context* ctx, const float* y, const float* x, int64_t 
  * atan2(a, b), a b. */
 int agwn_probe_math_f64(agwn_context* ctx, const double* a, const double* b, int64_t n, double* quotient, double* root,
                         double* angle, double* product);
+/* The exact float form's square root and atan2, sqrt(a) and atan2(a, b): by themselves, and on packed pairs (root2,
+ * angle2; the same bits). */
+int agwn_probe_math_f32(agwn_context* ctx, const float* a, const float* b, int64_t n, float* root, float* root2,
+                        float* angle, float* angle2);
 
 #ifdef __cplusplus
 }
