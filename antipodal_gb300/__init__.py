@@ -467,21 +467,23 @@ def build_boundary_segments(dispatcher: CudaDispatcher, vertices, indices):
     dt, kind = _float_kind(vertices)
     v = _View(vertices, dt, 3, "vertices")
     i = _View(indices, np.int32, None, "indices")
-    fn = getattr(library(), f"agwn_build_boundary_segments_{kind}")
+    fn = getattr(library(), f"agwn_build_boundary_segments_alloc_{kind}")
+    made = []
+
+    def rows(_, n):  # an exception must not leave through the library: it is raised after the call
+        try:
+            made.append(_empty_like_input(vertices, (n, 7), dt))
+            return _View(made[0], dt, None, "out", writable=True).ptr if n else None
+        except Exception as e:  # noqa: BLE001
+            made.append(e)
+            return None
+
     cnt = C.c_int64()
-    # Most boundaries fit the first call's rows, and a longer one takes a second call with its count.  The result owns its
-    # rows alone: a slice would keep all 8,192 (458 KB) alive with every small boundary.
-    rows = 8192
-    while True:
-        out = _empty_like_input(vertices, (rows, 7), dt)
-        o = _View(out, dt, None, "out", writable=True)
-        _check(fn(dispatcher.handle, v.ptr, v.n, i.ptr, i.n, o.ptr, rows, C.byref(cnt)), "build_boundary_segments")
-        if cnt.value <= rows:
-            break
-        rows = cnt.value
-    if cnt.value == rows:
-        return out
-    return out[:cnt.value].clone() if _is_torch(out) else out[:cnt.value].copy()
+    status = fn(dispatcher.handle, v.ptr, v.n, i.ptr, i.n, _lib.ALLOC_ROWS(rows), None, C.byref(cnt))
+    if made and isinstance(made[-1], Exception):
+        raise made[-1]
+    _check(status, "build_boundary_segments")
+    return made[0]
 
 
 class CudaRobustBatch:

@@ -14,6 +14,7 @@ _I64 = C.c_int64
 _I = C.c_int
 _D = C.c_double
 _PP = C.POINTER(C.c_void_p)
+ALLOC_ROWS = C.CFUNCTYPE(C.c_void_p, C.c_void_p, C.c_int64)
 
 AGWN_OK = 0
 STATUS = {0: "ok", 1: "invalid argument", 2: "CUDA runtime error", 3: "out of device memory",
@@ -78,6 +79,8 @@ SIGNATURES = {
     "agwn_robust_eval_grid_f32": (_I, [_P, _P, _P, _P, _I64, _I64, _I64, _P, _P, _P]),
     "agwn_build_boundary_segments_f64": (_I, [_P, _P, _I64, _P, _I64, _P, _I64, _P]),
     "agwn_build_boundary_segments_f32": (_I, [_P, _P, _I64, _P, _I64, _P, _I64, _P]),
+    "agwn_build_boundary_segments_alloc_f64": (_I, [_P, _P, _I64, _P, _I64, ALLOC_ROWS, _P, _P]),
+    "agwn_build_boundary_segments_alloc_f32": (_I, [_P, _P, _I64, _P, _I64, ALLOC_ROWS, _P, _P]),
     "agwn_batch_create": (_I, [_P, _P, C.c_int32, _P, _P, _P, _P, _PP]),
     "agwn_batch_destroy": (_I, [_P]),
     "agwn_batch_tune": (_I, [_P, _P, C.c_int32]),

@@ -236,9 +236,43 @@ __global__ void k_edge_emit(const unsigned long long* __restrict__ keys, const i
     }
 }
 
-// The extraction by radix sort (bins above kBinMax): the first `capacity` rows into the device array d_out.
+// Where the rows go: given their number by prepare, the first `rows` of them into the device array `dev`, then (finish)
+// to `host` if that is the output.  out_for(number, &out, &rows) is the caller's choice of array and rows.
 template <class T>
-int boundary_radix(Context& ctx, const T* dv, int64_t nv, const int32_t* di, int64_t m, T* d_out, int64_t capacity,
+struct RowsOut
+{
+    T* dev = nullptr;
+    T* host = nullptr;
+    int64_t rows = 0;
+
+    template <class OutFor>
+    int prepare(Context& ctx, OutFor out_for, int64_t number)
+    {
+        T* out = nullptr;
+        AGWN_TRY(out_for(number, &out, &rows));
+        if (rows == 0)
+            return AGWN_OK;
+        dev = out;
+        if (!is_device_pointer(out))
+        {
+            host = out;
+            AGWN_TRY(ctx.scratch_reserve(S_MISC2, sizeof(T) * 7 * size_t(rows), reinterpret_cast<void**>(&dev)));
+        }
+        return AGWN_OK;
+    }
+    int finish(Context& ctx) const
+    {
+        if (rows == 0)
+            return AGWN_OK;
+        if (host)
+            AGWN_TRY_CUDA(cudaMemcpyAsync(host, dev, sizeof(T) * 7 * size_t(rows), cudaMemcpyDeviceToHost, ctx.stream));
+        return ctx.check_flags();
+    }
+};
+
+// The extraction by radix sort (bins above kBinMax).
+template <class T, class OutFor>
+int boundary_radix(Context& ctx, const T* dv, int64_t nv, const int32_t* di, int64_t m, OutFor out_for, RowsOut<T>& o,
                    int64_t* n_segments)
 {
     cudaStream_t const st = ctx.stream;
@@ -301,19 +335,20 @@ int boundary_radix(Context& ctx, const T* dv, int64_t nv, const int32_t* di, int
     }
     int64_t const count = int64_t(last_off) + int64_t(last_sum);
     *n_segments = count;
-    if (count == 0 || capacity == 0)
+    AGWN_TRY(o.prepare(ctx, out_for, count));
+    if (o.rows == 0)
         return AGWN_OK;
     AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-    k_edge_emit<T><<<grid, 256, 0, st>>>(kin, net.as<int>(), emit.as<unsigned>(), pos.as<unsigned>(), m, capacity, dv,
-                                         d_out);
+    k_edge_emit<T><<<grid, 256, 0, st>>>(kin, net.as<int>(), emit.as<unsigned>(), pos.as<unsigned>(), m, o.rows, dv,
+                                         o.dev);
     return ctx.launch_end(AGWN_K_OTHER);
 }
 
-// The extraction by bins: *n_segments and the first `rows` rows into d_out, both set by rows_for(*n_segments); or *radix
-// and nothing else where a bin is above kBinMax.  Its buffers are given back before the radix sort takes its own.
-template <class T, class RowsFor>
-int boundary_bins(Context& ctx, const T* dv, int64_t nv, const int32_t* di, int64_t m, RowsFor rows_for, T* const& d_out,
-                  int64_t const& rows, int64_t* n_segments, bool* radix)
+// The extraction by bins, or *radix and nothing else where a bin is above kBinMax.  Its buffers are given back before the
+// radix sort takes its own.
+template <class T, class OutFor>
+int boundary_bins(Context& ctx, const T* dv, int64_t nv, const int32_t* di, int64_t m, OutFor out_for, RowsOut<T>& o,
+                  int64_t* n_segments, bool* radix)
 {
     cudaStream_t const st = ctx.stream;
     ArenaScope scope(ctx);
@@ -347,63 +382,75 @@ int boundary_bins(Context& ctx, const T* dv, int64_t nv, const int32_t* di, int6
     if (*radix)
         return AGWN_OK;
     *n_segments = back[0];
-    AGWN_TRY(rows_for(int64_t(back[0])));
-    if (rows == 0)
+    AGWN_TRY(o.prepare(ctx, out_for, int64_t(back[0])));
+    if (o.rows == 0)
         return AGWN_OK;
     AGWN_TRY(ctx.launch_begin(AGWN_K_OTHER));
-    k_edge_rows<T><<<grid, 256, 0, st>>>(lo.as<int>(), hi.as<unsigned>(), m, bin, net.as<int>(), emitted, dv, rows, d_out);
+    k_edge_rows<T><<<grid, 256, 0, st>>>(lo.as<int>(), hi.as<unsigned>(), m, bin, net.as<int>(), emitted, dv, o.rows,
+                                         o.dev);
     return ctx.launch_end(AGWN_K_OTHER);
 }
 
-template <class T>
-int boundary_build(agwn_context* ctx, const T* vertices, int64_t nv, const int32_t* indices, int64_t n_idx, T* out,
-                   int64_t capacity, int64_t* n_segments)
+template <class T, class OutFor>
+int boundary_build(agwn_context* ctx, const T* vertices, int64_t nv, const int32_t* indices, int64_t n_idx, OutFor out_for,
+                   int64_t* n_segments)
 {
     AGWN_CHECK_ARG(ctx && n_segments, "null context/count");
-    AGWN_CHECK_ARG(nv >= 0 && n_idx >= 0 && n_idx % 3 == 0 && capacity >= 0, "bad sizes");
+    AGWN_CHECK_ARG(nv >= 0 && n_idx >= 0 && n_idx % 3 == 0, "bad sizes");
     AGWN_CHECK_ARG(n_idx == 0 || (vertices && indices), "null geometry");
     AGWN_CHECK_ARG(nv <= (int64_t(1) << 31) && n_idx / 3 < (int64_t(1) << 31), "mesh too large");
     clear_message();
     AGWN_TRY_CUDA(cudaSetDevice(ctx->device));
     *n_segments = 0;
     int64_t const m = n_idx; // one entry per triangle edge
+    RowsOut<T> o;
     if (m == 0)
-        return AGWN_OK;
+        return o.prepare(*ctx, out_for, 0);
     const void *dv = nullptr, *di = nullptr;
     AGWN_TRY(stage_in(*ctx, vertices, sizeof(T) * 3 * nv, S_MISC0, &dv));
     AGWN_TRY(stage_in(*ctx, indices, sizeof(int32_t) * n_idx, S_MISC1, &di));
     const T* const verts = static_cast<const T*>(dv);
     const int32_t* const ip = static_cast<const int32_t*>(di);
-    bool const host_out = out && !is_device_pointer(out);
-    T* d_out = out;
-    int64_t count = 0, rows = 0;
-    // where `count` rows go on the device, at most the capacity
-    auto const rows_for = [&](int64_t most) -> int
-    {
-        rows = out ? std::min(capacity, most) : 0;
-        if (host_out && rows > 0)
-        {
-            void* p = nullptr;
-            AGWN_TRY(ctx->scratch_reserve(S_MISC2, sizeof(T) * 7 * size_t(rows), &p));
-            d_out = static_cast<T*>(p);
-        }
-        return AGWN_OK;
-    };
     bool radix = nv > 16 * m + 65536;
     if (!radix)
-        AGWN_TRY(boundary_bins<T>(*ctx, verts, nv, ip, m, rows_for, d_out, rows, &count, &radix));
+        AGWN_TRY(boundary_bins<T>(*ctx, verts, nv, ip, m, out_for, o, n_segments, &radix));
     if (radix)
-    {
-        AGWN_TRY(rows_for(m));
-        AGWN_TRY(boundary_radix<T>(*ctx, verts, nv, ip, m, d_out, rows, &count));
-    }
-    *n_segments = count;
-    rows = std::min(rows, count);
-    if (rows == 0)
-        return AGWN_OK;
-    if (host_out)
-        AGWN_TRY_CUDA(cudaMemcpyAsync(out, d_out, sizeof(T) * 7 * size_t(rows), cudaMemcpyDeviceToHost, ctx->stream));
-    return ctx->check_flags();
+        AGWN_TRY(boundary_radix<T>(*ctx, verts, nv, ip, m, out_for, o, n_segments));
+    return o.finish(*ctx);
+}
+
+// The rows into a given array, up to its capacity (out may be null: the count alone).
+template <class T>
+int boundary_into(agwn_context* ctx, const T* vertices, int64_t nv, const int32_t* indices, int64_t n_idx, T* out,
+                  int64_t capacity, int64_t* n_segments)
+{
+    AGWN_CHECK_ARG(capacity >= 0, "bad sizes");
+    return boundary_build<T>(ctx, vertices, nv, indices, n_idx,
+                             [&](int64_t number, T** dst, int64_t* rows) -> int
+                             {
+                                 *dst = out;
+                                 *rows = out ? std::min(capacity, number) : 0;
+                                 return AGWN_OK;
+                             },
+                             n_segments);
+}
+
+// All rows into the array that alloc gives for their number.
+template <class T>
+int boundary_alloc(agwn_context* ctx, const T* vertices, int64_t nv, const int32_t* indices, int64_t n_idx,
+                   agwn_alloc_rows alloc, void* user, int64_t* n_segments)
+{
+    AGWN_CHECK_ARG(alloc, "null alloc");
+    return boundary_build<T>(ctx, vertices, nv, indices, n_idx,
+                             [&](int64_t number, T** dst, int64_t* rows) -> int
+                             {
+                                 *dst = static_cast<T*>(alloc(user, number));
+                                 *rows = number;
+                                 return *dst || number == 0 ? int(AGWN_OK)
+                                                            : fail(AGWN_ERR_NOMEM, "no array for %lld boundary rows",
+                                                                   (long long)number);
+                             },
+                             n_segments);
 }
 } // namespace
 } // namespace agwn
@@ -414,11 +461,23 @@ extern "C" int agwn_build_boundary_segments_f64(agwn_context* ctx, const double*
                                                 const int32_t* indices, int64_t n_indices, double* out,
                                                 int64_t capacity, int64_t* n_segments)
 {
-    return boundary_build<double>(ctx, vertices, n_vertices, indices, n_indices, out, capacity, n_segments);
+    return boundary_into<double>(ctx, vertices, n_vertices, indices, n_indices, out, capacity, n_segments);
 }
 extern "C" int agwn_build_boundary_segments_f32(agwn_context* ctx, const float* vertices, int64_t n_vertices,
                                                 const int32_t* indices, int64_t n_indices, float* out,
                                                 int64_t capacity, int64_t* n_segments)
 {
-    return boundary_build<float>(ctx, vertices, n_vertices, indices, n_indices, out, capacity, n_segments);
+    return boundary_into<float>(ctx, vertices, n_vertices, indices, n_indices, out, capacity, n_segments);
+}
+extern "C" int agwn_build_boundary_segments_alloc_f64(agwn_context* ctx, const double* vertices, int64_t n_vertices,
+                                                      const int32_t* indices, int64_t n_indices, agwn_alloc_rows alloc,
+                                                      void* user, int64_t* n_segments)
+{
+    return boundary_alloc<double>(ctx, vertices, n_vertices, indices, n_indices, alloc, user, n_segments);
+}
+extern "C" int agwn_build_boundary_segments_alloc_f32(agwn_context* ctx, const float* vertices, int64_t n_vertices,
+                                                      const int32_t* indices, int64_t n_indices, agwn_alloc_rows alloc,
+                                                      void* user, int64_t* n_segments)
+{
+    return boundary_alloc<float>(ctx, vertices, n_vertices, indices, n_indices, alloc, user, n_segments);
 }

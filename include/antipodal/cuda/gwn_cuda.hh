@@ -548,29 +548,30 @@ template <class T>
     static_assert(sizeof(weighted_segment3<T>) == 7 * sizeof(T));
     auto const* v = cuda::detail::raw(vertices);
     auto const* i = reinterpret_cast<std::int32_t const*>(indices.data());
-    auto run = [&](weighted_segment3<T>* out, std::int64_t cap, std::int64_t* n)
+    std::vector<weighted_segment3<T>> out;
+    // the rows, once their number is known; an exception must not leave through the C interface
+    auto const rows = [](void* user, std::int64_t n) -> void*
     {
-        if constexpr (std::is_same_v<T, double>)
-            cuda::check(agwn_build_boundary_segments_f64(dispatcher.handle(), v, std::int64_t(vertices.size()), i,
-                                                         std::int64_t(indices.size()),
-                                                         reinterpret_cast<double*>(out), cap, n),
-                        "build_boundary_segments");
-        else
-            cuda::check(agwn_build_boundary_segments_f32(dispatcher.handle(), v, std::int64_t(vertices.size()), i,
-                                                         std::int64_t(indices.size()),
-                                                         reinterpret_cast<float*>(out), cap, n),
-                        "build_boundary_segments");
+        auto& o = *static_cast<std::vector<weighted_segment3<T>>*>(user);
+        try
+        {
+            o.resize(static_cast<std::size_t>(n));
+        }
+        catch (...)
+        {
+            return nullptr;
+        }
+        return o.data();
     };
-    // most boundaries fit the first call's rows; a longer one takes a second call with its count
     std::int64_t n = 0;
-    std::vector<weighted_segment3<T>> out(4096);
-    run(out.data(), std::int64_t(out.size()), &n);
-    bool const more = n > std::int64_t(out.size());
-    out.resize(static_cast<std::size_t>(n));
-    if (more)
-        run(out.data(), n, &n);
+    if constexpr (std::is_same_v<T, double>)
+        cuda::check(agwn_build_boundary_segments_alloc_f64(dispatcher.handle(), v, std::int64_t(vertices.size()), i,
+                                                           std::int64_t(indices.size()), rows, &out, &n),
+                    "build_boundary_segments");
     else
-        out.shrink_to_fit(); // the caller keeps its rows alone
+        cuda::check(agwn_build_boundary_segments_alloc_f32(dispatcher.handle(), v, std::int64_t(vertices.size()), i,
+                                                           std::int64_t(indices.size()), rows, &out, &n),
+                    "build_boundary_segments");
     return out;
 }
 

@@ -277,6 +277,15 @@ int agwn_build_boundary_segments_f64(agwn_context* ctx, const double* vertices, 
 int agwn_build_boundary_segments_f32(agwn_context* ctx, const float* vertices, int64_t n_vertices,
                                      const int32_t* indices, int64_t n_indices, float* out, int64_t capacity,
                                      int64_t* n_segments);
+/* The same with all rows written to the array (host or device, 7 * rows scalars) that alloc returns once their number is
+ * known, from the calling thread; NULL ends the call with AGWN_ERR_NOMEM (for no rows it is not used). */
+typedef void* (*agwn_alloc_rows)(void* user, int64_t rows);
+int agwn_build_boundary_segments_alloc_f64(agwn_context* ctx, const double* vertices, int64_t n_vertices,
+                                           const int32_t* indices, int64_t n_indices, agwn_alloc_rows alloc, void* user,
+                                           int64_t* n_segments);
+int agwn_build_boundary_segments_alloc_f32(agwn_context* ctx, const float* vertices, int64_t n_vertices,
+                                           const int32_t* indices, int64_t n_indices, agwn_alloc_rows alloc, void* user,
+                                           int64_t* n_segments);
 
 /* ---- many robust meshes in one persistent launch ----------------------------------------------------------
  * No single reference counterpart: the result equals calling eval_gwnr_mesh_batch_robust
