@@ -214,11 +214,12 @@ __device__ __forceinline__ V sqrt_lv(V a)
 }
 
 // atan2(n, d): with q = min / max of the magnitudes and its exact residual r in units of the quotient, atan(q + r) =
-// q + (q^3 Q(q^2) + r / (1 + q^2)), Q of degree 8 (a minimax fit, relative error of atan 2.6e-9) and 1 / (1 + q^2) by a
-// line (4% is near enough for r), then +-atan + {0, pi/2, pi} in one FMA: pi/2 is 1.8663789 x 0.84162778 to 1.6e-14.
-// Errors in ulp over 4,194,304 arguments each, mean and largest, the library's atan2f in brackets: normal 0.261, 1.30
-// (0.289, 1.79); ratios of any size 0.266, 1.29 (0.275, 1.74); next to the diagonals 0.289, 1.33 (0.291, 1.38), where a fit
-// of degree 7 has 0.313 and 1.40.
+// q + (q^3 Q(q^2) + r / (1 + q^2)), Q of degree 7 and 1 / (1 + q^2) by a line (4% is near enough for r), then +-atan +
+// {0, pi/2, pi} in one FMA: pi/2 is 1.8663789 x 0.84162778 to 1.6e-14.  Q is a minimax fit whose error counts 2.5 times
+// from q = 0.75 on, where the sums' own roundings are largest; with its float coefficients atan's relative error is below
+// 2.8e-8.  Errors in ulp over 4,194,304 arguments each, mean and largest, the library's atan2f in brackets: normal 0.266,
+// 1.22 (0.289, 1.79); ratios of any size 0.267, 1.10 (0.275, 1.74); next to the diagonals 0.275, 1.16 (0.291, 1.38).  (A
+// fit that weighs all q alike: 0.313 and 1.40 there.)
 template <class V>
 __device__ __forceinline__ V atan2_lv(V n, V d)
 {
@@ -242,15 +243,14 @@ __device__ __forceinline__ V atan2_lv(V n, V d)
     V const rem = lv_mul(lv_fma(lv_flip(q), mx, mn), rc);
     V const s = lv_mul(q, q);
     V const slope = lv_fma(lv_set<V>(-0.5f), s, lv_set<V>(0.95710678f));
-    V p = lv_set<V>(-0.001793622737750411f);
-    p = lv_fma(p, s, lv_set<V>(0.01091461069881916f));
-    p = lv_fma(p, s, lv_set<V>(-0.031177856028079987f));
-    p = lv_fma(p, s, lv_set<V>(0.05795760452747345f));
-    p = lv_fma(p, s, lv_set<V>(-0.0840345099568367f));
-    p = lv_fma(p, s, lv_set<V>(0.10952185839414597f));
-    p = lv_fma(p, s, lv_set<V>(-0.14264242351055145f));
-    p = lv_fma(p, s, lv_set<V>(0.19998548924922943f));
-    p = lv_fma(p, s, lv_set<V>(-0.33333298563957214f));
+    V p = lv_set<V>(0.0026763607747852802f);
+    p = lv_fma(p, s, lv_set<V>(-0.015392192639410496f));
+    p = lv_fma(p, s, lv_set<V>(0.041636910289525986f));
+    p = lv_fma(p, s, lv_set<V>(-0.0742095410823822f));
+    p = lv_fma(p, s, lv_set<V>(0.1060626283288002f));
+    p = lv_fma(p, s, lv_set<V>(-0.14196659624576569f));
+    p = lv_fma(p, s, lv_set<V>(0.19992151856422424f));
+    p = lv_fma(p, s, lv_set<V>(-0.3333309292793274f));
     a = lv_add(q, lv_fma(lv_mul(q, s), p, lv_mul(rem, slope)));
 #pragma unroll
     for (int h = 0; h < W; ++h)
