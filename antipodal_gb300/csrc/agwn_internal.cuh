@@ -134,7 +134,7 @@ struct CellGrid
     int64_t entries = 0;
     int per_leaf = 0;   // cells per leaf it was built with
     int64_t calls = 0;  // calls prepared for on this hierarchy so far
-    bool pinned = false; // a captured call reads it: its buffers stay as they are
+    bool pinned = false; // a captured call reads it: no finer grid takes its place while this hierarchy is cached
     bool valid = false;
     void release()
     {
@@ -165,6 +165,10 @@ struct Context
     long long* d_counters = nullptr; // kCounters: [0] fp64 pairs, [1] pairs, [2] parametric skips, [3] certified pairs, [4..7] integer, [8..11] patches
                                      // term: queries, cell-list entries, candidate leaves, exact tests
     DevBuf scratch[S_COUNT];
+    // Buffers that a captured call was given: a graph holds their addresses, so one that has to grow is set aside, not
+    // freed, until the context ends or is trimmed.
+    bool scratch_captured[S_COUNT] = {};
+    std::vector<void*> set_aside;
     Arena arena;
     static constexpr int kArrivals = 2048;
     int* d_arrivals = nullptr; // kArrivals zeroed counters, left zeroed by each kernel that uses them
@@ -228,6 +232,7 @@ struct Context
     }
 
     int scratch_reserve(int slot, size_t bytes, void** out);
+    void scratch_drop(int slot); // frees a slot's buffer (nothing queued reads it), or sets it aside
     // scratch_reserve of fixed + unit * *units bytes; *units is halved, down to 1, while there is no memory for them
     int scratch_reserve_units(int slot, size_t fixed, size_t unit, int64_t* units, void** out);
     // Brackets a launch with timing events when AGWN_OPT_TIMING is on; always counts the launch.

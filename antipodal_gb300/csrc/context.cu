@@ -143,8 +143,14 @@ int Context::scratch_reserve(int slot, size_t bytes, void** out)
     // queued work may still read.
     if (bytes > scratch_limit)
         return fail(AGWN_ERR_NOMEM, "%zu bytes of scratch exceed the context's limit of %zu", bytes, scratch_limit);
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess)
+        cudaGetLastError(); // (the legacy stream beside another stream's capture: the call's launches will say so)
     if (bytes > scratch[slot].cap)
+    {
         AGWN_TRY_CUDA(cudaStreamSynchronize(stream));
+        scratch_drop(slot);
+    }
     int s = scratch[slot].reserve(bytes == 0 ? 1 : bytes, scratch_limit);
     if (s == AGWN_ERR_NOMEM && arena.depth == 0 && !arena.chunks.empty())
     {
@@ -155,8 +161,21 @@ int Context::scratch_reserve(int slot, size_t bytes, void** out)
         s = scratch[slot].reserve(bytes, scratch_limit);
     }
     AGWN_TRY(s);
+    scratch_captured[slot] |= status != cudaStreamCaptureStatusNone;
     *out = scratch[slot].ptr;
     return AGWN_OK;
+}
+
+void Context::scratch_drop(int slot)
+{
+    DevBuf& b = scratch[slot];
+    if (scratch_captured[slot] && b.ptr)
+    {
+        set_aside.push_back(b.ptr);
+        b = DevBuf{};
+    }
+    b.release();
+    scratch_captured[slot] = false;
 }
 
 int Context::scratch_reserve_units(int slot, size_t fixed, size_t unit, int64_t* units, void** out)
@@ -290,6 +309,18 @@ int stage_out(Context& ctx, void* dst, size_t bytes, int slot, void** dev, bool*
 
 using namespace agwn;
 
+static void release_scratch(Context& ctx)
+{
+    for (int k = 0; k < S_COUNT; ++k)
+    {
+        ctx.scratch[k].release();
+        ctx.scratch_captured[k] = false;
+    }
+    for (void* p : ctx.set_aside)
+        cudaFree(p);
+    ctx.set_aside.clear();
+}
+
 extern "C"
 {
 const char* agwn_status_string(int status)
@@ -385,8 +416,7 @@ int agwn_context_destroy(agwn_context* ctx)
     cudaSetDevice(ctx->device);
     if (ctx->stream)
         cudaStreamSynchronize(ctx->stream);
-    for (auto& b : ctx->scratch)
-        b.release();
+    release_scratch(*ctx);
     ctx->arena.release();
     ctx->bernstein.release();
     ctx->ray_cache.h.release();
@@ -431,8 +461,7 @@ int agwn_context_trim(agwn_context* ctx)
     AGWN_TRY_CUDA(cudaSetDevice(ctx->device));
     AGWN_TRY(ctx->check_flags()); // nothing queued reads what is freed below
     ctx->arena.release();
-    for (DevBuf& b : ctx->scratch)
-        b.release();
+    release_scratch(*ctx);
     return AGWN_OK;
 }
 

@@ -787,8 +787,8 @@ int param_chunks(Context& ctx, int64_t n, int64_t n_curves, int64_t most, double
         // the larger buffers of this attempt or an earlier call make room
         clear_message();
         AGWN_TRY_CUDA(cudaStreamSynchronize(ctx.stream));
-        ctx.scratch[S_SEGS_RAW].release();
-        ctx.scratch[S_FRAME].release();
+        ctx.scratch_drop(S_SEGS_RAW);
+        ctx.scratch_drop(S_FRAME);
     }
     if (d_nodes)
         AGWN_TRY_CUDA(cudaMemsetAsync(d_nodes, 0, sizeof(int32_t) * n, ctx.stream));
