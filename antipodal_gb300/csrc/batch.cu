@@ -277,8 +277,10 @@ extern "C" int agwn_batch_create(agwn_context* ctx, const agwn_robust* const* me
                         b->candidates.push_back({block, k, tile, stack});
     // Untuned: 128 threads, so that a small batch spreads over the SMs, and 256 where the int64_grid form has blocks to
     // spare, since twice the queries then share a staged tile (mixed, 16,864 queries on 4 meshes: 73 us with 128 threads
-    // against 82; 175,645 on 8: 151 against 169; 536,007 on 6: 380 against 362; 3.1e6 on 16: 1451 against 1308).  The
-    // other policies are bound by FP64 and never faster with 256 (int128_grid, 2,055,880: 19.6 ms against 19.7).
+    // against 82; 175,645 on 8: 151 against 169; 536,007 on 6: 380 against 362; 3.1e6 on 16: 1451 against 1308; exact,
+    // 222,319 on 6: 749 against 800; 754,661: 4.50 ms against 4.53; 1.2e6 on 12: 4.02 against 3.92; 6.8e6 on 32: 26.1
+    // against 26.0).  The other policies are bound by FP64 and never faster with 256 (int128_grid, 2,055,880: 19.6 ms
+    // against 19.7).
     int const block = ops_of(policy).has_mixed && total_q >= int64_t(1) << 19 ? 256 : 128;
     b->conf = {block, 1, 512, max_depth < 32 ? 32 : 64};
     *plan = b;

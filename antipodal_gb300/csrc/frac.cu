@@ -596,8 +596,8 @@ int mesh_batch(agwn_context* ctx, const agwn_bvh* bvh, const T* positions, int64
     // From 2^21 queries; in float, whose counts take a good part of a call, from 3 x 2^18 (float, 102 segments, in one
     // piece against halves: 500,000 queries 202 us against 206, 884,736 342 against 316, 1,815,848 659 against 610; double,
     // 884,736: 6608 against 6592).
-    if (n >= (sizeof(T) == 4 ? int64_t(3) << 18 : int64_t(1) << 21) && want_frac && bvh && bvh->n_tri > 0 && is_device_pointer(positions) &&
-        is_device_pointer(out))
+    if (n >= (sizeof(T) == 4 ? int64_t(3) << 18 : int64_t(1) << 21) && want_frac && bvh && bvh->n_tri > 0 &&
+        is_device_pointer(positions) && is_device_pointer(out))
     {
         AGWN_TRY(stage_in(*ctx, boundary, sizeof(T) * 7 * n_seg, S_MISC0, &dseg));
         AGWN_TRY(mesh_batch_chunked<T>(*ctx, bvh, positions, n, out, x0, static_cast<const T*>(dseg), n_seg));

@@ -74,10 +74,12 @@ enum agwn_option
        evaluated in FP64 with the reference arithmetic.  Default 4. */
     AGWN_OPT_MIXED_TAU = 1,
     /* Queries owned by each thread in the fractional kernels (1, 2, 4 or 8; the mixed kernel packs them in pairs
-       and runs 1 as 2).  Default 2. */
+       and runs 1 as 2).  Default 2.  The exact form in double takes one, and calls on few queries (fewer than 256 per
+       SM), which are shared out by segment, one per lane, whatever this says; no value depends on it. */
     AGWN_OPT_QUERIES_PER_THREAD = 2,
-    /* Threads per block of the fractional kernels (64..256, a multiple of 32), or 0 (default): 128, and 256 for the
-       mixed kernel when the boundary spans more than one segment tile (more queries share each staged tile). */
+    /* Threads per block of the fractional kernels (64..256, a multiple of 32), or 0 (default): 64 for the exact form in
+       double, 128 in float; 128 for the mixed kernel, and 256 when its entries span more than one segment tile or one
+       tile of more than 512 (more queries share each staged tile).  Calls on few queries take 128. */
     AGWN_OPT_FRAC_BLOCK = 3,
     /* Record CUDA events around the library's kernels and accumulate their device time (0/1).  Default 0. */
     AGWN_OPT_TIMING = 4,
@@ -227,7 +229,9 @@ int agwn_mesh_batch_integer_ties_f64(agwn_context* ctx, const double* vertices, 
  * (src/antipodal/math/robust_predicates.hh).  The evaluator owns device copies of the quantised (or, for
  * exact_float, double) triangles and swapped boundary, and a hierarchy that replaces Embree's traversal; the
  * caller's arrays need not outlive it.  Counts equal the reference's bit for bit; the fractional term matches it
- * up to the last bits of atan2.  Precision policy: */
+ * up to the last bits of atan2 and, under int64_grid with up to 4,096 segments, of the sum: those evaluators add
+ * their segments in the order of the boundary's chains, not the caller's.  Contexts on several host threads may
+ * evaluate one evaluator at the same time.  Precision policy: */
 enum agwn_robust_policy
 {
     AGWN_ROBUST_INT64_GRID = 0,  /* 20-bit grid, 64-bit determinants (the reference's default for float)     */
