@@ -62,7 +62,8 @@ __device__ __forceinline__ int batch_count(const BMesh& m, const Frame32& f, qv3
 // What bounds the mixed form: issue (81% busy, the FMA pipe 49%) with 32 warps an SM.  It is compiled for 4 blocks of 256
 // (one query per thread) or 3 (two): left to itself the compiler takes 64 or 80 registers with the smallest change and
 // spills either way (16 meshes of up to 20,000 triangles, 72^3 grids: 1440 us at 80, 1290 at 64 with 16 bytes spilled,
-// 1321 at 48).  The exact form takes what it takes.
+// 1321 at 48).  The exact form is held by FP64 and left to the compiler (64 registers and 72 bytes spilled with one query
+// per thread, 122 and none with two).
 template <class T, class P, int K, int kStack, bool Mixed>
 __global__ void __launch_bounds__(256, Mixed ? (K == 1 ? 4 : 3) : 0) k_batch(
     const BMesh* __restrict__ meshes, const BItem* __restrict__ items, int n_items, int* __restrict__ head, int tile,
